@@ -91,7 +91,8 @@ struct SideHost {
     int n_init_leaves = 0;
     int64_t npairs = 0;
     SibGroups sib;                      // Toeplitz I2O by sibling groups (ngroups = 0: per node)
-    GroupTiles grp;                     // dense I2O for few right-hand sides, grouped by stored block
+    PairTiles pairs;                    // dense I2O by stored block, products in a workspace's buffer
+    PairTiles pairs_small;              // the same in small units, for h2b_farmul_noalloc
     int maxslen = 1;
     std::vector<int64_t> mom_off_host;  // moment offsets per unit rhs (host copy)
     std::vector<int64_t> spec_off_host; // spectrum offsets per unit rhs (host copy)
@@ -141,6 +142,8 @@ struct h2b_workspace {
     int max_nrhs = 1;
     void *am = nullptr, *dm = nullptr, *as = nullptr, *ds = nullptr;
     void *xbuf = nullptr, *ybuf = nullptr;  // staging for h2b_matvec_host
+    void *prod = nullptr;   // pair products of the dense I2O
+    size_t prod_bytes = 0;
     void *xnear = nullptr;  // gathered x rows for the tensor-core near kernel (real, >= 8 RHS)
     unsigned *timeouts = nullptr;  // pinned: the device's tensor-core wait timeouts before / after a call
     std::atomic<int> busy{0};
@@ -481,71 +484,103 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
     return H2B_OK;
 }
 
-// Chunks and tiles of the grouped dense I2O (GroupTiles) for the receiving nodes of side `s`:
-// chunks of up to GT_R consecutive receiving nodes of one level -- fewer when the map has too few
-// receiving nodes to give every SM a full chunk (down to 4 per chunk: a small map trades block
-// reuse for SMs; with two chunks per SM as the target the large maps lost more reuse than they
-// gained SMs); per chunk, its pairs sorted by
-// stored block, then by their rank among the receiver's pairs reading that block, then by receiver,
-// and cut into tiles of at most GT_P pairs with one block and distinct receivers.
-h2b_status build_group_tiles(h2b_core *c, const h2b_side_desc &s, SideHost &h,
-                             const std::vector<int64_t> &cpl_elem_off) {
+// A unit's pair products take at most this much of a workspace per right-hand side, and a workspace's
+// buffer holds as many right-hand sides as fit in it.
+constexpr int64_t PAIR_BUFFER_BYTES = 256ll << 20;
+// the pair products of h2b_farmul_noalloc, beside its scratch
+constexpr int64_t NOALLOC_PRODUCT_BYTES = 4 << 20;
+
+// Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of side `s`,
+// a unit's products taking at most `unit_bytes` per right-hand side. Left empty (per-node kernel)
+// when one receiving node's products alone exceed that.
+h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, const h2b_side_desc &s, const h2b_side_desc &other,
+                            const std::vector<int64_t> &cpl_elem_off, const std::vector<int64_t> &perm_set,
+                            int64_t unit_bytes, PairTiles &out) {
+    const int np = s.i2o_ptr[s.nnodes];
+    if (np == 0) return H2B_OK;
+    // every pair's key {block, rows, k, permutations}: one per coupling, unless a coupling is used
+    // with two shapes
+    struct Key { int64_t off, perm; int nc, snc; };
+    auto same_block = [](const Key &a, const Key &b) { return a.off == b.off && a.nc == b.nc && a.snc == b.snc; };
+    std::vector<Key> keys;
+    std::vector<int> key(np), of_coupling((size_t)std::max<int64_t>(d.ncouplings, 1), -1);
+    std::map<std::tuple<int64_t, int, int>, int> other_shapes;
     std::vector<int> recv;
-    for (int n = 0; n < s.nnodes; ++n)
-        if (s.i2o_ptr[n + 1] > s.i2o_ptr[n]) recv.push_back(n);
-    if (recv.empty()) return H2B_OK;
-    int nsm = 148;
-    CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    const int R = std::min(GT_R, std::max(4, (int)(recv.size() / (size_t)nsm)));
-    std::vector<int> chunk_ptr{0}, rcv, tile_ptr{0}, tile_pp{0}, pair;
-    std::vector<unsigned char> slot;
-    struct E { int64_t key; int rank, slot, p; };
-    size_t i = 0;
-    while (i < recv.size()) {
-        const int lvl = s.level[recv[i]];
-        const size_t j0 = i;
-        while (i < recv.size() && (int)(i - j0) < R && s.level[recv[i]] == lvl) rcv.push_back(recv[i++]);
-        std::vector<E> es;
-        for (size_t j = j0; j < i; ++j) {
-            const int n = recv[j];
-            std::map<int64_t, int> rank;
-            for (int p = s.i2o_ptr[n]; p < s.i2o_ptr[n + 1]; ++p) {
-                const int64_t key = cpl_elem_off[p];
-                es.push_back({key, rank[key]++, (int)(j - j0), p});
+    int pstride = 1;
+    for (int n = 0; n < s.nnodes; ++n) {
+        if (s.i2o_ptr[n + 1] == s.i2o_ptr[n]) continue;
+        recv.push_back(n);
+        const int nc = (int)ncoef_host(s, s.level[n]);
+        pstride = std::max(pstride, nc);
+        for (int p = s.i2o_ptr[n]; p < s.i2o_ptr[n + 1]; ++p) {
+            const int64_t k = s.i2o_coupling[p];
+            const int snc = (int)ncoef_host(other, other.level[s.i2o_src[p]]);
+            int *id = &of_coupling[k];
+            if (*id >= 0 && (keys[*id].nc != nc || keys[*id].snc != snc))
+                id = &other_shapes.emplace(std::make_tuple(k, nc, snc), -1).first->second;
+            if (*id < 0) {
+                *id = (int)keys.size();
+                keys.push_back({cpl_elem_off[k], perm_set.empty() ? -1 : perm_set[k], nc, snc});
             }
+            key[p] = *id;
         }
-        std::sort(es.begin(), es.end(), [](const E &a, const E &b) {
-            return a.key != b.key ? a.key < b.key : (a.rank != b.rank ? a.rank < b.rank : a.slot < b.slot);
-        });
-        unsigned used = 0;
-        int64_t key = -1;
-        int len = 0;
-        for (const E &e : es) {
-            if (len > 0 && (e.key != key || len == GT_P || (used >> e.slot & 1u))) {
-                tile_pp.push_back((int)pair.size());
-                used = 0;
-                len = 0;
-            }
-            key = e.key;
-            used |= 1u << e.slot;
-            ++len;
-            pair.push_back(e.p);
-            slot.push_back((unsigned char)e.slot);
-        }
-        if (len > 0) tile_pp.push_back((int)pair.size());
-        chunk_ptr.push_back((int)rcv.size());
-        tile_ptr.push_back((int)tile_pp.size() - 1);
     }
-    GroupTiles &g = h.grp;
+    std::vector<int> order(keys.size()), rank(keys.size());
+    for (size_t i = 0; i < keys.size(); ++i) order[i] = (int)i;
+    std::sort(order.begin(), order.end(), [&](int a, int b) {
+        const Key &x = keys[a], &y = keys[b];
+        return std::tie(x.off, x.nc, x.snc, x.perm, a) < std::tie(y.off, y.nc, y.snc, y.perm, b);
+    });
+    for (size_t i = 0; i < keys.size(); ++i) rank[order[i]] = (int)i;
+    for (int p = 0; p < np; ++p) key[p] = rank[key[p]];
+
+    const int64_t max_pairs = unit_bytes / ((c->field == H2B_COMPLEX ? 16 : 8) * (int64_t)pstride);
+    std::vector<int> pair(np), count;
+    std::vector<int4> tile;
+    std::vector<PairUnit> units;
+    int64_t most = 0;
+    for (size_t i = 0; i < recv.size();) {
+        const size_t i0 = i;
+        const int p0 = s.i2o_ptr[recv[i]];
+        while (i < recv.size() && s.i2o_ptr[recv[i] + 1] - p0 <= max_pairs) ++i;
+        if (i == i0) return H2B_OK;
+        const int p1 = s.i2o_ptr[recv[i - 1] + 1];
+        most = std::max<int64_t>(most, p1 - p0);
+        // the unit's pairs by key, in list order within a key
+        if ((size_t)(p1 - p0) >= keys.size() / 8) {
+            count.assign(keys.size() + 1, 0);
+            for (int p = p0; p < p1; ++p) ++count[key[p] + 1];
+            for (size_t k = 0; k < keys.size(); ++k) count[k + 1] += count[k];
+            for (int p = p0; p < p1; ++p) pair[p0 + count[key[p]]++] = p;
+        } else {
+            for (int p = p0; p < p1; ++p) pair[p] = p;
+            std::sort(pair.begin() + p0, pair.begin() + p1,
+                      [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
+        }
+        PairUnit u{(int)tile.size(), 0, 0, (int)i0, (int)(i - i0), p0};
+        for (int a = p0; a < p1;) {
+            const Key &k = keys[order[key[pair[a]]]];
+            int b = a + 1;
+            while (b < p1 && same_block(keys[order[key[pair[b]]]], k)) ++b;
+            const int nt = (b - a + PAIR_TILE - 1) / PAIR_TILE;  // tiles of the run, of equal pairs
+            for (int t = 0; t < nt; ++t) {
+                const int e0 = a + (int)((int64_t)(b - a) * t / nt), e1 = a + (int)((int64_t)(b - a) * (t + 1) / nt);
+                tile.push_back(make_int4(e0, e1 - e0, k.nc, k.snc));
+                u.maxpairs = std::max(u.maxpairs, e1 - e0);
+            }
+            a = b;
+        }
+        u.ntiles = (int)tile.size() - u.tile0;
+        units.push_back(u);
+    }
     int *q;
-    unsigned char *u;
-    CUDA_TRY(c->upload(&q, chunk_ptr.data(), chunk_ptr.size())); g.chunk_ptr = q;
-    CUDA_TRY(c->upload(&q, rcv.data(), rcv.size())); g.rcv = q;
-    CUDA_TRY(c->upload(&q, tile_ptr.data(), tile_ptr.size())); g.tile_ptr = q;
-    CUDA_TRY(c->upload(&q, tile_pp.data(), tile_pp.size())); g.tile_pp = q;
-    CUDA_TRY(c->upload(&q, pair.data(), pair.size())); g.pair = q;
-    CUDA_TRY(c->upload(&u, slot.data(), slot.size())); g.slot = u;
-    g.nchunks = (int)chunk_ptr.size() - 1;
+    int4 *t4;
+    CUDA_TRY(c->upload(&q, pair.data(), pair.size())); out.pair = q;
+    CUDA_TRY(c->upload(&q, recv.data(), recv.size())); out.rcv = q;
+    CUDA_TRY(c->upload(&t4, tile.data(), tile.size())); out.tile = t4;
+    out.units = units;
+    out.unit_elems = most * pstride;
+    out.pstride = pstride;
     return H2B_OK;
 }
 
@@ -1114,7 +1149,16 @@ h2b_status build_core(h2b_core *c, const h2b_map_desc &d) {
             st = build_sibling_groups(c, sd, h, o.spec_off_host, off);
             if (st) return st;
         } else if (d.coupling_kind == H2B_COUPLING_DENSE) {
-            st = build_group_tiles(c, sd, h, pcpl);
+            const h2b_side_desc &so = side == 0 ? d.trial : d.test;
+            st = build_pair_tiles(c, d, sd, so, off, perm_set, PAIR_BUFFER_BYTES, h.pairs);
+            if (st) return st;
+            // h2b_farmul_noalloc: only maps whose moments can fit its scratch ever take it
+            const int64_t far = (c->precision == H2B_FP64 ? 8 : 4) * (cplx ? 2 : 1);
+            const int64_t sum = cplx ? 16 : 8;
+            if (h.pairs.unit_elems * sum <= NOALLOC_PRODUCT_BYTES && h.pairs.units.size() == 1)
+                h.pairs_small = h.pairs;
+            else if (2 * std::max(c->test.mom_total, c->trial.mom_total) * far <= (int64_t)H2B_NOALLOC_SCRATCH_BYTES)
+                st = build_pair_tiles(c, d, sd, so, off, perm_set, NOALLOC_PRODUCT_BYTES, h.pairs_small);
             if (st) return st;
         }
     }
@@ -1262,6 +1306,16 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
     if (e == cudaSuccess) e = al(&ws->dm, mom * tsz);
     if (e == cudaSuccess) e = al(&ws->as, spec * ssz);
     if (e == cudaSuccess) e = al(&ws->ds, spec * ssz);
+    // pair products of the dense I2O: all right-hand sides of its largest unit, within the buffer's
+    // bound (the FP32 form takes that path up to PAIR_MAX_COLS32 field columns only)
+    const int64_t cols = core->precision == H2B_FP64
+                             ? (int64_t)max_nrhs * core->dmap.ncomp
+                             : std::min<int64_t>((int64_t)max_nrhs * core->dmap.ncomp, PAIR_MAX_COLS32 / (cplx ? 2 : 1));
+    for (const SideHost *h : {&core->test, &core->trial}) {
+        const int64_t unit = h->pairs.unit_elems * (int64_t)vsz;
+        ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min(unit * cols, std::max(unit, PAIR_BUFFER_BYTES)));
+    }
+    if (e == cudaSuccess) e = al(&ws->prod, ws->prod_bytes);
     if (e == cudaSuccess) e = al(&ws->xbuf, ndof * vsz);
     if (e == cudaSuccess) e = al(&ws->ybuf, ndof * vsz);
     if (e == cudaSuccess && !cplx && max_nrhs >= 8)
@@ -1316,10 +1370,11 @@ h2b_status run_i2o(h2b_core *c, const SideHost &D, const SideHost &A, const FarA
         return H2B_OK;
     }
     const bool cplx = c->field == H2B_COMPLEX;
-    if (D.grp.nchunks > 0 && i2o_grouped_eligible(cplx, c->precision, c->dmap, c->dmap.ncomp * fa.nrhs, maxcoef)) {
-        CUDA_TRY(launch_i2o_grouped(cplx, c->precision, c->dmap, D.d, A.d, D.grp, maxcoef, fa, st));
-        return H2B_OK;
-    }
+    for (const PairTiles *pt : {&D.pairs, &D.pairs_small})
+        if (i2o_pairs_eligible(cplx, c->precision, c->dmap, c->dmap.ncomp * fa.nrhs, *pt, fa.prod_bytes)) {
+            CUDA_TRY(launch_i2o_pairs(cplx, c->precision, c->dmap, D.d, *pt, fa, D.maxcoef, st));
+            return H2B_OK;
+        }
     CUDA_TRY(launch_i2o(cplx, c->precision, c->dmap, D.d, A.d, D.d_recv, D.n_recv, fa,
                         maxcoef, maxt, D.maxhalf, st));
     return H2B_OK;
@@ -1405,7 +1460,7 @@ h2b_status far_passes_fa(h2b_core *c, const FarArgs &fa, const void *x, int64_t 
 h2b_status far_passes(h2b_workspace *ws, int mode, int nrhs, const void *x, int64_t ldx, void *y,
                       int64_t ldy, cdouble alpha_eff, cdouble beta, cudaStream_t st,
                       cudaEvent_t wait_before_scatter, PassTimer *tm = nullptr) {
-    const FarArgs fa{mode, nrhs, ws->am, ws->dm, ws->as, ws->ds};
+    const FarArgs fa{mode, nrhs, ws->am, ws->dm, ws->as, ws->ds, ws->prod, ws->prod_bytes};
     return far_passes_fa(ws->core, fa, x, ldx, y, ldy, alpha_eff, beta, st, wait_before_scatter, tm);
 }
 
@@ -1607,11 +1662,11 @@ h2b_status h2b_profile_matvec(h2b_workspace *ws, int32_t mode, int32_t nrhs, con
 // =============================================================================================
 namespace {
 
-// The scratch array (H2B_NOALLOC_SCRATCH_BYTES on every device that loads the library, until the
-// process exits). Device code may name it directly; host code must not pass `g_noalloc_scratch`
+// The scratch array (H2B_NOALLOC_SCRATCH_BYTES and the dense I2O's pair products behind them, on
+// every device that loads the library, until the process exits). Device code may name it directly; host code must not pass `g_noalloc_scratch`
 // itself to a kernel -- on the host that name is only a stand-in, not a device address -- and
 // asks the runtime for the address on each device instead (noalloc_scratch below).
-static __device__ __align__(256) unsigned char g_noalloc_scratch[H2B_NOALLOC_SCRATCH_BYTES];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[H2B_NOALLOC_SCRATCH_BYTES + NOALLOC_PRODUCT_BYTES];
 
 }  // namespace
 
@@ -1672,7 +1727,8 @@ extern "C" h2b_status h2b_farmul_noalloc(const h2b_core *core_in, int32_t mode, 
     // Nothing in the scratch needs clearing: every pass overwrites a moment or spectrum slot
     // before any pass reads it (leaf products and first-child / first-pair writes overwrite),
     // so whatever the previous call left there is never read.
-    FarArgs fa{mode, nrhs, b, b + mom, b + 2 * mom, b + 2 * mom + spec};
+    FarArgs fa{mode, nrhs, b, b + mom, b + 2 * mom, b + 2 * mom + spec, b + H2B_NOALLOC_SCRATCH_BYTES,
+               (size_t)NOALLOC_PRODUCT_BYTES};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const cdouble aA = c->alpha[mode];
     if (!alpha) {

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "../../include/h2b200.h"
 
 namespace h2b {
@@ -156,22 +158,24 @@ struct SibGroups {
     const int *kof = nullptr;          // [nentries*8] coupling offset of (source, slot), -1 if no pair
 };
 
-// Dense I2O for few right-hand sides, grouped by stored block. The receiving nodes are cut into
-// chunks of at most GT_R nodes of one level; a chunk's pairs are listed in tiles, each tile a run of
-// pairs that read the same stored (canonical) coupling block, from distinct receiving nodes. One CTA
-// per chunk stages a block once per tile and applies it to all of the tile's pairs (the symmetry
-// permutations act on the gathered moments and on the output rows), summing into the chunk's
-// receiving nodes in shared memory: each pair's block is read once per tile instead of once per pair.
-constexpr int GT_R = 16;  // receiving nodes per chunk
-constexpr int GT_P = 16;  // pairs per tile
-struct GroupTiles {
-    int nchunks = 0;
-    const int *chunk_ptr = nullptr;      // [nchunks+1] into rcv
-    const int *rcv = nullptr;            // receiving nodes, chunk by chunk
-    const int *tile_ptr = nullptr;       // [nchunks+1] into tile_pp
-    const int *tile_pp = nullptr;        // [ntiles+1] into pair / slot
-    const int *pair = nullptr;           // pair index (into the side's pair arrays)
-    const unsigned char *slot = nullptr; // receiving node of the pair as its position in the chunk
+// Dense I2O with FP64 sums (h2b_pairs.cu): the pairs of one receiving side in units of consecutive
+// receiving nodes, sorted inside a unit by the stored coupling block that they read (then by its
+// permutations), and cut into tiles of at most PAIR_TILE pairs of one block. A unit's products take
+// unit_elems scalars at most per right-hand side: pair p's at (p - p0) pstride.
+constexpr int PAIR_TILE = 64;
+struct PairUnit {
+    int tile0, ntiles;  // tiles of the unit
+    int maxpairs;       // pairs of its largest tile
+    int rcv0, nrcv;     // its receiving nodes
+    int p0;             // its first pair
+};
+struct PairTiles {
+    std::vector<PairUnit> units;  // host
+    const int *pair = nullptr;    // pair ids, tile by tile
+    const int4 *tile = nullptr;   // {first index into pair, pairs, rows, k}
+    const int *rcv = nullptr;     // receiving nodes, unit by unit
+    int64_t unit_elems = 0;
+    int pstride = 1;              // scalars per pair and right-hand side
 };
 
 // Per-call arguments of the far passes.
@@ -182,6 +186,8 @@ struct FarArgs {
     void *dm;     // disaggregation moments (T)
     void *as;     // aggregation spectra (complex of T's real)
     void *ds;     // disaggregation spectra
+    void *prod = nullptr;   // pair products of the dense I2O
+    size_t prod_bytes = 0;
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -216,15 +222,12 @@ cudaError_t copy_umma_timeouts_async(unsigned *host, cudaStream_t st);
 cudaError_t set_umma_wait_limit(unsigned limit);
 cudaError_t launch_i2o_siblings(bool cplx, int precision, const DMap &m, const DSide &recv,
                                 const SibGroups &g, int maxslen, const FarArgs &fa, cudaStream_t st);
-// The grouped dense I2O (GroupTiles) for W x nq <= GT_MAX_COLS field columns (W = 2 complex);
-// wider blocks take the tensor-core I2O (measured on a 65,536-point Laplace map, p = 6, FP32 form:
-// grouped 8.5 / 16.8 / 41.5 / 46.6 / 74.6 / 96.2 ms for 1-6 real right-hand sides against
-// 98 / 150 / 152 ms for the per-node tile kernel and 84 ms for the tcgen05 kernel from 4 columns
-// on; with 5 and 6 columns grouped, the batched-uneven pass did not change).
-constexpr int GT_MAX_COLS = 4;
-bool i2o_grouped_eligible(bool cplx, int precision, const DMap &m, int nq, int maxcoef);
-cudaError_t launch_i2o_grouped(bool cplx, int precision, const DMap &m, const DSide &recv, const DSide &src,
-                               const GroupTiles &gt, int maxcoef, const FarArgs &fa, cudaStream_t st);
+// The dense I2O by stored block (PairTiles) with FP64 sums: every FP64 map whose pair products fit
+// `prod_bytes`, and FP32 maps of at most PAIR_MAX_COLS32 field columns (W x nq, W = 2 complex).
+constexpr int PAIR_MAX_COLS32 = 4;
+bool i2o_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes);
+cudaError_t launch_i2o_pairs(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
+                             const FarArgs &fa, int maxcoef, cudaStream_t st);
 cudaError_t launch_transfer_down(bool cplx, int precision, const DMap &m, const DSide &s,
                                  const int *nodes, int nnodes, const uint8_t *received,
                                  const FarArgs &fa, int maxcoef, int maxsep, cudaStream_t st);

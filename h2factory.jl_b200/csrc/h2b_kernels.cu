@@ -1138,179 +1138,6 @@ __global__ void __launch_bounds__(512) i2o_kernel(DMap m, DSide r, DSide t, cons
 }
 
 // ---------------------------------------------------------------------------------------------
-// B1 for few right-hand sides, grouped by stored block (GroupTiles). One CTA per chunk of receiving
-// nodes of one level. For each run of pairs reading one stored block the block is staged in 64 x 32
-// pieces (cp.async, two stages: the next chunk's copies fly while the tensor cores work on this
-// one), each piece applied to up to GT_NB column blocks of TG_Q columns (pairs x right-hand sides)
-// on the FP64 tensor cores; each pair's symmetry permutation moves into the gather of its moments
-// (column permutation) and the row its products land on (row permutation), the canonical form of
-// symmetryreduceddense.jl:84-95. Products add into the chunk's sums in shared memory; the tiles
-// follow one another behind the tile product's block barriers, and within a tile every pair has
-// its own receiver, so no two threads add into one sum at once. The sums are written once at the
-// end (overwriting each receiving node's I2O output, as the per-node kernels do).
-// ---------------------------------------------------------------------------------------------
-// column blocks of TG_Q columns held at once per staged piece of a block (their FP64 fragments:
-// 4 doubles per block and lane for real sums, 8 for complex)
-template <class A> constexpr int gt_nb() { return sizeof(A) == 16 ? 4 : 8; }
-
-// element copy global -> shared (cp.async); ok = false writes zeros and reads nothing
-template <int EB>
-__device__ __forceinline__ void cp_async_elem(void *dst, const void *src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src), "n"(EB), "r"(ok ? EB : 0)
-                 : "memory");
-}
-
-template <class T>
-__global__ void __launch_bounds__(256)
-i2o_grouped_kernel(DMap m, DSide r, DSide t, GroupTiles gt, int mode, int nrhs, int maxcoef,
-                   const T *__restrict__ am, T *__restrict__ dm) {
-    using A = typename ScalarTraits<T>::Acc;
-    constexpr int GT_NB = gt_nb<A>();
-    constexpr int EB = sizeof(T);
-    constexpr int MS = TG_M * TG_LD, XS = GT_NB * TG_K * TG_Q;  // one stage of the block / moments
-    extern __shared__ unsigned char smem_raw[];
-    // the receivers' FP64 sums, then two stages of the block piece and the moments in the storage
-    // type (copied with cp.async one chunk ahead, widened when the products read them)
-    const int nq = m.ncomp * nrhs;
-    A *Sum = reinterpret_cast<A *>(smem_raw);
-    T *Mst = reinterpret_cast<T *>(Sum + GT_R * nq * maxcoef);
-    T *Xst = Mst + 2 * MS;
-    // per pair of the current run (slot b * TG_Q + j: pair j of column block b): its moments' offset,
-    // its permutation set (-1: none) and its receiver's position in the chunk
-    __shared__ int64_t run_src[GT_NB * TG_Q], run_perm[GT_NB * TG_Q];
-    __shared__ int run_slot[GT_NB * TG_Q];
-    const int ch = blockIdx.x;
-    const int r0 = gt.chunk_ptr[ch], nr = gt.chunk_ptr[ch + 1] - r0;
-    const int nc = ncoef_of(r, r.level[gt.rcv[r0]]);
-    const bool fwd = mode == H2B_FORWARD, adj = mode == H2B_ADJOINT;
-    const T *B0 = static_cast<const T *>(m.cpl);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
-    for (int o = threadIdx.x; o < nr * nq * nc; o += blockDim.x) Sum[o] = A{};
-    const int pq = TG_Q / nq;  // pairs per column block
-    const int t_end = gt.tile_ptr[ch + 1];
-    for (int tl = gt.tile_ptr[ch]; tl < t_end;) {
-        // a run of tiles reading one stored block, cut into column blocks of pq pairs (at most
-        // GT_NB): every block holds pairs of distinct receivers, since each tile does
-        const int pf = gt.pair[gt.tile_pp[tl]];
-        const int64_t key = r.pair_cpl[pf];
-        int bs[GT_NB], bn[GT_NB], nb = 0;  // first pair and pair count of each block
-        int tl2 = tl;
-        while (tl2 < t_end && r.pair_cpl[gt.pair[gt.tile_pp[tl2]]] == key) {
-            const int e0 = gt.tile_pp[tl2], e1 = gt.tile_pp[tl2 + 1];
-            const int need = (e1 - e0 + pq - 1) / pq;
-            if (nb + need > GT_NB) break;
-            for (int e = e0; e < e1; e += pq) {
-                bs[nb] = e;
-                bn[nb] = min(pq, e1 - e);
-                ++nb;
-            }
-            ++tl2;
-        }
-        tl = tl2;
-        const int snc = ncoef_of(t, t.level[r.i2o_src[pf]]);
-        const T *B = B0 + key;  // the run's stored block
-        __syncthreads();  // the previous run's stores have read its pair table
-        for (int j = threadIdx.x; j < GT_NB * TG_Q; j += blockDim.x) {
-            const int b = j / TG_Q, jj = j % TG_Q;
-            if (b < nb && jj < bn[b]) {
-                const int e = bs[b] + jj;
-                const int p = gt.pair[e];
-                run_src[j] = r.pair_src[p] * nrhs;
-                run_perm[j] = r.pair_perm ? r.pair_perm[p] : -1;
-                run_slot[j] = gt.slot[e];
-            }
-        }
-        __syncthreads();
-        const int nk = (snc + TG_K - 1) / TG_K;
-        for (int m0 = 0; m0 < nc; m0 += TG_M) {
-            const int mt = min(TG_M, nc - m0);
-            // chunk kc's copies into stage kc & 1: the block piece (forward reads the stored (r, t)
-            // block nc x snc down its columns, transposed orientations the stored (t, r) block
-            // snc x nc along k) and each column block's moments, read through the pair's column
-            // permutation (forward) or row permutation (transposed); past the block: zeros
-            auto issue = [&](int kc) {
-                const int k0 = kc * TG_K, kv = min(TG_K, snc - k0);
-                T *ms = Mst + (kc & 1) * MS;
-                if (fwd) {
-                    for (int idx = threadIdx.x; idx < mt * TG_K; idx += blockDim.x) {
-                        const int i = idx % mt, k = idx / mt;
-                        const bool ok = k < kv;
-                        cp_async_elem<EB>(ms + i * TG_LD + k, ok ? B + m0 + i + (int64_t)(k0 + k) * nc : B, ok);
-                    }
-                } else {
-                    for (int idx = threadIdx.x; idx < mt * TG_K; idx += blockDim.x) {
-                        const int k = idx % TG_K, i = idx / TG_K;
-                        const bool ok = k < kv;
-                        cp_async_elem<EB>(ms + i * TG_LD + k, ok ? B + k0 + k + (int64_t)(m0 + i) * snc : B, ok);
-                    }
-                }
-                T *xst = Xst + (kc & 1) * XS;
-                for (int b = 0; b < nb; ++b) {
-                    const int ncol = bn[b] * nq;
-                    T *xs = xst + b * TG_K * TG_Q;
-                    for (int idx = threadIdx.x; idx < TG_K * ncol; idx += blockDim.x) {
-                        const int k = idx % TG_K, c = idx / TG_K;
-                        const int j = b * TG_Q + c / nq;
-                        const bool ok = k < kv;
-                        const int64_t ps = run_perm[j];
-                        const int kk = !ok ? 0 : (ps < 0 ? k0 + k : m.perm[ps + (fwd ? 2 * snc : 0) + k0 + k]);
-                        cp_async_elem<EB>(xs + k * TG_Q + c, am + run_src[j] + (int64_t)(c % nq) * snc + kk, ok);
-                    }
-                }
-            };
-            MmaAcc<A> acc[GT_NB];
-#pragma unroll
-            for (int b = 0; b < GT_NB; ++b) acc[b].zero();
-            issue(0);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            for (int kc = 0; kc < nk; ++kc) {
-                if (kc + 1 < nk) issue(kc + 1);  // its stage was last read before the barrier below
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's chunk kc
-                __syncthreads();                                      // ... and everyone's
-                if (8 * warp < mt) {
-                    const T *mrow = Mst + (kc & 1) * MS + (8 * warp + g4) * TG_LD + t4;
-                    const T *xst = Xst + (kc & 1) * XS;
-#pragma unroll
-                    for (int k = 0; k < TG_K; k += 4) {
-                        const A a = wide(cj(mrow[k], adj));
-#pragma unroll
-                        for (int b = 0; b < GT_NB; ++b) {
-                            if (b < nb) {
-                                const T *xcol = xst + b * TG_K * TG_Q + (t4 + k) * TG_Q + g4;
-                                const A bb[2] = {wide(xcol[0]), wide(xcol[8])};
-                                acc[b].step(a, bb);
-                            }
-                        }
-                    }
-                }
-                __syncthreads();  // stage kc & 1 is free for chunk kc + 2
-            }
-            // the blocks' products into the receivers' sums, one block after another
-#pragma unroll
-            for (int b = 0; b < GT_NB; ++b) {
-                if (b < nb) {
-                    __syncthreads();
-                    mma_store(acc[b], mt, bn[b] * nq, [&](int i, int c, A v) {
-                        const int j = b * TG_Q + c / nq;
-                        const int64_t ps = run_perm[j];
-                        const int row = ps < 0 ? m0 + i : m.perm[ps + (fwd ? 0 : 2 * nc) + m0 + i];
-                        A &sum = Sum[(run_slot[j] * nq + c % nq) * nc + row];
-                        sum = sum + v;
-                    });
-                }
-            }
-        }
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o < nr * nq * nc; o += blockDim.x) {
-        const int ls = o / (nq * nc);
-        narrow(Sum[o], dm[r.mom_off[gt.rcv[r0 + ls]] * nrhs + o % (nq * nc)]);
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
 // B2 by sibling groups: the Toeplitz I2O of the receiving children of one parent together. One CTA
 // per (group, block of right-hand sides), one thread per stored frequency. The CTA walks the union
 // of the siblings' sources once; each source spectrum value is loaded once and applied from
@@ -1795,34 +1622,6 @@ cudaError_t launch_toeplitz_in(bool cplx, int precision, const DMap &m, const DS
         }
         err = cube7 ? launch(toeplitz_in_kernel<T, 7, 7>)
                     : (maxaxis <= 7 ? launch(toeplitz_in_kernel<T, 7, 0>) : launch(toeplitz_in_kernel<T, 15, 0>));
-    });
-    return err != cudaSuccess ? err : cudaGetLastError();
-}
-
-bool i2o_grouped_eligible(bool cplx, int precision, const DMap &m, int nq, int maxcoef) {
-    if (m.coupling_kind != H2B_COUPLING_DENSE || (cplx ? 2 : 1) * nq > GT_MAX_COLS) return false;
-    // the chunk's sums (FP64) and two stages of the block piece and the moments (storage type)
-    // fit in a CTA's shared memory
-    const size_t a = cplx ? sizeof(cdouble) : sizeof(double);
-    const size_t e = (cplx ? 2 : 1) * (precision == H2B_FP32 ? 4 : 8);
-    const size_t nb = cplx ? gt_nb<cdouble>() : gt_nb<double>();
-    return 2 * (TG_M * TG_LD + nb * TG_K * TG_Q) * e + (size_t)GT_R * nq * maxcoef * a <= 227u * 1024u - 4096u;
-}
-
-cudaError_t launch_i2o_grouped(bool cplx, int precision, const DMap &m, const DSide &recv, const DSide &src,
-                               const GroupTiles &gt, int maxcoef, const FarArgs &fa, cudaStream_t st) {
-    if (gt.nchunks == 0) return cudaSuccess;
-    const int nq = m.ncomp * fa.nrhs;
-    cudaError_t err = cudaSuccess;
-    H2B_DISPATCH_T(cplx, precision, {
-        using A = typename ScalarTraits<T>::Acc;
-        const size_t sm = (size_t)GT_R * nq * maxcoef * sizeof(A) +
-                          2 * (size_t)(TG_M * TG_LD + gt_nb<A>() * TG_K * TG_Q) * sizeof(T);
-        auto kern = &i2o_grouped_kernel<T>;
-        err = allow_smem(kern, sm);
-        if (err == cudaSuccess)
-            kern<<<gt.nchunks, 256, sm, st>>>(m, recv, src, gt, fa.mode, fa.nrhs, maxcoef,
-                                              static_cast<const T *>(fa.am), static_cast<T *>(fa.dm));
     });
     return err != cudaSuccess ? err : cudaGetLastError();
 }

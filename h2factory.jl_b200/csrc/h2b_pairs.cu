@@ -1,0 +1,288 @@
+// B1 dense I2O with FP64 sums: one matrix product per stored coupling block, then one sum per
+// receiving node.
+//
+// l_r = sum over the pairs of r of op(B_pair) m_src (translateintonode!,
+// src/farinteractions/traversalhelpers.jl:167-219, with applycouplingkernel! of
+// src/farinteractions/i2otranslations/i2otranslationcollection.jl:367-409 and the orientation rule
+// of i2oprotocol.jl:87-92). Many pairs read one stored block (a translation in a uniform tree, a
+// symmetry orbit of translations when the couplings are symmetry-reduced), so the pairs are sorted
+// by block when the core is built and the I2O runs as two launches:
+//   * i2o_pairs_kernel: the moments of a run of pairs are the columns of one matrix product with
+//     the block they share; every pair's product goes to its own column of a buffer;
+//   * i2o_pairs_sum_kernel: every receiving node adds its pairs' columns in list order (the same
+//     order on every call: no atomics) and writes its moments once.
+// The permutations of a symmetry-reduced pair (symmetryreduceddense.jl:84-95) move to the gather of
+// its moments (columns of the block) and to the row its sum reads (rows of the block), so pairs of
+// one orbit share a tile whatever their permutations are.
+//
+// What bounds it: the FP64 tensor cores (37 TFLOP/s here, mma.sync m8n8k4 .f64). A product reads
+// its block once per 64 columns and writes 16 bytes per complex sum (8 real) per row, read once by
+// the sums: 8.5 % of the time at 216 complex coefficients, about half at 64 real ones. Measured
+// (I2O per product, FP64): 65,536-point Helmholtz sphere, p = 6, 1 right-hand side 7.73 -> 1.12 ms;
+// 262,144 points, 32 right-hand sides 211 -> 134 ms (22 TFLOP/s); 8,192-point Laplace cube, p = 4,
+// unreduced blocks 2.56 -> 0.077 ms, against chunks of 16 receiving nodes that each staged every
+// block they read (1-4 field columns) and one CTA per receiving node (wider blocks).
+#include <algorithm>
+
+#include "h2b_internal.cuh"
+
+namespace h2b {
+
+namespace {
+
+constexpr int PK_THREADS = 256;
+constexpr int PK_WARPS = PK_THREADS / 32;
+constexpr int PK_N = PAIR_TILE;  // columns per tile: one 8-wide column block per warp
+// Rows per tile: at most 72, nine 8-row blocks, so that 216 coefficients (6^3) are three whole
+// tiles and 125 (5^3) two of 64; a warp then reuses each column fragment for nine products.
+constexpr int PK_MB = 9;
+constexpr int PK_STAGES = 4;
+
+// k per stage: 128 bytes per row (so two CTAs' stages fit an SM's shared memory), 32 bytes of
+// padding in front of the next row. The strides keep a fragment's 32 lanes (8 rows or columns x 4
+// k) on distinct banks: rows of KC + 4 elements where k is contiguous, columns of 72 + 4 (8-byte
+// elements), 72 + 2 (16-byte) or 72 + 0 (4-byte) elements where rows are.
+template <class T> struct PkGeom {
+    static constexpr int KC = sizeof(T) == 16 ? 8 : 16;
+    static constexpr int LDK = KC + 4;                                          // k contiguous
+    static constexpr int LDM = 8 * PK_MB + (sizeof(T) == 16 ? 2 : sizeof(T) == 8 ? 4 : 0);  // rows contiguous
+    static constexpr int ASZ = 8 * PK_MB * LDK > KC * LDM ? 8 * PK_MB * LDK : KC * LDM;
+    static constexpr int XSZ = PK_N * LDK;
+    static constexpr size_t BYTES = (size_t)PK_STAGES * (ASZ + XSZ) * sizeof(T);
+};
+
+__device__ __forceinline__ int pk_ncoef(const DSide &s, int lvl) {
+    return s.shape[3 * lvl] * s.shape[3 * lvl + 1] * s.shape[3 * lvl + 2];
+}
+
+// element copy global -> shared; ok = false writes zeros and reads nothing
+template <int EB>
+__device__ __forceinline__ void pk_copy(uint32_t dst, const void *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(EB), "r"(ok ? EB : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ void pk_dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// One 8 x 8 block of sums: lane holds C[lane / 4][2 (lane % 4) + h]; complex blocks take four real
+// products per step (re = ar br - ai bi, im = ar bi + ai br).
+template <class A> struct PkAcc;
+template <> struct PkAcc<double> {
+    double c[2];
+    __device__ __forceinline__ void zero() { c[0] = c[1] = 0.0; }
+    __device__ __forceinline__ void step(double a, double b) { pk_dmma(c, a, b); }
+    __device__ __forceinline__ double get(int h) const { return c[h]; }
+};
+template <> struct PkAcc<cdouble> {
+    double re[2], im[2];
+    __device__ __forceinline__ void zero() { re[0] = re[1] = im[0] = im[1] = 0.0; }
+    __device__ __forceinline__ void step(cdouble a, cdouble b) {
+        pk_dmma(re, a.x, b.x);
+        pk_dmma(im, a.x, b.y);
+        pk_dmma(re, -a.y, b.y);
+        pk_dmma(im, a.y, b.x);
+    }
+    __device__ __forceinline__ cdouble get(int h) const { return {re[h], im[h]}; }
+};
+
+// Tile blockIdx.x of the unit, row tile blockIdx.y, columns [64 blockIdx.z, + 64) of the tile's
+// pairs x qn right-hand sides (pair-major). FWD: the stored block is (receiver x source), rows
+// contiguous; otherwise it is the (source x receiver) block of the mirrored pair, read transposed
+// (conjugated for adjoint maps), k contiguous. Pair p's product for right-hand side q0 + q starts
+// at prod[((p - pbase) qn + q) pstride].
+template <class T, bool FWD>
+__global__ void __launch_bounds__(PK_THREADS, 2)
+i2o_pairs_kernel(DMap m, DSide r, const int *__restrict__ pair, const int4 *__restrict__ tile, int tile0, bool adj,
+                 int nrhs, int q0, int qn, int pbase, int pstride, const T *__restrict__ am,
+                 typename ScalarTraits<T>::Acc *__restrict__ prod) {
+    using A = typename ScalarTraits<T>::Acc;
+    using G = PkGeom<T>;
+    constexpr int KC = G::KC, EB = sizeof(T);
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    __shared__ int64_t col_src[PK_N], col_out[PK_N];  // per column: its moments and its product
+    __shared__ int64_t col_perm[PK_N];                // the permutation its moments are read through, -1: none
+    const int4 tl = tile[tile0 + blockIdx.x];         // {first pair, pairs, rows, k}
+    const int c0 = blockIdx.z * PK_N;
+    const int nc = tl.z, kk = tl.w;
+    const int nmt = (nc + 8 * PK_MB - 1) / (8 * PK_MB);      // row tiles of equal 8-row blocks
+    const int bm = 8 * ((nc + 8 * nmt - 1) / (8 * nmt));
+    const int m0 = blockIdx.y * bm;
+    if (c0 >= tl.y * qn || m0 >= nc) return;
+    const int ncol = min(PK_N, tl.y * qn - c0), mt = min(bm, nc - m0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const T *B = static_cast<const T *>(m.cpl) + r.pair_cpl[pair[tl.x]];
+    for (int c = tid; c < ncol; c += PK_THREADS) {
+        const int p = pair[tl.x + (c0 + c) / qn], q = (c0 + c) % qn;
+        col_src[c] = r.pair_src[p] * nrhs + (int64_t)(q0 + q) * kk;
+        col_out[c] = ((int64_t)(p - pbase) * qn + q) * pstride;
+        const int64_t ps = r.pair_perm ? r.pair_perm[p] : -1;
+        // sets [rowperm | rowperm^-1 | colperm | colperm^-1] of n each: forward products run over the
+        // block's columns (x read through colperm), transposed ones over its rows (rowperm)
+        col_perm[c] = ps < 0 ? -1 : ps + (FWD ? 2 * kk : 0);
+    }
+    __syncthreads();
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(pk_smem);
+    auto issue = [&](int kc) {
+        const int k0 = kc * KC, kv = min(KC, kk - k0);
+        const uint32_t as = smem + (uint32_t)((kc % PK_STAGES) * (G::ASZ + G::XSZ) * EB);
+        const uint32_t xs = as + (uint32_t)(G::ASZ * EB);
+        if constexpr (FWD) {
+            for (int e = tid; e < 8 * PK_MB * KC; e += PK_THREADS) {
+                const int k = e / (8 * PK_MB), i = e % (8 * PK_MB);
+                const bool ok = k < kv && i < mt;
+                if (i < bm) pk_copy<EB>(as + (uint32_t)((k * G::LDM + i) * EB), ok ? B + m0 + i + (int64_t)(k0 + k) * nc : B, ok);
+            }
+        } else {
+            for (int e = tid; e < 8 * PK_MB * KC; e += PK_THREADS) {
+                const int i = e / KC, k = e % KC;
+                const bool ok = k < kv && i < mt;
+                if (i < bm) pk_copy<EB>(as + (uint32_t)((i * G::LDK + k) * EB), ok ? B + k0 + k + (int64_t)(m0 + i) * kk : B, ok);
+            }
+        }
+        for (int e = tid; e < ncol * KC; e += PK_THREADS) {
+            const int c = e / KC, k = e % KC;
+            const bool ok = k < kv;
+            const int64_t ps = col_perm[c];
+            const int ks = !ok ? 0 : (ps < 0 ? k0 + k : __ldg(m.perm + ps + k0 + k));
+            pk_copy<EB>(xs + (uint32_t)((c * G::LDK + k) * EB), am + col_src[c] + ks, ok);
+        }
+    };
+    // warps over the tile's 8 x 8 blocks: one column block per warp and all row blocks, or, for
+    // narrow tiles, several warps per column block sharing its row blocks
+    const int nblk = (ncol + 7) / 8, mblk = (mt + 7) / 8;
+    const int wn = nblk > 4 ? 8 : (nblk > 2 ? 4 : (nblk > 1 ? 2 : 1)), wm = PK_WARPS / wn;
+    const int nb = warp % wn, mb0 = warp / wn;
+    const int g4 = lane >> 2, t4 = lane & 3;
+    PkAcc<A> acc[PK_MB];
+#pragma unroll
+    for (int j = 0; j < PK_MB; ++j) acc[j].zero();
+    const int nk = (kk + KC - 1) / KC;
+#pragma unroll
+    for (int s = 0; s < PK_STAGES - 1; ++s) {
+        if (s < nk) issue(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int kc = 0; kc < nk; ++kc) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(PK_STAGES - 2) : "memory");  // this thread's stage kc
+        __syncthreads();  // everyone's; and the stage issued next was read in the last step
+        if (kc + PK_STAGES - 1 < nk) issue(kc + PK_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (nb < nblk) {
+            const T *as = reinterpret_cast<const T *>(pk_smem) + (kc % PK_STAGES) * (G::ASZ + G::XSZ);
+            const T *xs = as + G::ASZ + (8 * nb + g4) * G::LDK + t4;
+#pragma unroll
+            for (int k = 0; k < KC; k += 4) {
+                const A b = wide(xs[k]);
+#pragma unroll
+                for (int j = 0; j < PK_MB; ++j) {
+                    const int mb = mb0 + j * wm;
+                    if (mb < mblk) {
+                        const int i = 8 * mb + g4;
+                        const T a = FWD ? as[(k + t4) * G::LDM + i] : as[i * G::LDK + k + t4];
+                        acc[j].step(wide(cj(a, adj)), b);
+                    }
+                }
+            }
+        }
+    }
+    if (nb >= nblk) return;
+#pragma unroll
+    for (int j = 0; j < PK_MB; ++j) {
+        const int i = 8 * (mb0 + j * wm) + g4;
+        if (i < mt) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * nb + 2 * t4 + h;
+                if (c < ncol) prod[col_out[c] + m0 + i] = acc[j].get(h);
+            }
+        }
+    }
+}
+
+// Receiving node nodes[blockIdx.x]: its moments for right-hand sides [q0, q0 + qn) as the sum of
+// its pairs' columns, read through each pair's row permutation. Loads of eight pairs are in flight
+// per thread; the sum runs in list order.
+template <class T>
+__global__ void __launch_bounds__(128)
+i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, int nrhs, int q0, int qn, int pbase,
+                     int pstride, const typename ScalarTraits<T>::Acc *__restrict__ prod, T *__restrict__ dm) {
+    using A = typename ScalarTraits<T>::Acc;
+    constexpr int U = 8;
+    const int node = nodes[blockIdx.x];
+    const int nc = pk_ncoef(r, r.level[node]);
+    const int e = blockIdx.y * 128 + threadIdx.x;
+    if (e >= nc * qn) return;
+    const int q = e / nc, i = e % nc;
+    const int p0 = r.i2o_ptr[node], p1 = r.i2o_ptr[node + 1];
+    // forward: out[i] += Y[rowperm^-1[i]]; transposed: out[j] += Y[colperm^-1[j]]
+    const int set = fwd ? nc : 3 * nc;
+    A sum = sc_zero<A>();
+    for (int p = p0; p < p1; p += U) {
+        A v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int pp = min(p + u, p1 - 1);
+            const int64_t ps = r.pair_perm ? __ldg(r.pair_perm + pp) : -1;
+            const int row = ps < 0 ? i : __ldg(m.perm + ps + set + i);
+            v[u] = prod[((int64_t)(pp - pbase) * qn + q) * pstride + row];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (p + u < p1) sum = sum + v[u];
+    }
+    narrow(sum, dm[r.mom_off[node] * nrhs + (int64_t)(q0 + q) * nc + i]);
+}
+
+template <class T>
+cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, const FarArgs &fa, int maxcoef,
+                           cudaStream_t st) {
+    using A = typename ScalarTraits<T>::Acc;
+    const bool fwd = fa.mode == H2B_FORWARD, adj = fa.mode == H2B_ADJOINT;
+    const int nq = m.ncomp * fa.nrhs;
+    const size_t sm = PkGeom<T>::BYTES;
+    auto kern = fwd ? &i2o_pairs_kernel<T, true> : &i2o_pairs_kernel<T, false>;
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (err != cudaSuccess) return err;
+    // right-hand sides per pass: as many as the largest unit's products leave room for
+    const int64_t unit = pt.unit_elems * (int64_t)sizeof(A);
+    // (and as the grids' second and third extents allow)
+    const int qc = (int)std::min<int64_t>(std::min(nq, 1024), (int64_t)fa.prod_bytes / unit);
+    const int mtiles = (maxcoef + 8 * PK_MB - 1) / (8 * PK_MB);
+    A *prod = static_cast<A *>(fa.prod);
+    for (const PairUnit &u : pt.units)
+        for (int q0 = 0; q0 < nq; q0 += qc) {
+            const int qn = std::min(qc, nq - q0);
+            const dim3 grid(u.ntiles, mtiles, (u.maxpairs * qn + PK_N - 1) / PK_N);
+            kern<<<grid, PK_THREADS, sm, st>>>(m, r, pt.pair, pt.tile, u.tile0, adj, fa.nrhs, q0, qn, u.p0, pt.pstride,
+                                               static_cast<const T *>(fa.am), prod);
+            const dim3 gs(u.nrcv, ((int64_t)maxcoef * qn + 127) / 128);
+            i2o_pairs_sum_kernel<T><<<gs, 128, 0, st>>>(m, r, pt.rcv + u.rcv0, fwd, fa.nrhs, q0, qn, u.p0, pt.pstride,
+                                                        prod, static_cast<T *>(fa.dm));
+        }
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+bool i2o_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes) {
+    if (pt.units.empty() || m.coupling_kind != H2B_COUPLING_DENSE) return false;
+    // the FP32 form's products have FP64 sums up to PAIR_MAX_COLS32 field columns; wider blocks take
+    // the tcgen05 kernel
+    if (precision == H2B_FP32 && (cplx ? 2 : 1) * nq > PAIR_MAX_COLS32) return false;
+    return (int64_t)prod_bytes >= pt.unit_elems * (int64_t)(cplx ? sizeof(cdouble) : sizeof(double));
+}
+
+cudaError_t launch_i2o_pairs(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
+                             const FarArgs &fa, int maxcoef, cudaStream_t st) {
+    if (!cplx)
+        return precision == H2B_FP64 ? launch_pairs_t<double>(m, recv, pt, fa, maxcoef, st)
+                                     : launch_pairs_t<float>(m, recv, pt, fa, maxcoef, st);
+    return precision == H2B_FP64 ? launch_pairs_t<cdouble>(m, recv, pt, fa, maxcoef, st)
+                                 : launch_pairs_t<cfloat>(m, recv, pt, fa, maxcoef, st);
+}
+
+}  // namespace h2b

@@ -338,7 +338,8 @@ h2b_status h2b_nearmul(h2b_workspace *ws, int32_t mode, int32_t nrhs, const void
  * another allocator (a framework's caching pool that holds the GPU), a real-time loop that
  * forbids allocation after start-up, or a binding that cannot create and keep a workspace.
  * Instead of a workspace's moment and spectrum arenas it uses one scratch array compiled into
- * the library (H2B_NOALLOC_SCRATCH_BYTES per device, held by every GPU that loads the library
+ * the library (H2B_NOALLOC_SCRATCH_BYTES per device for the arenas and 4 MiB behind them for the
+ * dense I2O's pair products, held by every GPU that loads the library
  * until the process exits). Same semantics as h2b_farmul on `core`.
  *
  * Limits and rules:
