@@ -91,8 +91,7 @@ struct SideHost {
     int n_init_leaves = 0;
     int64_t npairs = 0;
     SibGroups sib;                      // Toeplitz I2O by sibling groups (ngroups = 0: per node)
-    PairTiles pairs;                    // dense I2O by stored block, products in a workspace's buffer
-    PairTiles pairs_small;              // the same in small units, for h2b_farmul_noalloc
+    std::vector<PairTiles> pairs;       // dense I2O by stored block: plans of ever smaller units
     int maxslen = 1;
     std::vector<int64_t> mom_off_host;  // moment offsets per unit rhs (host copy)
     std::vector<int64_t> spec_off_host; // spectrum offsets per unit rhs (host copy)
@@ -484,20 +483,23 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
     return H2B_OK;
 }
 
-// A unit's pair products take at most this much of a workspace per right-hand side, and a workspace's
-// buffer holds as many right-hand sides as fit in it.
+// A workspace's buffer of pair products, and the units of the dense I2O (PairTiles) that it is used
+// with: plans whose units take at most these shares of it per right-hand side, so that a wide block
+// runs all its right-hand sides in one pass over smaller units. The last one is also what
+// h2b_farmul_noalloc's buffer holds.
 constexpr int64_t PAIR_BUFFER_BYTES = 256ll << 20;
-// the pair products of h2b_farmul_noalloc, beside its scratch
-constexpr int64_t NOALLOC_PRODUCT_BYTES = 4 << 20;
+constexpr int PAIR_PLANS[] = {1, 4, 16, 64};
+constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 64;
 
-// Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of side `s`,
-// a unit's products taking at most `unit_bytes` per right-hand side. Left empty (per-node kernel)
-// when one receiving node's products alone exceed that.
-h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, const h2b_side_desc &s, const h2b_side_desc &other,
-                            const std::vector<int64_t> &cpl_elem_off, const std::vector<int64_t> &perm_set,
-                            int64_t unit_bytes, PairTiles &out) {
+// Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of one side, a
+// plan for each share of PAIR_PLANS that cuts them differently. A plan is left out when one receiving
+// node's products alone exceed its units.
+h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, const std::vector<int64_t> &cpl_elem_off,
+                            const std::vector<int64_t> &perm_set, std::vector<PairTiles> &plans) {
+    const h2b_side_desc &s = test_side ? d.test : d.trial, &other = test_side ? d.trial : d.test;
     const int np = s.i2o_ptr[s.nnodes];
     if (np == 0) return H2B_OK;
+    const int W = c->field == H2B_COMPLEX ? 2 : 1;
     // every pair's key {block, rows, k, permutations}: one per coupling, unless a coupling is used
     // with two shapes
     struct Key { int64_t off, perm; int nc, snc; };
@@ -534,53 +536,109 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, const h2b_side_d
     for (size_t i = 0; i < keys.size(); ++i) rank[order[i]] = (int)i;
     for (int p = 0; p < np; ++p) key[p] = rank[key[p]];
 
-    const int64_t max_pairs = unit_bytes / ((c->field == H2B_COMPLEX ? 16 : 8) * (int64_t)pstride);
-    std::vector<int> pair(np), count;
-    std::vector<int4> tile;
-    std::vector<PairUnit> units;
-    int64_t most = 0;
-    for (size_t i = 0; i < recv.size();) {
-        const size_t i0 = i;
-        const int p0 = s.i2o_ptr[recv[i]];
-        while (i < recv.size() && s.i2o_ptr[recv[i] + 1] - p0 <= max_pairs) ++i;
-        if (i == i0) return H2B_OK;
-        const int p1 = s.i2o_ptr[recv[i - 1] + 1];
-        most = std::max<int64_t>(most, p1 - p0);
-        // the unit's pairs by key, in list order within a key
-        if ((size_t)(p1 - p0) >= keys.size() / 8) {
-            count.assign(keys.size() + 1, 0);
-            for (int p = p0; p < p1; ++p) ++count[key[p] + 1];
-            for (size_t k = 0; k < keys.size(); ++k) count[k + 1] += count[k];
-            for (int p = p0; p < p1; ++p) pair[p0 + count[key[p]]++] = p;
-        } else {
-            for (int p = p0; p < p1; ++p) pair[p] = p;
-            std::sort(pair.begin() + p0, pair.begin() + p1,
-                      [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
-        }
-        PairUnit u{(int)tile.size(), 0, 0, (int)i0, (int)(i - i0), p0};
-        for (int a = p0; a < p1;) {
-            const Key &k = keys[order[key[pair[a]]]];
-            int b = a + 1;
-            while (b < p1 && same_block(keys[order[key[pair[b]]]], k)) ++b;
-            const int nt = (b - a + PAIR_TILE - 1) / PAIR_TILE;  // tiles of the run, of equal pairs
-            for (int t = 0; t < nt; ++t) {
-                const int e0 = a + (int)((int64_t)(b - a) * t / nt), e1 = a + (int)((int64_t)(b - a) * (t + 1) / nt);
-                tile.push_back(make_int4(e0, e1 - e0, k.nc, k.snc));
-                u.maxpairs = std::max(u.maxpairs, e1 - e0);
+    // the FP32 form's tensor-core tiles: every block's chunks of 32 FP32 values of K pair up into
+    // accumulation segments (an odd count would carry a segment from one pair into the next)
+    PairTiles base;
+    bool tensor = c->precision == H2B_FP32 && d.coupling_kind == H2B_COUPLING_DENSE;
+    for (const Key &k : keys) tensor &= ((W * k.snc + 31) / 32) % 2 == 0;
+    // their blocks, rows x k: as stored (or the transposed copy) where the columns are whole 16 bytes,
+    // else copied with padded columns; per key (in order) the block's offset
+    std::vector<int64_t> off32(keys.size(), 0);
+    if (tensor && c->dmap.cpl_vec) {
+        base.blocks32 = test_side ? c->dmap.cpl : c->dmap.cpl_t;
+        for (size_t i = 0; i < keys.size(); ++i) off32[i] = keys[order[i]].off;
+    } else if (tensor) {
+        std::vector<float> blocks;
+        for (size_t i = 0; i < keys.size(); ++i) {
+            const Key &k = keys[order[i]];
+            if (i > 0 && same_block(k, keys[order[i - 1]])) {
+                off32[i] = off32[i - 1];
+                continue;
             }
-            a = b;
+            const int V = 4 / W, ld = (k.nc + V - 1) / V * V;
+            off32[i] = (int64_t)blocks.size() / W;
+            blocks.resize(blocks.size() + (size_t)ld * k.snc * W, 0.0f);
+            float *dst = blocks.data() + off32[i] * W;
+            const double *src = d.coupling + k.off * W;
+            for (int j = 0; j < k.snc; ++j)
+                for (int r = 0; r < k.nc; ++r)
+                    for (int w = 0; w < W; ++w)
+                        dst[((int64_t)j * ld + r) * W + w] =
+                            (float)src[(test_side ? r + (int64_t)j * k.nc : j + (int64_t)r * k.snc) * W + w];
         }
-        u.ntiles = (int)tile.size() - u.tile0;
-        units.push_back(u);
+        float *fp;
+        CUDA_TRY(c->upload(&fp, blocks.data(), blocks.size()));
+        base.blocks32 = fp;
     }
     int *q;
-    int4 *t4;
-    CUDA_TRY(c->upload(&q, pair.data(), pair.size())); out.pair = q;
-    CUDA_TRY(c->upload(&q, recv.data(), recv.size())); out.rcv = q;
-    CUDA_TRY(c->upload(&t4, tile.data(), tile.size())); out.tile = t4;
-    out.units = units;
-    out.unit_elems = most * pstride;
-    out.pstride = pstride;
+    CUDA_TRY(c->upload(&q, recv.data(), recv.size()));
+    base.rcv = q;
+    base.pstride = pstride;
+    for (int share : PAIR_PLANS) {
+        const int64_t max_pairs = PAIR_BUFFER_BYTES / share / (8 * W * (int64_t)pstride);
+        if (!plans.empty() && plans.back().units.size() == 1 && np <= max_pairs) continue;  // the same plan again
+        PairTiles out = base;
+        std::vector<int> pair(np), count;
+        std::vector<int4> tile, tile32;
+        std::vector<int64_t> tile32_off;
+        int64_t most = 0;
+        bool fits = true;
+        for (size_t i = 0; i < recv.size();) {
+            const size_t i0 = i;
+            const int p0 = s.i2o_ptr[recv[i]];
+            while (i < recv.size() && s.i2o_ptr[recv[i] + 1] - p0 <= max_pairs) ++i;
+            if (!(fits = i > i0)) break;
+            const int p1 = s.i2o_ptr[recv[i - 1] + 1];
+            most = std::max<int64_t>(most, p1 - p0);
+            // the unit's pairs by key, in list order within a key
+            if ((size_t)(p1 - p0) >= keys.size() / 8) {
+                count.assign(keys.size() + 1, 0);
+                for (int p = p0; p < p1; ++p) ++count[key[p] + 1];
+                for (size_t k = 0; k < keys.size(); ++k) count[k + 1] += count[k];
+                for (int p = p0; p < p1; ++p) pair[p0 + count[key[p]]++] = p;
+            } else {
+                for (int p = p0; p < p1; ++p) pair[p] = p;
+                std::sort(pair.begin() + p0, pair.begin() + p1,
+                          [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
+            }
+            PairUnit u{(int)tile.size(), 0, 0, (int)tile32.size(), 0, 0, (int)i0, (int)(i - i0), p0};
+            // runs of pairs for which same(other, first) holds, each cut into tiles of equal pairs
+            auto cut = [&](std::vector<int4> &to, int &maxpairs, auto same, auto each) {
+                for (int a = p0; a < p1;) {
+                    const int ka = key[pair[a]];
+                    const Key &k = keys[order[ka]];
+                    int b = a + 1;
+                    while (b < p1 && (key[pair[b]] == ka || same(keys[order[key[pair[b]]]], k))) ++b;
+                    const int nt = (b - a + PAIR_TILE - 1) / PAIR_TILE;
+                    for (int t = 0; t < nt; ++t) {
+                        const int e0 = a + (int)((int64_t)(b - a) * t / nt), e1 = a + (int)((int64_t)(b - a) * (t + 1) / nt);
+                        to.push_back(make_int4(e0, e1 - e0, k.nc, k.snc));
+                        each(ka);
+                        maxpairs = std::max(maxpairs, e1 - e0);
+                    }
+                    a = b;
+                }
+            };
+            cut(tile, u.maxpairs, same_block, [](int) {});
+            if (tensor)
+                cut(tile32, u.maxpairs32, [&](const Key &x, const Key &y) { return same_block(x, y) && x.perm == y.perm; },
+                    [&](int ka) { tile32_off.push_back(off32[ka]); });
+            u.ntiles = (int)tile.size() - u.tile0;
+            u.ntiles32 = (int)tile32.size() - u.tile32_0;
+            out.units.push_back(u);
+        }
+        if (!fits) break;  // nor will smaller units hold that receiving node
+        int4 *t4;
+        CUDA_TRY(c->upload(&q, pair.data(), pair.size())); out.pair = q;
+        CUDA_TRY(c->upload(&t4, tile.data(), tile.size())); out.tile = t4;
+        if (tensor) {
+            int64_t *o;
+            CUDA_TRY(c->upload(&t4, tile32.data(), tile32.size())); out.tile32 = t4;
+            CUDA_TRY(c->upload(&o, tile32_off.data(), tile32_off.size())); out.tile32_off = o;
+        }
+        out.unit_elems = most * pstride;
+        plans.push_back(out);
+    }
     return H2B_OK;
 }
 
@@ -1149,16 +1207,7 @@ h2b_status build_core(h2b_core *c, const h2b_map_desc &d) {
             st = build_sibling_groups(c, sd, h, o.spec_off_host, off);
             if (st) return st;
         } else if (d.coupling_kind == H2B_COUPLING_DENSE) {
-            const h2b_side_desc &so = side == 0 ? d.trial : d.test;
-            st = build_pair_tiles(c, d, sd, so, off, perm_set, PAIR_BUFFER_BYTES, h.pairs);
-            if (st) return st;
-            // h2b_farmul_noalloc: only maps whose moments can fit its scratch ever take it
-            const int64_t far = (c->precision == H2B_FP64 ? 8 : 4) * (cplx ? 2 : 1);
-            const int64_t sum = cplx ? 16 : 8;
-            if (h.pairs.unit_elems * sum <= NOALLOC_PRODUCT_BYTES && h.pairs.units.size() == 1)
-                h.pairs_small = h.pairs;
-            else if (2 * std::max(c->test.mom_total, c->trial.mom_total) * far <= (int64_t)H2B_NOALLOC_SCRATCH_BYTES)
-                st = build_pair_tiles(c, d, sd, so, off, perm_set, NOALLOC_PRODUCT_BYTES, h.pairs_small);
+            st = build_pair_tiles(c, d, side == 0, off, perm_set, h.pairs);
             if (st) return st;
         }
     }
@@ -1307,13 +1356,14 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
     if (e == cudaSuccess) e = al(&ws->as, spec * ssz);
     if (e == cudaSuccess) e = al(&ws->ds, spec * ssz);
     // pair products of the dense I2O: all right-hand sides of its largest unit, within the buffer's
-    // bound (the FP32 form takes that path up to PAIR_MAX_COLS32 field columns only)
-    const int64_t cols = core->precision == H2B_FP64
-                             ? (int64_t)max_nrhs * core->dmap.ncomp
-                             : std::min<int64_t>((int64_t)max_nrhs * core->dmap.ncomp, PAIR_MAX_COLS32 / (cplx ? 2 : 1));
+    // bound (the FP32 form without tensor-core tiles takes that path up to PAIR_MAX_COLS32 field
+    // columns only)
     for (const SideHost *h : {&core->test, &core->trial}) {
-        const int64_t unit = h->pairs.unit_elems * (int64_t)vsz;
-        ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min(unit * cols, std::max(unit, PAIR_BUFFER_BYTES)));
+        if (h->pairs.empty()) continue;
+        int64_t cols = (int64_t)max_nrhs * core->dmap.ncomp;
+        if (core->precision == H2B_FP32 && !h->pairs[0].tile32) cols = std::min<int64_t>(cols, PAIR_MAX_COLS32 / (cplx ? 2 : 1));
+        const int64_t unit = h->pairs[0].unit_elems * (int64_t)vsz;
+        ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min(unit * cols, PAIR_BUFFER_BYTES));
     }
     if (e == cudaSuccess) e = al(&ws->prod, ws->prod_bytes);
     if (e == cudaSuccess) e = al(&ws->xbuf, ndof * vsz);
@@ -1370,11 +1420,22 @@ h2b_status run_i2o(h2b_core *c, const SideHost &D, const SideHost &A, const FarA
         return H2B_OK;
     }
     const bool cplx = c->field == H2B_COMPLEX;
-    for (const PairTiles *pt : {&D.pairs, &D.pairs_small})
-        if (i2o_pairs_eligible(cplx, c->precision, c->dmap, c->dmap.ncomp * fa.nrhs, *pt, fa.prod_bytes)) {
-            CUDA_TRY(launch_i2o_pairs(cplx, c->precision, c->dmap, D.d, *pt, fa, D.maxcoef, st));
-            return H2B_OK;
-        }
+    // the plan of the largest units whose products fit the buffer for all right-hand sides at once, else
+    // the smallest units, some right-hand sides at a time
+    const int nq = c->dmap.ncomp * fa.nrhs;
+    const PairTiles *pt = nullptr;
+    for (const PairTiles &t : D.pairs) {
+        pt = &t;
+        if ((size_t)t.unit_elems * (cplx ? 16 : 8) * nq <= fa.prod_bytes) break;
+    }
+    if (pt && i2o_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
+        CUDA_TRY(launch_i2o_pairs(cplx, c->precision, c->dmap, D.d, *pt, fa, D.maxcoef, st));
+        return H2B_OK;
+    }
+    if (pt && i2o_umma_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
+        CUDA_TRY(launch_i2o_umma_pairs(cplx, c->dmap, D.d, *pt, fa, D.maxcoef, st));
+        return H2B_OK;
+    }
     CUDA_TRY(launch_i2o(cplx, c->precision, c->dmap, D.d, A.d, D.d_recv, D.n_recv, fa,
                         maxcoef, maxt, D.maxhalf, st));
     return H2B_OK;

@@ -166,6 +166,7 @@ constexpr int PAIR_TILE = 64;
 struct PairUnit {
     int tile0, ntiles;  // tiles of the unit
     int maxpairs;       // pairs of its largest tile
+    int tile32_0, ntiles32, maxpairs32;  // the same of tile32
     int rcv0, nrcv;     // its receiving nodes
     int p0;             // its first pair
 };
@@ -174,6 +175,12 @@ struct PairTiles {
     const int *pair = nullptr;    // pair ids, tile by tile
     const int4 *tile = nullptr;   // {first index into pair, pairs, rows, k}
     const int *rcv = nullptr;     // receiving nodes, unit by unit
+    // FP32 form on the tcgen05 tensor cores: tiles of pairs that read one block through one
+    // permutation, the element offset of each one's block in `blocks32` (rows x k, column-major, columns
+    // padded to whole 16 bytes: the stored blocks forward, their transposes for the other orientations)
+    const int4 *tile32 = nullptr;
+    const int64_t *tile32_off = nullptr;
+    const void *blocks32 = nullptr;
     int64_t unit_elems = 0;
     int pstride = 1;              // scalars per pair and right-hand side
 };
@@ -214,6 +221,13 @@ cudaError_t launch_toeplitz_out(bool cplx, int precision, const DMap &m, const D
 bool i2o_umma_eligible(bool cplx, int precision, const DMap &m, int nq);
 cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const DSide &src, const int *nodes,
                             int nnodes, const FarArgs &fa, int maxcoef, cudaStream_t st);
+// The sums of one unit's pair products (right-hand sides [q0, q0 + qn)) into the receiving nodes' moments.
+cudaError_t launch_i2o_pairs_sum(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
+                                 const PairUnit &u, const FarArgs &fa, int maxcoef, int q0, int qn, cudaStream_t st);
+// The FP32 form's dense I2O by stored block on the tcgen05 tensor cores (PairTiles::tile32).
+bool i2o_umma_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes);
+cudaError_t launch_i2o_umma_pairs(bool cplx, const DMap &m, const DSide &recv, const PairTiles &pt, const FarArgs &fa,
+                                  int maxcoef, cudaStream_t st);
 // mbarrier waits of the tensor-core kernels that gave up on the current device (0 in a healthy run)
 cudaError_t read_umma_timeouts(unsigned *count);
 // the same count copied to host memory in order on `st`

@@ -238,6 +238,15 @@ i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, i
 }
 
 template <class T>
+void launch_sum_t(const DMap &m, const DSide &r, const PairTiles &pt, const PairUnit &u, const FarArgs &fa, int maxcoef,
+                  int q0, int qn, cudaStream_t st) {
+    using A = typename ScalarTraits<T>::Acc;
+    const dim3 grid(u.nrcv, (unsigned)(((int64_t)maxcoef * qn + 127) / 128));
+    i2o_pairs_sum_kernel<T><<<grid, 128, 0, st>>>(m, r, pt.rcv + u.rcv0, fa.mode == H2B_FORWARD, fa.nrhs, q0, qn, u.p0,
+                                                  pt.pstride, static_cast<const A *>(fa.prod), static_cast<T *>(fa.dm));
+}
+
+template <class T>
 cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, const FarArgs &fa, int maxcoef,
                            cudaStream_t st) {
     using A = typename ScalarTraits<T>::Acc;
@@ -259,9 +268,7 @@ cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, c
             const dim3 grid(u.ntiles, mtiles, (u.maxpairs * qn + PK_N - 1) / PK_N);
             kern<<<grid, PK_THREADS, sm, st>>>(m, r, pt.pair, pt.tile, u.tile0, adj, fa.nrhs, q0, qn, u.p0, pt.pstride,
                                                static_cast<const T *>(fa.am), prod);
-            const dim3 gs(u.nrcv, ((int64_t)maxcoef * qn + 127) / 128);
-            i2o_pairs_sum_kernel<T><<<gs, 128, 0, st>>>(m, r, pt.rcv + u.rcv0, fwd, fa.nrhs, q0, qn, u.p0, pt.pstride,
-                                                        prod, static_cast<T *>(fa.dm));
+            launch_sum_t<T>(m, r, pt, u, fa, maxcoef, q0, qn, st);
         }
     return cudaGetLastError();
 }
@@ -283,6 +290,15 @@ cudaError_t launch_i2o_pairs(bool cplx, int precision, const DMap &m, const DSid
                                      : launch_pairs_t<float>(m, recv, pt, fa, maxcoef, st);
     return precision == H2B_FP64 ? launch_pairs_t<cdouble>(m, recv, pt, fa, maxcoef, st)
                                  : launch_pairs_t<cfloat>(m, recv, pt, fa, maxcoef, st);
+}
+
+cudaError_t launch_i2o_pairs_sum(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
+                                 const PairUnit &u, const FarArgs &fa, int maxcoef, int q0, int qn, cudaStream_t st) {
+    if (!cplx && precision == H2B_FP64) launch_sum_t<double>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
+    else if (!cplx) launch_sum_t<float>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
+    else if (precision == H2B_FP64) launch_sum_t<cdouble>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
+    else launch_sum_t<cfloat>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
+    return cudaGetLastError();
 }
 
 }  // namespace h2b

@@ -20,10 +20,9 @@
 //   * moment warps (4-6): cp.async each chunk's source moments into a raw shared-memory ring four
 //     chunks ahead, then write them as the B operand, TF32 high parts plus remainders, in the
 //     canonical no-swizzle K-major layout (a complex piece is split once for its two rows);
-//   * one MMA thread (warp 11): per 8-wide k step the products hi*hi + hi*lo + lo*hi (the lo*lo
+//   * one MMA warp (warp 11): per 8-wide k step the products hi*hi + hi*lo + lo*hi (the lo*lo
 //     term is below FP32 rounding), N = 64 columns each, into an FP32 accumulator in tensor memory;
-//     one commit per chunk releases both operand stages. A tcgen05.mma costs its issuing thread
-//     about 50 cycles whatever its N (measured), so products are made as wide as the block allows;
+//     one commit per chunk releases both operand stages;
 //   * drain warps (7-10, one per tensor-memory lane quarter): the tensor cores round each
 //     accumulation toward zero, so one FP32 accumulator over a whole interaction list loses ~1e-4;
 //     accumulators live for 64 values of K (2 chunks) only, two alternate, and each finished one is
@@ -40,6 +39,8 @@
 // (h2b_tensor_wait_timeouts) and sets the CTA's abort flag; every role then leaves its loop, the
 // MMA thread waits (with the full bound) for the products it issued, the moment warps for their
 // copies, and the CTA frees its tensor memory and returns with its output tile unwritten.
+
+#include <algorithm>
 
 #include "h2b_internal.cuh"
 
@@ -122,19 +123,32 @@ __device__ __forceinline__ void split2(float x, uint32_t &hi, uint32_t &lo) {
     lo = tf32_bits(x - __uint_as_float(hi));
 }
 
-// D (+)= A (tensor memory) * B (shared memory), kind::tf32
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+// D (+)= A (tensor memory) * B (shared memory), kind::tf32, and the commit of the products so far.
+// One lane of a converged warp, as a predicate for the two calls below. The whole warp runs the issuing
+// loop and only the instruction is predicated: its operands then stay in uniform registers, and a
+// product costs 10 cycles to issue (32 at N = 64, the tensor cores' own rate) against 45 from a branch
+// that one lane took (measured, M = 128, tensor-memory A).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
 }
-
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(bar))
-                 : "memory");
+__device__ __forceinline__ void umma_ts_if(uint32_t elected, uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(elected));
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t elected, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(su32(bar)),
+        "r"(elected)
+        : "memory");
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
@@ -735,45 +749,553 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
                 }
             }
         }
-    } else if (lane == 0) {
-        // ---------------- MMA thread: six products of N = np columns per chunk ----------------
-        const uint32_t idesc = tf32_idesc(UM_M, np);
+    } else {
+        // ---------------- MMA warp: twelve products of N = np columns per chunk ----------------
+        const uint32_t idesc = tf32_idesc(UM_M, np), el = elect_one();
+        const uint64_t desc0 = kmajor_desc(smem0);
         for (int c = 0; c < C; ++c) {
             const int s = c % UM_NS, g = c / UM_SEG, a = g & 1;
-            if (c % UM_SEG == 0 && g >= 2 && !mbar_wait(&acc_empty[a], ((g >> 1) - 1) & 1, limit)) abort_s = 1;
-            if (!abort_s && !mbar_wait(&a_full[s], (c / UM_NS) & 1, limit)) abort_s = 1;
-            if (!abort_s && !mbar_wait(&b_full[s], (c / UM_NS) & 1, limit)) abort_s = 1;
-            if (abort_s) break;
+            if (c % UM_SEG == 0 && g >= 2 && !warp_wait(&acc_empty[a], ((g >> 1) - 1) & 1, limit)) abort_s = 1;
+            if (!warp_aborted(&abort_s) && !warp_wait(&a_full[s], (c / UM_NS) & 1, limit)) abort_s = 1;
+            if (!warp_aborted(&abort_s) && !warp_wait(&b_full[s], (c / UM_NS) & 1, limit)) abort_s = 1;
+            if (warp_aborted(&abort_s)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d = tmem + (uint32_t)(a * np);
             const uint32_t ta = tmem + col_a + (uint32_t)s * (2u * UM_KC);
-            const uint32_t bh = smem0 + (uint32_t)s * b_stage_bytes, bl = bh + (uint32_t)np * (UM_KC * 4);
+            const uint64_t bh = desc0 + (uint64_t)(((uint32_t)s * b_stage_bytes) >> 4);
+            const uint64_t bl = bh + (uint64_t)(((uint32_t)np * (UM_KC * 4)) >> 4);
 #pragma unroll
             for (int j = 0; j < UM_KC / 8; ++j) {
-                const uint64_t dbh = kmajor_desc(bh + (uint32_t)j * 2 * UM_LBO);
-                const uint64_t dbl = kmajor_desc(bl + (uint32_t)j * 2 * UM_LBO);
-                const uint32_t first = (c % UM_SEG != 0 || j > 0) ? 1u : 0u;
-                umma_ts(d, ta + 8u * j, dbh, idesc, first);
-                umma_ts(d, ta + 8u * j, dbl, idesc, 1u);
-                umma_ts(d, ta + UM_KC + 8u * j, dbh, idesc, 1u);
+                const uint64_t dbh = bh + (uint64_t)((j * 2 * UM_LBO) >> 4), dbl = bl + (uint64_t)((j * 2 * UM_LBO) >> 4);
+                umma_ts_if(el, d, ta + 8u * j, dbh, idesc, (c % UM_SEG != 0 || j > 0) ? 1u : 0u);
+                umma_ts_if(el, d, ta + 8u * j, dbl, idesc, 1u);
+                umma_ts_if(el, d, ta + UM_KC + 8u * j, dbh, idesc, 1u);
             }
-            umma_commit(&empty[s]);
-            if (c % UM_SEG == UM_SEG - 1 || c == C - 1) umma_commit(&acc_full[a]);
+            umma_commit_if(el, &empty[s]);
+            if (c % UM_SEG == UM_SEG - 1 || c == C - 1) umma_commit_if(el, &acc_full[a]);
         }
+        umma_commit_if(el, &fin);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();  // every role has left its loop
-    if (warp == UM_WARPS - 1 && lane == 0) {
-        // products already issued (all of them, after a wait gave up) may still read the operand
-        // stages and write tensor memory: the issuing thread waits for them, with the full bound,
-        // before the CTA frees its memory
-        umma_commit(&fin);
-        mbar_wait(&fin, 0, UM_SPIN_FINAL);
-    }
+    // products already issued (all of them, after a wait gave up) may still read the operand stages and
+    // write tensor memory: they are waited for, with the full bound, before the CTA frees its memory
+    if (warp == UM_WARPS - 1 && lane == 0) mbar_wait(&fin, 0, UM_SPIN_FINAL);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same products by stored block: one tile of the pairs that read one block through one column
+// permutation (PairTiles::tile32) instead of one receiving node, so the split of a block's chunk
+// into TF32 parts serves all the columns of a tile (pairs x right-hand sides, packed without gaps)
+// instead of one pair's, and no column of the product is padding. Per (tile, 128 of the block's
+// rows, 64 product columns) item a persistent CTA runs the pipeline above over the K values of the
+// block; chunks, segments and the order of the products inside them are those of i2o_umma_kernel
+// (an item's chunk count is even, so no segment spans two pairs there either), hence the same FP32
+// segment sums. Each pair's FP64 sum goes to its column of the pair-product buffer; the row
+// permutation is left to i2o_pairs_sum_kernel, so the rows of a tile are contiguous in the block.
+//
+// What bounds it: the roles' instruction latency, about 1,400 cycles per chunk against 384 for its
+// products (ncu: 0.54 instructions per scheduler and cycle, DRAM 5 %, L2 15 %). Measured (I2O per
+// product, 65,536-point Helmholtz sphere, p = 6): 8 right-hand sides 14.2 -> 4.2 ms, 32 right-hand
+// sides 15.1 -> 14.7 ms against one receiving node per CTA. Roles (24 warps, six warpgroups):
+//   * scheduler: turns the CTA's items into records in a ring (the block, and every column's moments
+//     and product), so that no other role chases the plan's arrays;
+//   * two copy warps: the rows of each chunk's columns into a ring of UP_AR stages, 16 bytes per lane
+//     (cp.async: a bulk copy costs its issuing warp about 100 cycles per column, and a chunk has 16);
+//   * eight coupling warps, four per chunk in turn: read, split, write to tensor memory;
+//   * four moment warps, one chunk each in turn: cp.async its moments a turn ahead, split them into
+//     shared memory; operand stages hold a whole segment (two chunks), so the MMA thread waits once
+//     per 24 products;
+//   * MMA thread; eight drain warps, which keep the FP64 sums (32 each) in registers: the kernel starts
+//     with 80 registers a thread and moves them to the drain warps (setmaxnreg; 256 threads each at 72,
+//     64 and 104 make the 240 x 256 that the block was launched with).
+// ---------------------------------------------------------------------------------------------
+constexpr int UP_N = 64;                  // product columns per item
+constexpr int UP_NS = 3;                  // operand stages, one accumulation segment each
+template <int W> constexpr int up_ar() { return W == 2 ? 4 : 3; }  // coupling column stages
+// Item records: a moment warp that splits a chunk of record n has its copy cursor one turn (four
+// chunks) past the next turn's, at most four records of two chunks ahead, before it is done with n.
+constexpr int UP_IR = 8;
+constexpr int UP_B0 = 8, UP_COPY = 12, UP_MMA = 14, UP_SCHED = 15, UP_D0 = 16;  // first warps of the roles
+constexpr int UP_WARPS = 24, UP_THREADS = UP_WARPS * 32;
+constexpr int UP_BW = UP_COPY - UP_B0;    // moment warps
+constexpr int UP_RS = 2 * UP_BW;          // raw moment stages: two per moment warp
+constexpr int UP_READERS = UP_WARPS - 1;  // warps that read the item records
+static_assert(UM_SEG == 2, "an operand stage holds two chunks, one per half of the coupling warps");
+constexpr int UP_REG_A = 72, UP_REG_B = 64, UP_REG_D = 104;
+static_assert(UP_BW == 2 * UM_SEG && UP_NS * UM_SEG > UP_BW, "two moment warps fill a stage");
+
+// elements of a block's column as stored for the column copies: whole 16 bytes
+template <class T> __host__ __device__ constexpr int up_ld(int nc) {
+    return (nc + 16 / (int)sizeof(T) - 1) / (16 / (int)sizeof(T)) * (16 / (int)sizeof(T));
+}
+
+struct UpArgs {
+    const int *pair;
+    const int4 *tile;          // {first index into pair, pairs, rows, k}
+    const int64_t *tile_off;   // element offset of the tile's block
+    int tile0, ntiles, zt, mt; // tiles of the unit; column tiles and row tiles per tile (at most)
+    int mode, nrhs, q0, qn, pbase, pstride;
+};
+
+template <int NC> struct UpItem {
+    int nk, ncol, snc, rows, ld;  // nk = 0: no more items
+    int64_t blk;                  // the item's first row in `blocks`
+    int64_t perm;                 // k -> stored column in DMap::perm, -1: identity
+    int64_t src[NC], out[NC];     // per column: its moments, its product (at the item's first row)
+};
+
+// mbar_wait (for a whole warp, with one outcome, when WARP) that also ends (false, uncounted) once the CTA has given up: the flag is
+// read only after an attempt that found the phase incomplete, so a wait that finds it complete costs
+// one instruction
+template <bool WARP> __device__ __forceinline__ bool up_wait(uint64_t *bar, uint32_t parity, unsigned limit, volatile int *abort) {
+    const uint32_t a = su32(bar);
+    uint32_t done = 0;
+    unsigned it = 0;
+    for (; it < limit; ++it) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(a), "r"(parity), "n"(UM_SUSPEND_NS)
+            : "memory");
+        if (done || *abort) break;
+    }
+    if (it == limit && !done) atomicAdd(&g_umma_timeouts, 1u);
+    if constexpr (WARP) return __all_sync(0xffffffffu, done != 0);
+    return done != 0;
+}
+
+__device__ __forceinline__ void cp16_cg(uint32_t dst, const void *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+// store_split without the conjugation (the moment warps apply it) and with values past the block
+// zeroed only in its last, partial chunk
+template <int W>
+__device__ __forceinline__ void up_store_split(uint32_t ta, const float (&v)[UM_KC], int kv) {
+#pragma unroll
+    for (int h = 0; h < UM_KC / 16; ++h) {
+        uint32_t hi[16], lo[16];
+        if (kv >= UM_KC / W) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) split2(v[16 * h + e], hi[e], lo[e]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) split2((16 * h + e) / W < kv ? v[16 * h + e] : 0.0f, hi[e], lo[e]);
+        }
+        tmem_st16(ta + 16u * h, hi);
+        tmem_st16(ta + UM_KC + 16u * h, lo);
+    }
+    tmem_wait_st();
+}
+
+// product rows of one part (real, imaginary) of `ncol` columns: MMA N is a multiple of 16
+template <int W> __device__ __forceinline__ int up_part(int ncol) {
+    return W == 2 ? (ncol + 7) & ~7 : (ncol + 15) & ~15;
+}
+
+template <class T>
+__global__ void __launch_bounds__(UP_THREADS, 1)
+i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, const T *__restrict__ am,
+                      typename ScalarTraits<T>::Acc *__restrict__ prod) {
+    constexpr int W = UmScalar<T>::W;
+    constexpr int EB = sizeof(T);
+    constexpr int KQ = UM_KC / W;       // elements along k per chunk
+    constexpr int NC = UP_N / W;        // columns (pairs x right-hand sides) per item
+    constexpr uint32_t B_CHUNK = 2u * UP_N * UM_KC * 4, B_STAGE = UM_SEG * B_CHUNK;  // per chunk: hi then lo
+    constexpr uint32_t RAW_STAGE = (uint32_t)NC * UM_RAWROW;
+    constexpr uint32_t A_COL = UM_M * EB, A_STAGE = KQ * A_COL;
+    constexpr uint32_t COL_A = 2 * UP_N;  // tensor memory: two accumulators, then the coupling stages
+    extern __shared__ __align__(128) unsigned char um_smem[];
+    constexpr int UP_AR = up_ar<W>();
+    __shared__ uint64_t full[UP_NS], empty[UP_NS], ar_full[UP_AR], ar_empty[UP_AR];
+    __shared__ uint64_t acc_full[2], acc_empty[2], it_full[UP_IR], it_empty[UP_IR], fin;
+    __shared__ UpItem<NC> rec[UP_IR];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_s;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool fwd = g.mode == H2B_FORWARD, adj = g.mode == H2B_ADJOINT;
+    const unsigned limit = g_umma_wait_limit;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tmem_slot)), "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < UP_NS; ++s) {
+            mbar_init(&full[s], 256 + 32 * UM_SEG);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&acc_empty[a], 256);
+        }
+        for (int a = 0; a < UP_AR; ++a) {
+            mbar_init(&ar_full[a], 64);
+            mbar_init(&ar_empty[a], 128);
+        }
+        for (int a = 0; a < UP_IR; ++a) {
+            mbar_init(&it_full[a], 1);
+            mbar_init(&it_empty[a], UP_READERS);
+        }
+        mbar_init(&fin, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        abort_s = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const uint32_t smem0 = su32(um_smem);
+    const uint32_t raw0 = smem0 + UP_NS * B_STAGE;
+    const uint32_t araw0 = raw0 + ((UP_RS * RAW_STAGE + 127u) & ~127u);
+    // record n of the ring, for a whole warp; false when the wait gave up
+    auto wait = [&](uint64_t *bar, uint32_t parity) -> bool { return up_wait<true>(bar, parity, limit, &abort_s); };
+    auto item = [&](int n) -> bool { return wait(&it_full[n % UP_IR], (n / UP_IR) & 1); };
+    auto item_done = [&](int n) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&it_empty[n % UP_IR]);
+    };
+
+    if (warp < UP_B0) {
+        // ---------------- coupling warps: one tile row per thread, alternate chunks ----------------
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(UP_REG_A));
+        const int grp = warp >> 2, row = tid & 127;
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        int c = 0;  // chunks of the items before this one
+        bool run = true;
+        for (int n = 0; run; ++n) {
+            if (!(run = item(n))) break;
+            const UpItem<NC> &it = rec[n % UP_IR];
+            const int nk = it.nk, snc = it.snc;
+            if (nk == 0) break;
+            // (rows past the tile split whatever their stage holds: their products are never stored)
+            for (int k = grp; k < nk; k += 2) {
+                const int cc = c + k, st = cc % UP_AR, sg = cc / UM_SEG, s = sg % UP_NS;
+                if (!(run = wait(&ar_full[st], (cc / UP_AR) & 1))) break;
+                const uint32_t src = araw0 + (uint32_t)st * A_STAGE + (uint32_t)row * EB;
+                float v[UM_KC];
+#pragma unroll
+                for (int j = 0; j < KQ; ++j) {
+                    if constexpr (W == 2) {
+                        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                                     : "=f"(v[2 * j]), "=f"(v[2 * j + 1])
+                                     : "r"(src + (uint32_t)j * A_COL));
+                    } else {
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[j]) : "r"(src + (uint32_t)j * A_COL));
+                    }
+                }
+                mbar_arrive(&ar_empty[st]);
+                if (sg >= UP_NS && !(run = wait(&empty[s], ((sg / UP_NS) - 1) & 1))) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                up_store_split<W>(tl + COL_A + (uint32_t)(s * UM_SEG + grp) * (2u * UM_KC), v, snc - k * KQ);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive(&full[s]);
+            }
+            c += nk;
+            item_done(n);
+        }
+        if (!run) abort_s = 1;
+    } else if (warp < UP_D0) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(UP_REG_B));
+        if (warp < UP_COPY) {
+            // ---------------- moment warps: B operand into shared memory ----------------
+            // warp bw takes every fourth chunk on its own: copies it one turn ahead, waits for its own
+            // copies only and splits the whole chunk, so nothing but the operand stages ties the warps
+            const int bw = warp - UP_B0;
+            constexpr int EV = 16 / EB;  // elements per 16-byte piece
+            const uint32_t S = 0x80000000u, s_re = adj ? 0u : S, s_im = adj ? S : 0u;
+            int in = 0, ik = bw, turn = 0;  // copy cursor: record, chunk of it, chunks copied
+            bool run = item(0), more = run;
+            // moves the cursor to the next record with a chunk for this warp (at once: a record is
+            // reused after its last chunk)
+            auto enter = [&]() {
+                while (more && rec[in % UP_IR].nk != 0 && ik >= rec[in % UP_IR].nk) {
+                    ik -= rec[in % UP_IR].nk;
+                    more = run = item(++in);
+                }
+                more = more && rec[in % UP_IR].nk != 0;
+            };
+            auto copy = [&]() {
+                const UpItem<NC> &it = rec[in % UP_IR];
+                const uint32_t rb = raw0 + (uint32_t)(2 * bw + (turn & 1)) * RAW_STAGE;
+                const int ncol = it.ncol, snc = it.snc, ncp = up_part<W>(ncol);
+                const int kg = lane & 7, kp = ik * KQ + kg * EV;
+#pragma unroll
+                for (int u = 0; u < NC / 4; ++u) {
+                    const int q = (lane >> 3) + 4 * u;
+                    const uint32_t dst = rb + (uint32_t)q * UM_RAWROW + (uint32_t)kg * 16;
+                    if (q < ncol) {
+                        const int64_t o = it.src[q] + kp;
+                        if (kp + EV <= snc && o % EV == 0) {
+                            cp16_cg(dst, am + o, true);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < EV; ++e) {
+                                const bool ok = kp + e < snc;
+                                cp_elem<EB>(dst + (uint32_t)(e * EB), ok ? am + o + e : am, ok);
+                            }
+                        }
+                    } else if (q < ncp) {
+                        cp16_cg(dst, am, false);
+                    }
+                }
+                ++turn;
+                ik += UP_BW;
+            };
+            enter();
+            if (more) copy();
+            enter();
+            cp_commit_group();
+            int c = 0;  // chunks of the records before record n
+            for (int n = 0, done = 0; run; ++n) {
+                if (!(run = item(n))) break;
+                const UpItem<NC> &it = rec[n % UP_IR];
+                const int nk = it.nk, ncp = up_part<W>(it.ncol);
+                if (nk == 0) break;
+                for (int k = (bw - c) & (UP_BW - 1); k < nk; k += UP_BW, ++done) {
+                    if (more) copy();  // the next turn's, into the stage of the turn before this one
+                    enter();
+                    if (!run) break;
+                    cp_commit_group();
+                    cp_wait_group<1>();
+                    __syncwarp();
+                    const int cc = c + k, sg = cc / UM_SEG, s = sg % UP_NS;
+                    if (sg >= UP_NS && !(run = wait(&empty[s], ((sg / UP_NS) - 1) & 1))) break;
+                    const uint32_t rb = raw0 + (uint32_t)(2 * bw + (done & 1)) * RAW_STAGE;
+                    const uint32_t hb = smem0 + (uint32_t)s * B_STAGE + (uint32_t)(cc % UM_SEG) * B_CHUNK;
+                    const uint32_t lb = hb + UP_N * UM_KC * 4;
+                    // lane: column (and column + 32 of a real tile)
+#pragma unroll
+                    for (int g2 = 0; g2 < NC / 32; ++g2) {
+                        const int q = lane + 32 * g2;
+                        if (q >= ncp) continue;
+                        const uint32_t o0 = goff(q, 0), oi0 = W == 2 ? goff(ncp + q, 0) : 0;
+#pragma unroll
+                        for (int kg = 0; kg < UM_KG; ++kg) {
+                            float w[4];
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
+                                         : "r"(rb + (uint32_t)q * UM_RAWROW + (uint32_t)kg * 16));
+                            uint32_t h[4], l[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) split2(w[e], h[e], l[e]);
+                            const uint32_t o = o0 + (uint32_t)kg * UM_LBO;
+                            if constexpr (W == 1) {
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb + o), "r"(h[0]),
+                                             "r"(h[1]), "r"(h[2]), "r"(h[3]));
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb + o), "r"(l[0]),
+                                             "r"(l[1]), "r"(l[2]), "r"(l[3]));
+                            } else {
+                                // Re row (mr, -mi), Im row (mi, mr); conjugated blocks: (mr, mi), (mi, -mr)
+                                const uint32_t oi = oi0 + (uint32_t)kg * UM_LBO;
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb + o), "r"(h[0]),
+                                             "r"(h[1] ^ s_re), "r"(h[2]), "r"(h[3] ^ s_re));
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb + o), "r"(l[0]),
+                                             "r"(l[1] ^ s_re), "r"(l[2]), "r"(l[3] ^ s_re));
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb + oi), "r"(h[1]),
+                                             "r"(h[0] ^ s_im), "r"(h[3]), "r"(h[2] ^ s_im));
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(lb + oi), "r"(l[1]),
+                                             "r"(l[0] ^ s_im), "r"(l[3]), "r"(l[2] ^ s_im));
+                            }
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    mbar_arrive(&full[s]);
+                    __syncwarp();  // the stage of this turn is copied into in the next one
+                }
+                c += nk;
+                if (run) item_done(n);
+            }
+            if (!run) abort_s = 1;
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        } else if (warp < UP_MMA) {
+            // ---------------- copy warps: the rows of a chunk's columns, UP_AR chunks ahead ----------------
+            const int cw = warp - UP_COPY;  // this warp copies every other column
+            constexpr int PC = (int)A_COL / 512;  // warp copies (32 x 16 bytes) per column
+            int c = 0;
+            bool run = true;
+            for (int n = 0; run; ++n) {
+                if (!(run = item(n))) break;
+                const UpItem<NC> &it = rec[n % UP_IR];
+                const int nk = it.nk, snc = it.snc, ld = it.ld;
+                if (nk == 0) break;
+                const int *kmap = it.perm >= 0 ? m.perm + it.perm : nullptr;
+                const int bytes = it.rows * EB;  // a column's last 16 bytes may reach into its padding
+                const unsigned char *B = reinterpret_cast<const unsigned char *>(blocks + it.blk) + 16 * lane;
+                int col = lane < min(KQ, snc) ? (kmap ? __ldg(kmap + lane) : lane) : 0;
+                for (int k = 0; k < nk; ++k, ++c) {
+                    const int nv = min(KQ, snc - k * KQ), next = (k + 1) * KQ + lane;
+                    // the next chunk's columns, while this one's stage is waited for and filled
+                    const int coln = lane < KQ && next < snc ? (kmap ? __ldg(kmap + next) : next) : 0;
+                    const int st = c % UP_AR;
+                    int off[KQ / 2];  // byte offsets of this warp's columns
+#pragma unroll
+                    for (int j = 0; j < KQ / 2; ++j) off[j] = __shfl_sync(0xffffffffu, col, 2 * j + cw) * (ld * EB);
+                    if (c >= UP_AR && !(run = wait(&ar_empty[st], ((c / UP_AR) - 1) & 1))) break;
+                    const uint32_t dst = araw0 + (uint32_t)st * A_STAGE + 16u * lane + (uint32_t)cw * A_COL;
+#pragma unroll
+                    for (int h = 0; h < PC; ++h)
+                        if (16 * lane + 512 * h < bytes) {
+#pragma unroll
+                            for (int j = 0; j < KQ / 2; ++j)
+                                if (2 * j + cw < nv)
+                                    cp16_cg(dst + (uint32_t)(2 * j) * A_COL + 512u * h, B + off[j] + 512 * h, true);
+                        }
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(su32(&ar_full[st])) : "memory");
+                    col = coln;
+                }
+                item_done(n);
+            }
+            if (!run) abort_s = 1;
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        } else if (warp == UP_MMA) {
+            // ---------------- MMA warp: converged, one lane issues ----------------
+            int sg = 0;  // segments so far
+            bool run = true;
+            const uint32_t el = elect_one();
+            const uint64_t desc0 = kmajor_desc(smem0);
+            for (int n = 0; run; ++n) {
+                if (!(run = item(n))) break;
+                const int ns = rec[n % UP_IR].nk / UM_SEG;
+                if (ns == 0) break;
+                const uint32_t idesc = tf32_idesc(UM_M, W * up_part<W>(rec[n % UP_IR].ncol));
+                for (int k = 0; k < ns; ++k, ++sg) {
+                    const int s = sg % UP_NS, a = sg & 1;
+                    if (sg >= 2 && !(run = wait(&acc_empty[a], ((sg >> 1) - 1) & 1))) break;
+                    if (!(run = wait(&full[s], (sg / UP_NS) & 1))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t d = tmem + (uint32_t)(a * UP_N);
+                    const uint32_t ta = tmem + COL_A + (uint32_t)s * (UM_SEG * 2u * UM_KC);
+                    const uint64_t db = desc0 + (uint64_t)((uint32_t)s * (B_STAGE >> 4));
+#pragma unroll
+                    for (int j = 0; j < UM_SEG * UM_KC / 8; ++j) {
+                        const int h = j / (UM_KC / 8), i = j % (UM_KC / 8);  // chunk of the segment, its k step
+                        const uint64_t dbh = db + (uint64_t)((h * B_CHUNK + i * 2 * UM_LBO) >> 4);
+                        const uint64_t dbl = dbh + (uint64_t)((UP_N * UM_KC * 4) >> 4);
+                        const uint32_t ah = ta + (uint32_t)(h * 2 * UM_KC + 8 * i);
+                        umma_ts_if(el, d, ah, dbh, idesc, j > 0 ? 1u : 0u);
+                        umma_ts_if(el, d, ah, dbl, idesc, 1u);
+                        umma_ts_if(el, d, ah + UM_KC, dbh, idesc, 1u);
+                    }
+                    umma_commit_if(el, &empty[s]);
+                    umma_commit_if(el, &acc_full[a]);
+                }
+                item_done(n);
+            }
+            if (!run) abort_s = 1;
+            umma_commit_if(el, &fin);  // products already issued may still read the operands (see the end)
+        } else if (warp == UP_SCHED) {
+            // ---------------- scheduler: item records ----------------
+            const int items = g.ntiles * g.mt * g.zt;
+            int n = 0;
+            bool run = true;
+            for (int id = blockIdx.x; run; id += gridDim.x) {
+                const bool end = id >= items;
+                // column tiles slowest: every tile has a first one, fewer have the later ones, and a stride
+                // of the grid's CTAs meets them evenly
+                const int m0 = (id % g.mt) * UM_M, rest = id / g.mt, t = g.tile0 + rest % g.ntiles, z = rest / g.ntiles;
+                int4 tl = make_int4(0, 0, 0, 0);
+                if (!end) {
+                    tl = __ldg(g.tile + t);
+                    if (z * NC >= tl.y * g.qn || m0 >= tl.z) continue;
+                }
+                UpItem<NC> &it = rec[n % UP_IR];
+                if (n >= UP_IR && !(run = wait(&it_empty[n % UP_IR], ((n / UP_IR) - 1) & 1))) break;
+                if (!end) {
+                    const int ncol = min(NC, tl.y * g.qn - z * NC);
+                    for (int c = lane; c < ncol; c += 32) {
+                        const int f = z * NC + c, p = __ldg(g.pair + tl.x + f / g.qn), q = f % g.qn;
+                        it.src[c] = __ldg(r.pair_src + p) * g.nrhs + (int64_t)(g.q0 + q) * tl.w;
+                        it.out[c] = ((int64_t)(p - g.pbase) * g.qn + q) * g.pstride + m0;
+                    }
+                    if (lane == 0) {
+                        it.ncol = ncol;
+                        it.snc = tl.w;
+                        it.rows = min(UM_M, tl.z - m0);
+                        it.ld = up_ld<T>(tl.z);
+                        it.blk = __ldg(g.tile_off + t) + m0;
+                        // k -> stored column: the column permutation inverted forward, else the row permutation
+                        const int64_t ps = r.pair_perm ? __ldg(r.pair_perm + __ldg(g.pair + tl.x)) : -1;
+                        it.perm = ps < 0 ? -1 : ps + (fwd ? 3 * tl.w : tl.w);
+                    }
+                }
+                if (lane == 0) it.nk = end ? 0 : (W * tl.w + UM_KC - 1) / UM_KC;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&it_full[n % UP_IR]);
+                ++n;
+                if (end) break;
+            }
+            if (!run) abort_s = 1;
+        }
+    } else {
+        // ---------------- drain warps: FP64 sums of the segments, then the pairs' columns ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(UP_REG_D));
+        const int row = 32 * (warp & 3) + lane, half = (warp - UP_D0) >> 2;
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        constexpr int HC = NC / 2;  // columns of this warp: 16 complex or 32 real
+        int gs = 0;  // segments so far
+        bool run = true;
+        for (int n = 0; run; ++n) {
+            if (!(run = item(n))) break;
+            const UpItem<NC> &it = rec[n % UP_IR];
+            const int nk = it.nk, ncol = it.ncol;
+            if (nk == 0) break;
+            const bool mine = half * HC < ncol;
+            // first part: the columns' real (or only) sums, second: the imaginary ones / columns 16-31
+            const uint32_t part0 = (uint32_t)(half * HC);
+            const uint32_t part1 = W == 2 ? (uint32_t)(up_part<W>(ncol) + half * HC) : part0 + 16u;
+            double sum[2][16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) sum[0][e] = sum[1][e] = 0.0;
+            for (int k = 0; k < nk; k += UM_SEG, ++gs) {
+                const int a = gs & 1;
+                if (!(run = wait(&acc_full[a], (gs >> 1) & 1))) break;
+                if (mine) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t f[16];
+                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part0, f);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[0][e] += (double)__uint_as_float(f[e]);
+                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part1, f);
+                    tmem_wait_ld();
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(&acc_empty[a]);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[1][e] += (double)__uint_as_float(f[e]);
+                } else {
+                    mbar_arrive(&acc_empty[a]);
+                }
+            }
+            if (!run) break;
+            if (row < it.rows) {
+#pragma unroll
+                for (int e = 0; e < HC; ++e) {
+                    const int c = half * HC + e;
+                    if (c >= ncol) break;
+                    if constexpr (W == 2) prod[it.out[c] + row] = cdouble{sum[0][e], sum[1][e]};
+                    else prod[it.out[c] + row] = sum[e / 16][e % 16];
+                }
+            }
+            item_done(n);
+        }
+        if (!run) abort_s = 1;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();  // every role has left its loop
+    // products already issued may still read the operands and write tensor memory
+    if (warp == UP_MMA && lane == 0) mbar_wait(&fin, 0, UM_SPIN_FINAL);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
 bool i2o_umma_eligible(bool cplx, int precision, const DMap &m, int nq) {
@@ -819,6 +1341,47 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
     if (cplx)
         return go(&i2o_umma_kernel<cfloat>, static_cast<const cfloat *>(fa.am), static_cast<cfloat *>(fa.dm));
     return go(&i2o_umma_kernel<float>, static_cast<const float *>(fa.am), static_cast<float *>(fa.dm));
+}
+
+bool i2o_umma_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes) {
+    return i2o_umma_eligible(cplx, precision, m, nq) && pt.tile32 && !pt.units.empty() &&
+           (int64_t)prod_bytes >= pt.unit_elems * (int64_t)(cplx ? sizeof(cdouble) : sizeof(double));
+}
+
+cudaError_t launch_i2o_umma_pairs(bool cplx, const DMap &m, const DSide &recv, const PairTiles &pt, const FarArgs &fa,
+                                  int maxcoef, cudaStream_t st) {
+    const int nq = m.ncomp * fa.nrhs;
+    int dev = 0, nsm = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess) return err;
+    const int cols = UP_N / (cplx ? 2 : 1);
+    const size_t raw = ((size_t)UP_RS * cols * UM_RAWROW + 127) & ~(size_t)127;
+    const size_t smem = (size_t)UP_NS * UM_SEG * 2 * UP_N * UM_KC * 4 + raw +
+                        (size_t)(cplx ? up_ar<2>() : up_ar<1>()) * UM_KC * 4 * UM_M;
+    auto go = [&](auto kern, const auto *blocks, const auto *am, auto *prod) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        const int64_t unit = pt.unit_elems * (int64_t)sizeof(*prod);
+        const int qc = (int)std::min<int64_t>(std::min(nq, 1024), (int64_t)fa.prod_bytes / unit);
+        for (const PairUnit &u : pt.units)
+            for (int q0 = 0; q0 < nq; q0 += qc) {
+                const int qn = std::min(qc, nq - q0);
+                UpArgs g{pt.pair, pt.tile32, pt.tile32_off, u.tile32_0, u.ntiles32, (u.maxpairs32 * qn + cols - 1) / cols,
+                         (maxcoef + UM_M - 1) / UM_M, fa.mode, fa.nrhs, q0, qn, u.p0, pt.pstride};
+                const int64_t items = (int64_t)g.ntiles * g.zt * g.mt;
+                if (items > INT32_MAX) return cudaErrorInvalidValue;
+                kern<<<(unsigned)std::min<int64_t>(nsm, items), UP_THREADS, smem, st>>>(m, recv, g, blocks, am, prod);
+                e = launch_i2o_pairs_sum(cplx, H2B_FP32, m, recv, pt, u, fa, maxcoef, q0, qn, st);
+                if (e != cudaSuccess) return e;
+            }
+        return cudaGetLastError();
+    };
+    if (cplx)
+        return go(&i2o_umma_pairs_kernel<cfloat>, static_cast<const cfloat *>(pt.blocks32),
+                  static_cast<const cfloat *>(fa.am), static_cast<cdouble *>(fa.prod));
+    return go(&i2o_umma_pairs_kernel<float>, static_cast<const float *>(pt.blocks32), static_cast<const float *>(fa.am),
+              static_cast<double *>(fa.prod));
 }
 
 cudaError_t read_umma_timeouts(unsigned *count) {
