@@ -495,7 +495,8 @@ constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 64;
 // plan for each share of PAIR_PLANS that cuts them differently. A plan is left out when one receiving
 // node's products alone exceed its units.
 h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, const std::vector<int64_t> &cpl_elem_off,
-                            const std::vector<int64_t> &perm_set, std::vector<PairTiles> &plans) {
+                            const std::vector<int64_t> &perm_set, const std::vector<int64_t> &other_mom_off,
+                            std::vector<PairTiles> &plans) {
     const h2b_side_desc &s = test_side ? d.test : d.trial, &other = test_side ? d.trial : d.test;
     const int np = s.i2o_ptr[s.nnodes];
     if (np == 0) return H2B_OK;
@@ -527,6 +528,8 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
             key[p] = *id;
         }
     }
+    for (const Key &k : keys)
+        if (k.perm > INT32_MAX - 4 * (int64_t)std::max(k.nc, k.snc)) return H2B_OK;  // sets in 32 bits
     std::vector<int> order(keys.size()), rank(keys.size());
     for (size_t i = 0; i < keys.size(); ++i) order[i] = (int)i;
     std::sort(order.begin(), order.end(), [&](int a, int b) {
@@ -580,7 +583,7 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         PairTiles out = base;
         std::vector<int> pair(np), count;
         std::vector<int4> tile, tile32;
-        std::vector<int64_t> tile32_off;
+        std::vector<int64_t> tile_off, tile32_off;
         int64_t most = 0;
         bool fits = true;
         for (size_t i = 0; i < recv.size();) {
@@ -619,7 +622,7 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
                     a = b;
                 }
             };
-            cut(tile, u.maxpairs, same_block, [](int) {});
+            cut(tile, u.maxpairs, same_block, [&](int ka) { tile_off.push_back(keys[order[ka]].off); });
             if (tensor)
                 cut(tile32, u.maxpairs32, [&](const Key &x, const Key &y) { return same_block(x, y) && x.perm == y.perm; },
                     [&](int ka) { tile32_off.push_back(off32[ka]); });
@@ -629,10 +632,17 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         }
         if (!fits) break;  // nor will smaller units hold that receiving node
         int4 *t4;
-        CUDA_TRY(c->upload(&q, pair.data(), pair.size())); out.pair = q;
+        std::vector<int4> rec(np);
+        for (int i = 0; i < np; ++i) {
+            const int p = pair[i];
+            const int64_t src = other_mom_off[s.i2o_src[p]], ps = keys[order[key[p]]].perm;
+            rec[i] = make_int4((int)(uint32_t)src, (int)(src >> 32), (int)ps, p);
+        }
+        int64_t *o;
+        CUDA_TRY(c->upload(&t4, rec.data(), rec.size())); out.rec = t4;
         CUDA_TRY(c->upload(&t4, tile.data(), tile.size())); out.tile = t4;
+        CUDA_TRY(c->upload(&o, tile_off.data(), tile_off.size())); out.tile_off = o;
         if (tensor) {
-            int64_t *o;
             CUDA_TRY(c->upload(&t4, tile32.data(), tile32.size())); out.tile32 = t4;
             CUDA_TRY(c->upload(&o, tile32_off.data(), tile32_off.size())); out.tile32_off = o;
         }
@@ -1207,7 +1217,7 @@ h2b_status build_core(h2b_core *c, const h2b_map_desc &d) {
             st = build_sibling_groups(c, sd, h, o.spec_off_host, off);
             if (st) return st;
         } else if (d.coupling_kind == H2B_COUPLING_DENSE) {
-            st = build_pair_tiles(c, d, side == 0, off, perm_set, h.pairs);
+            st = build_pair_tiles(c, d, side == 0, off, perm_set, o.mom_off_host, h.pairs);
             if (st) return st;
         }
     }

@@ -172,8 +172,10 @@ struct PairUnit {
 };
 struct PairTiles {
     std::vector<PairUnit> units;  // host
-    const int *pair = nullptr;    // pair ids, tile by tile
-    const int4 *tile = nullptr;   // {first index into pair, pairs, rows, k}
+    const int4 *rec = nullptr;    // pairs, tile by tile: {source's moment offset (low, high 32 bits) per
+                                  // unit rhs, permutation set in DMap::perm or -1, pair}
+    const int4 *tile = nullptr;   // {first record, pairs, rows, k}
+    const int64_t *tile_off = nullptr;  // element offset of each tile's block in DMap::cpl
     const int *rcv = nullptr;     // receiving nodes, unit by unit
     // FP32 form on the tcgen05 tensor cores: tiles of pairs that read one block through one
     // permutation, the element offset of each one's block in `blocks32` (rows x k, column-major, columns

@@ -23,6 +23,7 @@
 // unreduced blocks 2.56 -> 0.077 ms, against chunks of 16 receiving nodes that each staged every
 // block they read (1-4 field columns) and one CTA per receiving node (wider blocks).
 #include <algorithm>
+#include <type_traits>
 
 #include "h2b_internal.cuh"
 
@@ -32,23 +33,26 @@ namespace {
 
 constexpr int PK_THREADS = 256;
 constexpr int PK_WARPS = PK_THREADS / 32;
-constexpr int PK_N = PAIR_TILE;  // columns per tile: one 8-wide column block per warp
+constexpr int PK_N = PAIR_TILE;  // columns per tile: eight 8-wide column blocks
 // Rows per tile: at most 72, nine 8-row blocks, so that 216 coefficients (6^3) are three whole
-// tiles and 125 (5^3) two of 64; a warp then reuses each column fragment for nine products.
+// tiles and 125 (5^3) two of 64.
 constexpr int PK_MB = 9;
-constexpr int PK_STAGES = 4;
 
-// k per stage: 128 bytes per row (so two CTAs' stages fit an SM's shared memory), 32 bytes of
-// padding in front of the next row. The strides keep a fragment's 32 lanes (8 rows or columns x 4
-// k) on distinct banks: rows of KC + 4 elements where k is contiguous, columns of 72 + 4 (8-byte
-// elements), 72 + 2 (16-byte) or 72 + 0 (4-byte) elements where rows are.
+// Stages in shared memory: k per stage, 128 bytes per row or column (64 for FP32 values), and the row
+// strides, which keep a fragment's 32 lanes (8 rows or columns x 4 k) on distinct banks: rows of
+// KC + 4 elements where k is contiguous, columns of 72 + 4 (8-byte elements), 72 + 2 (16-byte) or 72
+// (4-byte) elements where rows are. Real maps fit three CTAs on an SM (short products: a CTA's first
+// loads cost as much as half its arithmetic at 64 coefficients), complex ones two.
 template <class T> struct PkGeom {
+    static constexpr bool CPLX = ScalarTraits<T>::is_complex;
     static constexpr int KC = sizeof(T) == 16 ? 8 : 16;
+    static constexpr int STAGES = CPLX ? 4 : 3;
+    static constexpr int CTAS = CPLX ? 2 : 3;
     static constexpr int LDK = KC + 4;                                          // k contiguous
     static constexpr int LDM = 8 * PK_MB + (sizeof(T) == 16 ? 2 : sizeof(T) == 8 ? 4 : 0);  // rows contiguous
     static constexpr int ASZ = 8 * PK_MB * LDK > KC * LDM ? 8 * PK_MB * LDK : KC * LDM;
     static constexpr int XSZ = PK_N * LDK;
-    static constexpr size_t BYTES = (size_t)PK_STAGES * (ASZ + XSZ) * sizeof(T);
+    static constexpr size_t BYTES = (size_t)STAGES * (ASZ + XSZ) * sizeof(T);
 };
 
 __device__ __forceinline__ int pk_ncoef(const DSide &s, int lvl) {
@@ -89,117 +93,193 @@ template <> struct PkAcc<cdouble> {
     __device__ __forceinline__ cdouble get(int h) const { return {re[h], im[h]}; }
 };
 
+struct PkArgs {
+    const int4 *rec;           // per pair: {moment offset (low, high), permutation set or -1, pair}
+    const int4 *tile;          // {first record, pairs, rows, k}
+    const int64_t *tile_off;   // element offset of the tile's block
+    int tile0, nrhs, q0, qn, pbase, pstride;
+    bool adj;
+};
+
+// The product of one CTA's tile with MW x NW 8 x 8 blocks per warp: warp w takes column blocks
+// NW (w % WN) .. and row blocks w / WN, w / WN + WM, ... (past the tile: the last one again, never
+// stored).
+template <class T, bool FWD, int MW, int NW, int WN>
+__device__ __forceinline__ void pk_tile(const DMap &m, const PkArgs &g, const T *__restrict__ B, int nc, int kk, int m0,
+                                        int mt, int ncol, const int64_t *col_src, const int *col_perm,
+                                        const int64_t *col_out, const T *__restrict__ am, unsigned char *pk_smem,
+                                        typename ScalarTraits<T>::Acc *__restrict__ prod) {
+    using A = typename ScalarTraits<T>::Acc;
+    using G = PkGeom<T>;
+    constexpr int KC = G::KC, EB = sizeof(T), ST = G::STAGES, WM = PK_WARPS / WN;
+    constexpr uint32_t STAGE = (G::ASZ + G::XSZ) * EB;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nk = (kk + KC - 1) / KC;
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(pk_smem);
+
+    // the block: rows contiguous, a warp takes every eighth k and its lanes the rows, or k contiguous,
+    // a warp's lanes take KC k of 32 / KC rows
+    constexpr int RL = 32 / KC;  // rows (or columns) per warp copy where lanes run along k
+    constexpr int AJ = FWD ? (8 * PK_MB + 31) / 32 : (8 * PK_MB + RL * PK_WARPS - 1) / (RL * PK_WARPS);
+    constexpr int AK = FWD ? KC / PK_WARPS : 1;
+    const int kl = FWD ? warp : lane % KC, il = FWD ? lane : RL * warp + lane / KC;
+    const T *pa = FWD ? B + m0 + il + (int64_t)kl * nc : B + kl + (int64_t)(m0 + il) * kk;
+    const uint32_t da = smem + (uint32_t)((FWD ? kl * G::LDM + il : il * G::LDK + kl) * EB);
+    // the columns: KC k of 32 / KC columns per warp copy, read through the column's permutation, whose
+    // entries are loaded one stage ahead
+    constexpr int XU = PK_N / (RL * PK_WARPS);
+    const int xk = lane % KC;
+    const T *px[XU];
+    const int *pp[XU];
+    int xi[XU];
+    bool xok[XU];
+    const uint32_t dx = smem + (uint32_t)((G::ASZ + (RL * warp + lane / KC) * G::LDK + xk) * EB);
+#pragma unroll
+    for (int u = 0; u < XU; ++u) {
+        const int c = RL * (warp + PK_WARPS * u) + lane / KC;
+        xok[u] = c < ncol;
+        px[u] = am + (xok[u] ? col_src[c] : 0);
+        pp[u] = xok[u] && col_perm[c] >= 0 ? m.perm + col_perm[c] : nullptr;
+    }
+    auto fetch = [&](int kc) {
+        const int k = min(kc * KC + xk, kk - 1);
+#pragma unroll
+        for (int u = 0; u < XU; ++u) xi[u] = pp[u] ? __ldg(pp[u] + k) : k;
+    };
+    auto issue = [&](int kc) {
+        const uint32_t so = (uint32_t)(kc % ST) * STAGE;
+        const int k0 = kc * KC;
+#pragma unroll
+        for (int a = 0; a < AK; ++a) {
+            const bool kin = k0 + kl + (FWD ? PK_WARPS * a : 0) < kk;
+#pragma unroll
+            for (int j = 0; j < AJ; ++j) {
+                const int i = FWD ? il + 32 * j : il + RL * PK_WARPS * j;
+                if (i < mt) {
+                    if constexpr (FWD)
+                        pk_copy<EB>(da + so + (uint32_t)((PK_WARPS * a * G::LDM + 32 * j) * EB),
+                                    kin ? pa + 32 * j + (int64_t)(PK_WARPS * a) * nc : B, kin);
+                    else
+                        pk_copy<EB>(da + so + (uint32_t)(RL * PK_WARPS * j * G::LDK * EB),
+                                    kin ? pa + (int64_t)(RL * PK_WARPS * j) * kk : B, kin);
+                }
+            }
+        }
+        pa += FWD ? (int64_t)KC * nc : KC;
+        const bool xin = k0 + xk < kk;
+#pragma unroll
+        for (int u = 0; u < XU; ++u)
+            if (xok[u]) pk_copy<EB>(dx + so + (uint32_t)(RL * PK_WARPS * u * G::LDK * EB), px[u] + xi[u], xin);
+        fetch(kc + 1);
+    };
+
+    const int g4 = lane >> 2, t4 = lane & 3;
+    const int nb0 = NW * (warp % WN), mb0 = warp / WN;
+    const bool busy = 8 * nb0 < ncol;
+    int aoff[MW];  // element offset of the lane's row in a stage
+#pragma unroll
+    for (int j = 0; j < MW; ++j) {
+        const int i = 8 * min(mb0 + j * WM, PK_MB - 1) + g4;
+        aoff[j] = FWD ? t4 * G::LDM + i : i * G::LDK + t4;
+    }
+    PkAcc<A> acc[MW][NW];
+#pragma unroll
+    for (int j = 0; j < MW; ++j)
+#pragma unroll
+        for (int n = 0; n < NW; ++n) acc[j][n].zero();
+    fetch(0);
+#pragma unroll
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < nk) issue(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int kc = 0; kc < nk; ++kc) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");  // this thread's stage kc
+        __syncthreads();  // everyone's; and the stage issued next was read in the last step
+        if (kc + ST - 1 < nk) issue(kc + ST - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (busy) {
+            const T *as = reinterpret_cast<const T *>(pk_smem + (uint32_t)(kc % ST) * STAGE);
+            const T *xs = as + G::ASZ + (8 * nb0 + g4) * G::LDK + t4;
+#pragma unroll
+            for (int k = 0; k < KC; k += 4) {
+                A b[NW];
+#pragma unroll
+                for (int n = 0; n < NW; ++n) b[n] = wide(xs[8 * n * G::LDK + k]);
+#pragma unroll
+                for (int j = 0; j < MW; ++j) {
+                    const A a = wide(cj(as[aoff[j] + (FWD ? k * G::LDM : k)], g.adj));
+#pragma unroll
+                    for (int n = 0; n < NW; ++n) acc[j][n].step(a, b[n]);
+                }
+            }
+        }
+    }
+    if (!busy) return;
+#pragma unroll
+    for (int n = 0; n < NW; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = 8 * (nb0 + n) + 2 * t4 + h;
+            if (c >= ncol) continue;
+            A *out = prod + col_out[c];
+#pragma unroll
+            for (int j = 0; j < MW; ++j) {
+                const int i = 8 * (mb0 + j * WM) + g4;
+                if (i < mt) out[i] = acc[j][n].get(h);
+            }
+        }
+}
+
 // Tile blockIdx.x of the unit, row tile blockIdx.y, columns [64 blockIdx.z, + 64) of the tile's
 // pairs x qn right-hand sides (pair-major). FWD: the stored block is (receiver x source), rows
 // contiguous; otherwise it is the (source x receiver) block of the mirrored pair, read transposed
 // (conjugated for adjoint maps), k contiguous. Pair p's product for right-hand side q0 + q starts
 // at prod[((p - pbase) qn + q) pstride].
 template <class T, bool FWD>
-__global__ void __launch_bounds__(PK_THREADS, 2)
-i2o_pairs_kernel(DMap m, DSide r, const int *__restrict__ pair, const int4 *__restrict__ tile, int tile0, bool adj,
-                 int nrhs, int q0, int qn, int pbase, int pstride, const T *__restrict__ am,
-                 typename ScalarTraits<T>::Acc *__restrict__ prod) {
-    using A = typename ScalarTraits<T>::Acc;
-    using G = PkGeom<T>;
-    constexpr int KC = G::KC, EB = sizeof(T);
+__global__ void __launch_bounds__(PK_THREADS, PkGeom<T>::CTAS)
+i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTraits<T>::Acc *__restrict__ prod) {
     extern __shared__ __align__(16) unsigned char pk_smem[];
     __shared__ int64_t col_src[PK_N], col_out[PK_N];  // per column: its moments and its product
-    __shared__ int64_t col_perm[PK_N];                // the permutation its moments are read through, -1: none
-    const int4 tl = tile[tile0 + blockIdx.x];         // {first pair, pairs, rows, k}
+    __shared__ int col_perm[PK_N];                    // the permutation its moments are read through, -1: none
+    const int4 tl = __ldg(g.tile + g.tile0 + blockIdx.x);
+    const int64_t off = __ldg(g.tile_off + g.tile0 + blockIdx.x);
     const int c0 = blockIdx.z * PK_N;
     const int nc = tl.z, kk = tl.w;
     const int nmt = (nc + 8 * PK_MB - 1) / (8 * PK_MB);      // row tiles of equal 8-row blocks
     const int bm = 8 * ((nc + 8 * nmt - 1) / (8 * nmt));
     const int m0 = blockIdx.y * bm;
-    if (c0 >= tl.y * qn || m0 >= nc) return;
-    const int ncol = min(PK_N, tl.y * qn - c0), mt = min(bm, nc - m0);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const T *B = static_cast<const T *>(m.cpl) + r.pair_cpl[pair[tl.x]];
-    for (int c = tid; c < ncol; c += PK_THREADS) {
-        const int p = pair[tl.x + (c0 + c) / qn], q = (c0 + c) % qn;
-        col_src[c] = r.pair_src[p] * nrhs + (int64_t)(q0 + q) * kk;
-        col_out[c] = ((int64_t)(p - pbase) * qn + q) * pstride;
-        const int64_t ps = r.pair_perm ? r.pair_perm[p] : -1;
+    if (c0 >= tl.y * g.qn || m0 >= nc) return;
+    const int ncol = min(PK_N, tl.y * g.qn - c0), mt = min(bm, nc - m0);
+    const T *B = static_cast<const T *>(m.cpl) + off;
+    if (threadIdx.x < ncol) {
+        const int c = threadIdx.x, q = (c0 + c) % g.qn;
+        const int4 rc = __ldg(g.rec + tl.x + (c0 + c) / g.qn);
+        col_src[c] = ((int64_t)rc.y << 32 | (uint32_t)rc.x) * g.nrhs + (int64_t)(g.q0 + q) * kk;
+        col_out[c] = ((int64_t)(rc.w - g.pbase) * g.qn + q) * g.pstride + m0;
         // sets [rowperm | rowperm^-1 | colperm | colperm^-1] of n each: forward products run over the
         // block's columns (x read through colperm), transposed ones over its rows (rowperm)
-        col_perm[c] = ps < 0 ? -1 : ps + (FWD ? 2 * kk : 0);
+        col_perm[c] = rc.z < 0 ? -1 : rc.z + (FWD ? 2 * kk : 0);
     }
     __syncthreads();
-    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(pk_smem);
-    auto issue = [&](int kc) {
-        const int k0 = kc * KC, kv = min(KC, kk - k0);
-        const uint32_t as = smem + (uint32_t)((kc % PK_STAGES) * (G::ASZ + G::XSZ) * EB);
-        const uint32_t xs = as + (uint32_t)(G::ASZ * EB);
-        if constexpr (FWD) {
-            for (int e = tid; e < 8 * PK_MB * KC; e += PK_THREADS) {
-                const int k = e / (8 * PK_MB), i = e % (8 * PK_MB);
-                const bool ok = k < kv && i < mt;
-                if (i < bm) pk_copy<EB>(as + (uint32_t)((k * G::LDM + i) * EB), ok ? B + m0 + i + (int64_t)(k0 + k) * nc : B, ok);
-            }
-        } else {
-            for (int e = tid; e < 8 * PK_MB * KC; e += PK_THREADS) {
-                const int i = e / KC, k = e % KC;
-                const bool ok = k < kv && i < mt;
-                if (i < bm) pk_copy<EB>(as + (uint32_t)((i * G::LDK + k) * EB), ok ? B + k0 + k + (int64_t)(m0 + i) * kk : B, ok);
-            }
-        }
-        for (int e = tid; e < ncol * KC; e += PK_THREADS) {
-            const int c = e / KC, k = e % KC;
-            const bool ok = k < kv;
-            const int64_t ps = col_perm[c];
-            const int ks = !ok ? 0 : (ps < 0 ? k0 + k : __ldg(m.perm + ps + k0 + k));
-            pk_copy<EB>(xs + (uint32_t)((c * G::LDK + k) * EB), am + col_src[c] + ks, ok);
-        }
+    // 8 x 8 blocks per warp: wide tiles one column block per warp with all row blocks, or, for real
+    // tiles of 64 rows, two column blocks with half the row blocks (six loads for eight products
+    // instead of nine); narrow tiles spread the row blocks of their few column blocks over the warps
+    auto run = [&](auto mw, auto nw, auto wn) {
+        pk_tile<T, FWD, decltype(mw)::value, decltype(nw)::value, decltype(wn)::value>(
+            m, g, B, nc, kk, m0, mt, ncol, col_src, col_perm, col_out, am, pk_smem, prod);
     };
-    // warps over the tile's 8 x 8 blocks: one column block per warp and all row blocks, or, for
-    // narrow tiles, several warps per column block sharing its row blocks
-    const int nblk = (ncol + 7) / 8, mblk = (mt + 7) / 8;
-    const int wn = nblk > 4 ? 8 : (nblk > 2 ? 4 : (nblk > 1 ? 2 : 1)), wm = PK_WARPS / wn;
-    const int nb = warp % wn, mb0 = warp / wn;
-    const int g4 = lane >> 2, t4 = lane & 3;
-    PkAcc<A> acc[PK_MB];
-#pragma unroll
-    for (int j = 0; j < PK_MB; ++j) acc[j].zero();
-    const int nk = (kk + KC - 1) / KC;
-#pragma unroll
-    for (int s = 0; s < PK_STAGES - 1; ++s) {
-        if (s < nk) issue(s);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int kc = 0; kc < nk; ++kc) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(PK_STAGES - 2) : "memory");  // this thread's stage kc
-        __syncthreads();  // everyone's; and the stage issued next was read in the last step
-        if (kc + PK_STAGES - 1 < nk) issue(kc + PK_STAGES - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (nb < nblk) {
-            const T *as = reinterpret_cast<const T *>(pk_smem) + (kc % PK_STAGES) * (G::ASZ + G::XSZ);
-            const T *xs = as + G::ASZ + (8 * nb + g4) * G::LDK + t4;
-#pragma unroll
-            for (int k = 0; k < KC; k += 4) {
-                const A b = wide(xs[k]);
-#pragma unroll
-                for (int j = 0; j < PK_MB; ++j) {
-                    const int mb = mb0 + j * wm;
-                    if (mb < mblk) {
-                        const int i = 8 * mb + g4;
-                        const T a = FWD ? as[(k + t4) * G::LDM + i] : as[i * G::LDK + k + t4];
-                        acc[j].step(wide(cj(a, adj)), b);
-                    }
-                }
-            }
-        }
-    }
-    if (nb >= nblk) return;
-#pragma unroll
-    for (int j = 0; j < PK_MB; ++j) {
-        const int i = 8 * (mb0 + j * wm) + g4;
-        if (i < mt) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int c = 8 * nb + 2 * t4 + h;
-                if (c < ncol) prod[col_out[c] + m0 + i] = acc[j].get(h);
-            }
-        }
+    using std::integral_constant;
+    if (ncol > 32) {
+        if (mt > 64) run(integral_constant<int, 9>{}, integral_constant<int, 1>{}, integral_constant<int, 8>{});
+        else if (PkGeom<T>::CPLX) run(integral_constant<int, 8>{}, integral_constant<int, 1>{}, integral_constant<int, 8>{});
+        else run(integral_constant<int, 4>{}, integral_constant<int, 2>{}, integral_constant<int, 4>{});
+    } else if (ncol > 16) {
+        run(integral_constant<int, 5>{}, integral_constant<int, 1>{}, integral_constant<int, 4>{});
+    } else if (ncol > 8) {
+        run(integral_constant<int, 3>{}, integral_constant<int, 1>{}, integral_constant<int, 2>{});
+    } else {
+        run(integral_constant<int, 2>{}, integral_constant<int, 1>{}, integral_constant<int, 1>{});
     }
 }
 
@@ -266,8 +346,8 @@ cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, c
         for (int q0 = 0; q0 < nq; q0 += qc) {
             const int qn = std::min(qc, nq - q0);
             const dim3 grid(u.ntiles, mtiles, (u.maxpairs * qn + PK_N - 1) / PK_N);
-            kern<<<grid, PK_THREADS, sm, st>>>(m, r, pt.pair, pt.tile, u.tile0, adj, fa.nrhs, q0, qn, u.p0, pt.pstride,
-                                               static_cast<const T *>(fa.am), prod);
+            const PkArgs g{pt.rec, pt.tile, pt.tile_off, u.tile0, fa.nrhs, q0, qn, u.p0, pt.pstride, adj};
+            kern<<<grid, PK_THREADS, sm, st>>>(m, g, static_cast<const T *>(fa.am), prod);
             launch_sum_t<T>(m, r, pt, u, fa, maxcoef, q0, qn, st);
         }
     return cudaGetLastError();
