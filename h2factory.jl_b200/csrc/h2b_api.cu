@@ -15,6 +15,7 @@
 #include <new>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "h2b_internal.cuh"
@@ -539,16 +540,28 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
     for (size_t i = 0; i < keys.size(); ++i) rank[order[i]] = (int)i;
     for (int p = 0; p < np; ++p) key[p] = rank[key[p]];
 
-    // the FP32 form's tensor-core tiles: every block's chunks of 32 FP32 values of K pair up into
-    // accumulation segments (an odd count would carry a segment from one pair into the next)
+    // the FP32 form's tensor-core tiles: blocks of one shape (one tensor map names the columns of all of
+    // them, another those of the moments) whose chunks of 32 FP32 values of K pair up into accumulation
+    // segments (an odd count would carry a segment from one pair into the next)
     PairTiles base;
-    bool tensor = c->precision == H2B_FP32 && d.coupling_kind == H2B_COUPLING_DENSE;
-    for (const Key &k : keys) tensor &= ((W * k.snc + 31) / 32) % 2 == 0;
+    base.nc32 = keys[0].nc;
+    base.snc32 = keys[0].snc;
+    bool uniform = c->precision == H2B_FP32 && d.coupling_kind == H2B_COUPLING_DENSE;
+    bool stored = c->dmap.cpl_vec != 0;
+    for (const Key &k : keys) {
+        uniform &= k.nc == base.nc32 && k.snc == base.snc32;
+        stored &= k.off % k.nc == 0;
+    }
+    for (int n = 0; n < other.nnodes; ++n) uniform &= ncoef_host(other, other.level[n]) == base.snc32;
+    const bool tensor = uniform && ((W * base.snc32 + 31) / 32) % 2 == 0;
+    base.src_cols = (int64_t)other.nnodes * d.ncomp;
     // their blocks, rows x k: as stored (or the transposed copy) where the columns are whole 16 bytes,
     // else copied with padded columns; per key (in order) the block's offset
     std::vector<int64_t> off32(keys.size(), 0);
-    if (tensor && c->dmap.cpl_vec) {
+    if (uniform && stored) {
         base.blocks32 = test_side ? c->dmap.cpl : c->dmap.cpl_t;
+        base.cols32 = d.coupling_len / W / base.nc32;
+        base.stored32 = true;
         for (size_t i = 0; i < keys.size(); ++i) off32[i] = keys[order[i]].off;
     } else if (tensor) {
         std::vector<float> blocks;
@@ -572,11 +585,21 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         float *fp;
         CUDA_TRY(c->upload(&fp, blocks.data(), blocks.size()));
         base.blocks32 = fp;
+        base.cols32 = (int64_t)blocks.size() / W / ((base.nc32 + 4 / W - 1) / (4 / W) * (4 / W));
     }
-    int *q;
-    CUDA_TRY(c->upload(&q, recv.data(), recv.size()));
-    base.rcv = q;
+    // every plan's arrays in one upload (an allocation costs about as much as building a plan): their
+    // offsets stand in for the pointers until then
+    std::vector<unsigned char> arrays;
+    auto put = [&](auto *&ptr, const auto &v) {
+        using E = std::remove_reference_t<decltype(v[0])>;
+        const size_t at = (arrays.size() + 15) / 16 * 16;
+        arrays.resize(at + v.size() * sizeof(E));
+        memcpy(arrays.data() + at, v.data(), v.size() * sizeof(E));
+        ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(at);
+    };
+    put(base.rcv, recv);
     base.pstride = pstride;
+    const size_t first_plan = plans.size();
     for (int share : PAIR_PLANS) {
         const int64_t max_pairs = PAIR_BUFFER_BYTES / share / (8 * W * (int64_t)pstride);
         if (!plans.empty() && plans.back().units.size() == 1 && np <= max_pairs) continue;  // the same plan again
@@ -604,50 +627,73 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
                 std::sort(pair.begin() + p0, pair.begin() + p1,
                           [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
             }
-            PairUnit u{(int)tile.size(), 0, 0, (int)tile32.size(), 0, 0, (int)i0, (int)(i - i0), p0};
-            // runs of pairs for which same(other, first) holds, each cut into tiles of equal pairs
-            auto cut = [&](std::vector<int4> &to, int &maxpairs, auto same, auto each) {
+            PairUnit u{(int)tile.size(), 0, 0, (int)tile32.size(), {}, (int)i0, (int)(i - i0), p0};
+            // runs of pairs for which same(other, first) holds, each cut into whole tiles and a rest (tiles of
+            // equal pairs kept more column blocks busy: 514 pairs are 8.25 tiles' work that way, 9 the other),
+            // the tiles with more pairs first: {tile, its first pair's key}
+            std::vector<std::pair<int4, int>> cuts;
+            auto cut = [&](auto same) {
+                cuts.clear();
                 for (int a = p0; a < p1;) {
                     const int ka = key[pair[a]];
                     const Key &k = keys[order[ka]];
                     int b = a + 1;
                     while (b < p1 && (key[pair[b]] == ka || same(keys[order[key[pair[b]]]], k))) ++b;
-                    const int nt = (b - a + PAIR_TILE - 1) / PAIR_TILE;
-                    for (int t = 0; t < nt; ++t) {
-                        const int e0 = a + (int)((int64_t)(b - a) * t / nt), e1 = a + (int)((int64_t)(b - a) * (t + 1) / nt);
-                        to.push_back(make_int4(e0, e1 - e0, k.nc, k.snc));
-                        each(ka);
-                        maxpairs = std::max(maxpairs, e1 - e0);
-                    }
+                    for (; a < b; a += PAIR_TILE) cuts.emplace_back(make_int4(a, std::min(PAIR_TILE, b - a), k.nc, k.snc), ka);
                     a = b;
                 }
+                std::stable_sort(cuts.begin(), cuts.end(),
+                                 [](const auto &x, const auto &y) { return x.first.y > y.first.y; });
             };
-            cut(tile, u.maxpairs, same_block, [&](int ka) { tile_off.push_back(keys[order[ka]].off); });
-            if (tensor)
-                cut(tile32, u.maxpairs32, [&](const Key &x, const Key &y) { return same_block(x, y) && x.perm == y.perm; },
-                    [&](int ka) { tile32_off.push_back(off32[ka]); });
-            u.ntiles = (int)tile.size() - u.tile0;
-            u.ntiles32 = (int)tile32.size() - u.tile32_0;
+            cut(same_block);
+            for (const auto &t : cuts) {
+                tile.push_back(t.first);
+                tile_off.push_back(keys[order[t.second]].off);
+            }
+            u.ntiles = (int)cuts.size();
+            u.maxpairs = cuts[0].first.y;
+            if (tensor) {
+                cut([&](const Key &x, const Key &y) { return same_block(x, y) && x.perm == y.perm; });
+                for (const auto &t : cuts) {
+                    tile32.push_back(t.first);
+                    tile32_off.push_back(off32[t.second]);
+                    for (int c = 0; c < t.first.y; ++c) ++u.more32[c];
+                }
+            }
             out.units.push_back(u);
         }
         if (!fits) break;  // nor will smaller units hold that receiving node
-        int4 *t4;
         std::vector<int4> rec(np);
         for (int i = 0; i < np; ++i) {
             const int p = pair[i];
             const int64_t src = other_mom_off[s.i2o_src[p]], ps = keys[order[key[p]]].perm;
             rec[i] = make_int4((int)(uint32_t)src, (int)(src >> 32), (int)ps, p);
         }
-        int64_t *o;
-        CUDA_TRY(c->upload(&t4, rec.data(), rec.size())); out.rec = t4;
-        CUDA_TRY(c->upload(&t4, tile.data(), tile.size())); out.tile = t4;
-        CUDA_TRY(c->upload(&o, tile_off.data(), tile_off.size())); out.tile_off = o;
+        put(out.rec, rec);
+        put(out.tile, tile);
+        put(out.tile_off, tile_off);
         if (tensor) {
-            CUDA_TRY(c->upload(&t4, tile32.data(), tile32.size())); out.tile32 = t4;
-            CUDA_TRY(c->upload(&o, tile32_off.data(), tile32_off.size())); out.tile32_off = o;
+            put(out.tile32, tile32);
+            put(out.tile32_off, tile32_off);
         }
         out.unit_elems = most * pstride;
         plans.push_back(out);
+    }
+    unsigned char *mem;
+    CUDA_TRY(c->upload(&mem, arrays.data(), arrays.size()));
+    for (size_t i = first_plan; i < plans.size(); ++i) {
+        PairTiles &t = plans[i];
+        auto place = [&](auto *&ptr) {
+            ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(mem + reinterpret_cast<size_t>(ptr));
+        };
+        place(t.rcv);
+        place(t.rec);
+        place(t.tile);
+        place(t.tile_off);
+        if (tensor) {
+            place(t.tile32);
+            place(t.tile32_off);
+        }
     }
     return H2B_OK;
 }
@@ -1447,7 +1493,7 @@ h2b_status run_i2o(h2b_core *c, const SideHost &D, const SideHost &A, const FarA
         return H2B_OK;
     }
     CUDA_TRY(launch_i2o(cplx, c->precision, c->dmap, D.d, A.d, D.d_recv, D.n_recv, fa,
-                        maxcoef, maxt, D.maxhalf, st));
+                        maxcoef, maxt, D.maxhalf, pt, st));
     return H2B_OK;
 }
 

@@ -77,6 +77,21 @@ template <class R> __host__ __device__ __forceinline__ void from_cx(Cx<R> s, Cx<
 __host__ __device__ __forceinline__ void from_cx(cdouble s, float &out) { out = (float)s.x; }
 __host__ __device__ __forceinline__ void from_cx(cdouble s, cfloat &out) { out = {(float)s.x, (float)s.y}; }
 
+// One access per scalar for arrays of the library's own (a complex scalar's type only promises the
+// alignment of its parts, since x and y come from the caller; ours start on 16 bytes)
+template <class T> __device__ __forceinline__ T ldv(const T *p) { return *p; }
+template <> __device__ __forceinline__ cdouble ldv(const cdouble *p) {
+    const double2 v = *reinterpret_cast<const double2 *>(p);
+    return {v.x, v.y};
+}
+template <> __device__ __forceinline__ cfloat ldv(const cfloat *p) {
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    return {v.x, v.y};
+}
+template <class T> __device__ __forceinline__ void stv(T *p, T v) { *p = v; }
+template <> __device__ __forceinline__ void stv(cdouble *p, cdouble v) { *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y); }
+template <> __device__ __forceinline__ void stv(cfloat *p, cfloat v) { *reinterpret_cast<float2 *>(p) = make_float2(v.x, v.y); }
+
 // ---------------------------------------------------------------------------------------------
 // Device-resident side of a core (all pointers device memory).
 // ---------------------------------------------------------------------------------------------
@@ -160,13 +175,14 @@ struct SibGroups {
 
 // Dense I2O with FP64 sums (h2b_pairs.cu): the pairs of one receiving side in units of consecutive
 // receiving nodes, sorted inside a unit by the stored coupling block that they read (then by its
-// permutations), and cut into tiles of at most PAIR_TILE pairs of one block. A unit's products take
+// permutations), and cut into tiles of at most PAIR_TILE pairs of one block, most pairs first. A unit's products take
 // unit_elems scalars at most per right-hand side: pair p's at (p - p0) pstride.
 constexpr int PAIR_TILE = 64;
 struct PairUnit {
     int tile0, ntiles;  // tiles of the unit
     int maxpairs;       // pairs of its largest tile
-    int tile32_0, ntiles32, maxpairs32;  // the same of tile32
+    int tile32_0;          // its first one of tile32
+    int more32[PAIR_TILE]; // tiles of tile32 with more than c pairs
     int rcv0, nrcv;     // its receiving nodes
     int p0;             // its first pair
 };
@@ -183,6 +199,10 @@ struct PairTiles {
     const int4 *tile32 = nullptr;
     const int64_t *tile32_off = nullptr;
     const void *blocks32 = nullptr;
+    int nc32 = 0, snc32 = 0;      // rows and k of every block
+    int64_t cols32 = 0;           // columns in blocks32
+    bool stored32 = false;        // blocks32 is the stored array: a pair's block starts at its pair_cpl
+    int64_t src_cols = 0;         // source moment columns per unit rhs
     int64_t unit_elems = 0;
     int pstride = 1;              // scalars per pair and right-hand side
 };
@@ -214,7 +234,7 @@ cudaError_t launch_toeplitz_in(bool cplx, int precision, const DMap &m, const DS
                                int maxtsize, int maxaxis, cudaStream_t st);
 cudaError_t launch_i2o(bool cplx, int precision, const DMap &m, const DSide &recv,
                        const DSide &src, const int *nodes, int nnodes, const FarArgs &fa,
-                       int maxcoef, int maxtsize, int maxhalf, cudaStream_t st);
+                       int maxcoef, int maxtsize, int maxhalf, const PairTiles *pt, cudaStream_t st);
 cudaError_t launch_toeplitz_out(bool cplx, int precision, const DMap &m, const DSide &s,
                                 const int *nodes, int nnodes, bool inverse, const FarArgs &fa,
                                 int maxtsize, int maxaxis, cudaStream_t st);
@@ -222,7 +242,7 @@ cudaError_t launch_toeplitz_out(bool cplx, int precision, const DMap &m, const D
 // storage is dense and the right-hand sides make at least 4 FP32 columns (MMA N padded to 16).
 bool i2o_umma_eligible(bool cplx, int precision, const DMap &m, int nq);
 cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const DSide &src, const int *nodes,
-                            int nnodes, const FarArgs &fa, int maxcoef, cudaStream_t st);
+                            int nnodes, const FarArgs &fa, int maxcoef, const PairTiles *pt, cudaStream_t st);
 // The sums of one unit's pair products (right-hand sides [q0, q0 + qn)) into the receiving nodes' moments.
 cudaError_t launch_i2o_pairs_sum(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
                                  const PairUnit &u, const FarArgs &fa, int maxcoef, int q0, int qn, cudaStream_t st);

@@ -18,9 +18,9 @@
 // What bounds it: the FP64 tensor cores (37 TFLOP/s here, mma.sync m8n8k4 .f64). A product reads
 // its block once per 64 columns and writes 16 bytes per complex sum (8 real) per row, read once by
 // the sums: 8.5 % of the time at 216 complex coefficients, about half at 64 real ones. Measured
-// (I2O per product, FP64): 65,536-point Helmholtz sphere, p = 6, 1 right-hand side 7.73 -> 1.12 ms;
-// 262,144 points, 32 right-hand sides 211 -> 134 ms (22 TFLOP/s); 8,192-point Laplace cube, p = 4,
-// unreduced blocks 2.56 -> 0.077 ms, against chunks of 16 receiving nodes that each staged every
+// (I2O per product, FP64): 65,536-point Helmholtz sphere, p = 6, 1 right-hand side 7.73 -> 0.91 ms;
+// 262,144 points, 32 right-hand sides 211 -> 112 ms (26 TFLOP/s); 8,192-point Laplace cube, p = 4,
+// unreduced blocks 2.56 -> 0.052 ms, against chunks of 16 receiving nodes that each staged every
 // block they read (1-4 field columns) and one CTA per receiving node (wider blocks).
 #include <algorithm>
 #include <type_traits>
@@ -38,15 +38,17 @@ constexpr int PK_N = PAIR_TILE;  // columns per tile: eight 8-wide column blocks
 // tiles and 125 (5^3) two of 64.
 constexpr int PK_MB = 9;
 
-// Stages in shared memory: k per stage, 128 bytes per row or column (64 for FP32 values), and the row
-// strides, which keep a fragment's 32 lanes (8 rows or columns x 4 k) on distinct banks: rows of
+// Stages in shared memory: 16 values of k each (two whole stages hid the copies as well as four of 8
+// complex or three of 16 real values and halve the barriers: 262,144-point sphere, 32 right-hand sides
+// 121 -> 112 ms, 30,011-point cube, 16 right-hand sides 3.05 -> 2.80 ms; FP32 values lost 5 %), and the
+// row strides, which keep a fragment's 32 lanes (8 rows or columns x 4 k) on distinct banks: rows of
 // KC + 4 elements where k is contiguous, columns of 72 + 4 (8-byte elements), 72 + 2 (16-byte) or 72
 // (4-byte) elements where rows are. Real maps fit three CTAs on an SM (short products: a CTA's first
 // loads cost as much as half its arithmetic at 64 coefficients), complex ones two.
 template <class T> struct PkGeom {
     static constexpr bool CPLX = ScalarTraits<T>::is_complex;
-    static constexpr int KC = sizeof(T) == 16 ? 8 : 16;
-    static constexpr int STAGES = CPLX ? 4 : 3;
+    static constexpr int KC = 16;
+    static constexpr int STAGES = !CPLX && sizeof(T) == 4 ? 3 : 2;
     static constexpr int CTAS = CPLX ? 2 : 3;
     static constexpr int LDK = KC + 4;                                          // k contiguous
     static constexpr int LDM = 8 * PK_MB + (sizeof(T) == 16 ? 2 : sizeof(T) == 8 ? 4 : 0);  // rows contiguous
@@ -205,10 +207,10 @@ __device__ __forceinline__ void pk_tile(const DMap &m, const PkArgs &g, const T 
             for (int k = 0; k < KC; k += 4) {
                 A b[NW];
 #pragma unroll
-                for (int n = 0; n < NW; ++n) b[n] = wide(xs[8 * n * G::LDK + k]);
+                for (int n = 0; n < NW; ++n) b[n] = wide(ldv(xs + 8 * n * G::LDK + k));
 #pragma unroll
                 for (int j = 0; j < MW; ++j) {
-                    const A a = wide(cj(as[aoff[j] + (FWD ? k * G::LDM : k)], g.adj));
+                    const A a = wide(cj(ldv(as + aoff[j] + (FWD ? k * G::LDM : k)), g.adj));
 #pragma unroll
                     for (int n = 0; n < NW; ++n) acc[j][n].step(a, b[n]);
                 }
@@ -226,7 +228,7 @@ __device__ __forceinline__ void pk_tile(const DMap &m, const PkArgs &g, const T 
 #pragma unroll
             for (int j = 0; j < MW; ++j) {
                 const int i = 8 * (mb0 + j * WM) + g4;
-                if (i < mt) out[i] = acc[j][n].get(h);
+                if (i < mt) stv(out + i, acc[j][n].get(h));
             }
         }
 }
@@ -285,7 +287,8 @@ i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTrai
 
 // Receiving node nodes[blockIdx.x]: its moments for right-hand sides [q0, q0 + qn) as the sum of
 // its pairs' columns, read through each pair's row permutation. Loads of eight pairs are in flight
-// per thread; the sum runs in list order.
+// per thread; the sum runs in list order. (Columns copied to shared memory as they lie and permuted on
+// the reads from there were slower everywhere, 65,536-point sphere, 32 right-hand sides: 2.4 -> 5 ms.)
 template <class T>
 __global__ void __launch_bounds__(128)
 i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, int nrhs, int q0, int qn, int pbase,
@@ -308,22 +311,25 @@ i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, i
             const int pp = min(p + u, p1 - 1);
             const int64_t ps = r.pair_perm ? __ldg(r.pair_perm + pp) : -1;
             const int row = ps < 0 ? i : __ldg(m.perm + ps + set + i);
-            v[u] = prod[((int64_t)(pp - pbase) * qn + q) * pstride + row];
+            v[u] = ldv(prod + ((int64_t)(pp - pbase) * qn + q) * pstride + row);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (p + u < p1) sum = sum + v[u];
     }
-    narrow(sum, dm[r.mom_off[node] * nrhs + (int64_t)(q0 + q) * nc + i]);
+    T out;
+    narrow(sum, out);
+    stv(dm + r.mom_off[node] * nrhs + (int64_t)(q0 + q) * nc + i, out);
 }
 
 template <class T>
-void launch_sum_t(const DMap &m, const DSide &r, const PairTiles &pt, const PairUnit &u, const FarArgs &fa, int maxcoef,
-                  int q0, int qn, cudaStream_t st) {
+cudaError_t launch_sum_t(const DMap &m, const DSide &r, const PairTiles &pt, const PairUnit &u, const FarArgs &fa, int maxcoef,
+                         int q0, int qn, cudaStream_t st) {
     using A = typename ScalarTraits<T>::Acc;
     const dim3 grid(u.nrcv, (unsigned)(((int64_t)maxcoef * qn + 127) / 128));
     i2o_pairs_sum_kernel<T><<<grid, 128, 0, st>>>(m, r, pt.rcv + u.rcv0, fa.mode == H2B_FORWARD, fa.nrhs, q0, qn, u.p0,
                                                   pt.pstride, static_cast<const A *>(fa.prod), static_cast<T *>(fa.dm));
+    return cudaGetLastError();
 }
 
 template <class T>
@@ -348,7 +354,8 @@ cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, c
             const dim3 grid(u.ntiles, mtiles, (u.maxpairs * qn + PK_N - 1) / PK_N);
             const PkArgs g{pt.rec, pt.tile, pt.tile_off, u.tile0, fa.nrhs, q0, qn, u.p0, pt.pstride, adj};
             kern<<<grid, PK_THREADS, sm, st>>>(m, g, static_cast<const T *>(fa.am), prod);
-            launch_sum_t<T>(m, r, pt, u, fa, maxcoef, q0, qn, st);
+            err = launch_sum_t<T>(m, r, pt, u, fa, maxcoef, q0, qn, st);
+            if (err != cudaSuccess) return err;
         }
     return cudaGetLastError();
 }
@@ -374,11 +381,11 @@ cudaError_t launch_i2o_pairs(bool cplx, int precision, const DMap &m, const DSid
 
 cudaError_t launch_i2o_pairs_sum(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
                                  const PairUnit &u, const FarArgs &fa, int maxcoef, int q0, int qn, cudaStream_t st) {
-    if (!cplx && precision == H2B_FP64) launch_sum_t<double>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
-    else if (!cplx) launch_sum_t<float>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
-    else if (precision == H2B_FP64) launch_sum_t<cdouble>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
-    else launch_sum_t<cfloat>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
-    return cudaGetLastError();
+    if (!cplx)
+        return precision == H2B_FP64 ? launch_sum_t<double>(m, recv, pt, u, fa, maxcoef, q0, qn, st)
+                                     : launch_sum_t<float>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
+    return precision == H2B_FP64 ? launch_sum_t<cdouble>(m, recv, pt, u, fa, maxcoef, q0, qn, st)
+                                 : launch_sum_t<cfloat>(m, recv, pt, u, fa, maxcoef, q0, qn, st);
 }
 
 }  // namespace h2b

@@ -40,6 +40,9 @@
 // MMA thread waits (with the full bound) for the products it issued, the moment warps for their
 // copies, and the CTA frees its tensor memory and returns with its output tile unwritten.
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 
 #include "h2b_internal.cuh"
@@ -112,7 +115,8 @@ __device__ __forceinline__ uint32_t goff(int row, int kg) {
 
 // nearest TF32 value (10 explicit mantissa bits, ties away from zero) as FP32 bits with the 13 low
 // mantissa bits cleared: add half of their range to the magnitude, then clear them. Moments and
-// couplings are finite and far below the overflow edge.
+// couplings are finite and far below the overflow edge. (cvt.rna.tf32 is one instruction but shares a
+// 16-lane pipe with the drain warps' FP32 -> FP64 conversions: 5 % slower here.)
 __device__ __forceinline__ uint32_t tf32_bits(float a) {
     return (__float_as_uint(a) + 0x1000u) & 0xFFFFE000u;
 }
@@ -124,6 +128,15 @@ __device__ __forceinline__ void split2(float x, uint32_t &hi, uint32_t &lo) {
 }
 
 // D (+)= A (tensor memory) * B (shared memory), kind::tf32, and the commit of the products so far.
+// four rows {r0 .. r3} of a tensor map, from x on, into this CTA's shared memory
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *map, int x, int4 r, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], "
+        "[%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w), "r"(su32(bar))
+        : "memory");
+}
+
 // One lane of a converged warp, as a predicate for the two calls below. The whole warp runs the issuing
 // loop and only the instruction is predicated: its operands then stay in uniform registers, and a
 // product costs 10 cycles to issue (32 at N = 64, the tensor cores' own rate) against 45 from a branch
@@ -328,10 +341,16 @@ __device__ __forceinline__ float2 ldg2(const cfloat *p) { return __ldg(reinterpr
 
 }  // namespace
 
-template <class T>
-__global__ void __maxnreg__(168)
+// TMA: the coupling columns come four to a gather (`blocks` names the columns of all stored blocks, `ld`
+// elements each, copied `pitch` bytes apart) from a warp of its own, for blocks of at most 256 FP32
+// values per column; else the coupling warps issue a bulk copy per column (or read rows from global
+// memory). A gather or bulk copy costs its warp about 100 cycles: with 32 columns per chunk of a real
+// block, eight in each coupling warp, those were a third of the kernel's time.
+template <class T, bool TMA>
+__global__ void __maxnreg__(TMA ? 128 : 168)
 i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mode, int nrhs, int qt_max,
-                const T *__restrict__ am, T *__restrict__ dm) {
+                const T *__restrict__ am, T *__restrict__ dm, const __grid_constant__ CUtensorMap blocks, int pitch,
+                int ld) {
     constexpr int W = UmScalar<T>::W;
     constexpr int EB = sizeof(T);        // bytes per element (4 real, 8 complex)
     constexpr int KQ = UM_KC / W;        // elements along k per chunk
@@ -355,7 +374,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
     T *out = dm + r.mom_off[node] * nrhs;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (p0 == p1) {
-        for (int o = tid; o < mt * qt; o += UM_THREADS) out[(int64_t)(q0 + o / mt) * nc + m0 + o % mt] = T{};
+        for (int o = tid; o < mt * qt; o += (int)blockDim.x) out[(int64_t)(q0 + o / mt) * nc + m0 + o % mt] = T{};
         return;
     }
     const bool fwd = mode == H2B_FORWARD, adj = mode == H2B_ADJOINT;
@@ -398,7 +417,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
     const uint32_t tmem = tmem_slot;
     {  // chunks of the whole interaction list
         int mine = 0;
-        for (int p = p0 + tid; p < p1; p += UM_THREADS) mine += (W * um_ncoef(t, t.level[r.i2o_src[p]]) + UM_KC - 1) / UM_KC;
+        for (int p = p0 + tid; p < p1; p += (int)blockDim.x) mine += (W * um_ncoef(t, t.level[r.i2o_src[p]]) + UM_KC - 1) / UM_KC;
         if (mine) atomicAdd(&nchunks_s, mine);
         __syncthreads();
     }
@@ -408,11 +427,11 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
     const uint32_t b_stage_bytes = 2u * (uint32_t)np * (UM_KC * 4);  // hi then lo, canonical layout
     const uint32_t raw0 = smem0 + UM_NS * b_stage_bytes;
     const uint32_t raw_stage_bytes = (uint32_t)qt_max * UM_RAWROW;
-    const uint32_t acol_bytes = (uint32_t)nc * EB;                 // one stored coupling column
+    const uint32_t acol_bytes = TMA ? (uint32_t)pitch : (uint32_t)nc * EB;  // one stored coupling column
     const uint32_t astage_bytes = ((uint32_t)KQ * acol_bytes + 127u) & ~127u;
     const uint32_t araw0 = raw0 + ((UM_RS * raw_stage_bytes + 127u) & ~127u);
 
-    if (warp < 4 && m.cpl_vec) {
+    if (warp < 4 && (TMA || m.cpl_vec)) {
         // ---------------- coupling warps, bulk-copy path ----------------
         // Per chunk, lane j of issuing warp w copies column kmap[k0 + w KQ / UM_AI + j] of the pair's
         // stored block (nc contiguous values) into a shared-memory stage with a bulk copy, UM_ALA
@@ -429,7 +448,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
         UmPair<T> iu = lu;
         constexpr int JW = KQ / UM_AI;  // columns copied by each issuing warp
         const int jw = warp * JW;       // this warp's first column of a chunk
-        const bool issuer = warp < UM_AI;
+        const bool issuer = !TMA && warp < UM_AI;
         int kcol = 0;  // lane j: stored column of the copy chunk's k = ik KQ + jw + j
         auto fetch_col = [&]() {
             const int k = min(ik * KQ + jw + lane, iu.snc - 1);
@@ -468,7 +487,8 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
             const int st = c % UM_AR;
             bool landed = true;
 #pragma unroll
-            for (int w = 0; w < UM_AI; ++w) landed = landed && warp_wait(&ar_full[w][st], (c / UM_AR) & 1, limit);
+            for (int w = 0; w < (TMA ? 1 : UM_AI); ++w)
+                landed = landed && warp_wait(&ar_full[w][st], (c / UM_AR) & 1, limit);
             if (!landed) {
                 abort_s = 1;
                 break;
@@ -683,6 +703,49 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
             mbar_arrive(&b_full[s]);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (TMA && warp == UM_WARPS) {
+        // ---------------- copy warp: a chunk's columns, UM_AR chunks ahead ----------------
+        // lane j: the columns 4 j .. 4 j + 3 of a chunk (past the block: its last one), loaded a chunk before
+        // they are used
+        int ip = p0, ik = 0, c = 0;
+        UmPair<T> u = um_pair<T>(m, r, t, p0, nc, fwd, nrhs, q0, am);
+        int col0 = (int)(r.pair_cpl[p0] / ld);
+        auto columns = [&](int k) -> int4 {
+            int v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int kk = min(k * KQ + 4 * lane + e, u.snc - 1);
+                v[e] = u.kmap ? __ldg(u.kmap + kk) : kk;
+            }
+            return make_int4(v[0], v[1], v[2], v[3]);
+        };
+        int4 cols = make_int4(0, 0, 0, 0);
+        if (lane < KQ / 4) cols = columns(0);
+        for (; c < C; ++c) {
+            const int st = c % UM_AR, groups = (min(KQ, u.snc - ik * KQ) + 3) / 4, first = col0;
+            int4 next = cols;
+            if (++ik == u.nk) {
+                ik = 0;
+                if (++ip < p1) {
+                    u = um_pair<T>(m, r, t, ip, nc, fwd, nrhs, q0, am);
+                    col0 = (int)(r.pair_cpl[ip] / ld);
+                }
+            }
+            if (c + 1 < C && lane < KQ / 4) next = columns(ik);
+            if (warp_aborted(&abort_s) || (c >= UM_AR && !warp_wait(&ar_empty[st], ((c / UM_AR) - 1) & 1, limit))) {
+                abort_s = 1;
+                break;
+            }
+            if (lane == 0) mbar_expect_tx(&ar_full[0][st], (uint32_t)(4 * groups) * acol_bytes);
+            __syncwarp();
+            if (lane < groups)
+                tma_gather4(araw0 + (uint32_t)st * astage_bytes + (uint32_t)lane * (4 * acol_bytes), &blocks, 0,
+                            make_int4(cols.x + first, cols.y + first, cols.z + first, cols.w + first), &ar_full[0][st]);
+            __syncwarp();
+            cols = next;
+        }
+        // copies in flight write this CTA's shared memory: all have landed before the CTA can exit
+        for (int cc = max(0, c - UM_AR); cc < c; ++cc) mbar_wait(&ar_full[0][cc % UM_AR], (cc / UM_AR) & 1, UM_SPIN_FINAL);
     } else if (warp < UM_WARPS - 1) {
         // ---------------- drain warps: FP64 sum of the segments, then the epilogue ----------------
         const int lq = warp & 3;
@@ -798,21 +861,26 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
 // segment sums. Each pair's FP64 sum goes to its column of the pair-product buffer; the row
 // permutation is left to i2o_pairs_sum_kernel, so the rows of a tile are contiguous in the block.
 //
-// What bounds it: the roles' instruction latency, about 1,400 cycles per chunk against 384 for its
-// products (ncu: 0.54 instructions per scheduler and cycle, DRAM 5 %, L2 15 %). Measured (I2O per
-// product, 65,536-point Helmholtz sphere, p = 6): 8 right-hand sides 14.2 -> 4.2 ms, 32 right-hand
-// sides 15.1 -> 14.7 ms against one receiving node per CTA. Roles (24 warps, six warpgroups):
+// What bounds it: the roles' instructions, about 2,700 per chunk (1,360 cycles against 384 for the
+// chunk's products; ncu: 0.51 issued per scheduler and cycle, tensor operands and L2 far from full).
+// Taking one role's work away gains 4-10 % each (the coupling's split most). Measured (I2O per
+// product, 65,536-point Helmholtz sphere, p = 6): 8 right-hand sides 14.2 -> 3.7 ms, 32 right-hand
+// sides 15.1 -> 12.5 ms (2.4 of them the sums) against one receiving node per CTA.
+// Roles (24 warps, six warpgroups):
 //   * scheduler: turns the CTA's items into records in a ring (the block, and every column's moments
 //     and product), so that no other role chases the plan's arrays;
-//   * two copy warps: the rows of each chunk's columns into a ring of UP_AR stages, 16 bytes per lane
-//     (cp.async: a bulk copy costs its issuing warp about 100 cycles per column, and a chunk has 16);
+//   * a copy warp: the rows of each chunk's columns into a ring of UP_AR stages, four columns per TMA
+//     gather (a column permutation is which columns are named; one bulk copy per column cost its warp
+//     about 100 cycles each, and 16-byte cp.async pieces held every role up behind the SM's own
+//     load path);
+//   * a second copy warp for the moments, four columns of the product per TMA gather, where the
+//     moment columns are whole 16 bytes; else the moment warps copy them with cp.async a turn ahead;
 //   * eight coupling warps, four per chunk in turn: read, split, write to tensor memory;
-//   * four moment warps, one chunk each in turn: cp.async its moments a turn ahead, split them into
-//     shared memory; operand stages hold a whole segment (two chunks), so the MMA thread waits once
-//     per 24 products;
+//   * four moment warps, one chunk each in turn: split its moments into shared memory; operand stages
+//     hold a whole segment (two chunks), so the MMA warp waits once per 24 products;
 //   * MMA thread; eight drain warps, which keep the FP64 sums (32 each) in registers: the kernel starts
-//     with 80 registers a thread and moves them to the drain warps (setmaxnreg; 256 threads each at 72,
-//     64 and 104 make the 240 x 256 that the block was launched with).
+//     with 80 registers a thread and moves them to the drain warps (setmaxnreg; 256 threads each at 64,
+//     64 and 112 make the 240 x 256 that the block was launched with).
 // ---------------------------------------------------------------------------------------------
 constexpr int UP_N = 64;                  // product columns per item
 constexpr int UP_NS = 3;                  // operand stages, one accumulation segment each
@@ -823,10 +891,10 @@ constexpr int UP_IR = 8;
 constexpr int UP_B0 = 8, UP_COPY = 12, UP_MMA = 14, UP_SCHED = 15, UP_D0 = 16;  // first warps of the roles
 constexpr int UP_WARPS = 24, UP_THREADS = UP_WARPS * 32;
 constexpr int UP_BW = UP_COPY - UP_B0;    // moment warps
-constexpr int UP_RS = 2 * UP_BW;          // raw moment stages: two per moment warp
+constexpr int UP_RS = 2 * UP_BW;          // raw moment stages: a ring, or two per moment warp
 constexpr int UP_READERS = UP_WARPS - 1;  // warps that read the item records
 static_assert(UM_SEG == 2, "an operand stage holds two chunks, one per half of the coupling warps");
-constexpr int UP_REG_A = 72, UP_REG_B = 64, UP_REG_D = 104;
+constexpr int UP_REG_A = 64, UP_REG_B = 64, UP_REG_D = 112;
 static_assert(UP_BW == 2 * UM_SEG && UP_NS * UM_SEG > UP_BW, "two moment warps fill a stage");
 
 // elements of a block's column as stored for the column copies: whole 16 bytes
@@ -834,20 +902,33 @@ template <class T> __host__ __device__ constexpr int up_ld(int nc) {
     return (nc + 16 / (int)sizeof(T) - 1) / (16 / (int)sizeof(T)) * (16 / (int)sizeof(T));
 }
 
+// a raw moment stage: rows of a chunk's 128 bytes, swizzled (TMA) or padded (cp.async)
+template <bool TMA> constexpr uint32_t up_raw_row() { return TMA ? UM_KC * 4 : UM_RAWROW; }
+
 struct UpArgs {
-    const int *pair;
-    const int4 *tile;          // {first index into pair, pairs, rows, k}
+    const int4 *rec;           // per pair: {moment offset (low, high), permutation set or -1, pair}
+    const int4 *tile;          // {first record, pairs, rows, k}
     const int64_t *tile_off;   // element offset of the tile's block
-    int tile0, ntiles, zt, mt; // tiles of the unit; column tiles and row tiles per tile (at most)
+    int tile0, mt;             // the unit's first tile; row tiles of a block
+    int more[PAIR_TILE];       // tiles of the unit with more than c pairs
     int mode, nrhs, q0, qn, pbase, pstride;
+    int ld, pitch, rowbox;     // elements of a stored block column, bytes of a copied one; moment rows per copy
 };
 
 template <int NC> struct UpItem {
-    int nk, ncol, snc, rows, ld;  // nk = 0: no more items
-    int64_t blk;                  // the item's first row in `blocks`
-    int64_t perm;                 // k -> stored column in DMap::perm, -1: identity
-    int64_t src[NC], out[NC];     // per column: its moments, its product (at the item's first row)
+    int nk, ncol, snc, rows;   // nk = 0: no more items
+    int m0, col;               // first row of the block, column index of the block in its tensor map
+    int64_t perm;              // k -> stored column in DMap::perm, -1: identity
+    int64_t src[NC], out[NC];  // per column: its moments (TMA: its row in their map), its product
 };
+
+// the tensor map's box (its rows from r on), from x on
+__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int x, int r, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(r), "r"(su32(bar))
+        : "memory");
+}
 
 // mbar_wait (for a whole warp, with one outcome, when WARP) that also ends (false, uncounted) once the CTA has given up: the flag is
 // read only after an attempt that found the phase incomplete, so a wait that finds it complete costs
@@ -875,46 +956,28 @@ __device__ __forceinline__ void cp16_cg(uint32_t dst, const void *src, bool ok) 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-// store_split without the conjugation (the moment warps apply it) and with values past the block
-// zeroed only in its last, partial chunk
-template <int W>
-__device__ __forceinline__ void up_store_split(uint32_t ta, const float (&v)[UM_KC], int kv) {
-#pragma unroll
-    for (int h = 0; h < UM_KC / 16; ++h) {
-        uint32_t hi[16], lo[16];
-        if (kv >= UM_KC / W) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) split2(v[16 * h + e], hi[e], lo[e]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) split2((16 * h + e) / W < kv ? v[16 * h + e] : 0.0f, hi[e], lo[e]);
-        }
-        tmem_st16(ta + 16u * h, hi);
-        tmem_st16(ta + UM_KC + 16u * h, lo);
-    }
-    tmem_wait_st();
-}
-
 // product rows of one part (real, imaginary) of `ncol` columns: MMA N is a multiple of 16
 template <int W> __device__ __forceinline__ int up_part(int ncol) {
     return W == 2 ? (ncol + 7) & ~7 : (ncol + 15) & ~15;
 }
 
-template <class T>
+template <class T, bool TMA>
 __global__ void __launch_bounds__(UP_THREADS, 1)
-i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, const T *__restrict__ am,
+i2o_umma_pairs_kernel(DMap m, UpArgs g, const __grid_constant__ CUtensorMap blocks,
+                      const __grid_constant__ CUtensorMap moments, const T *__restrict__ am,
                       typename ScalarTraits<T>::Acc *__restrict__ prod) {
     constexpr int W = UmScalar<T>::W;
     constexpr int EB = sizeof(T);
     constexpr int KQ = UM_KC / W;       // elements along k per chunk
     constexpr int NC = UP_N / W;        // columns (pairs x right-hand sides) per item
     constexpr uint32_t B_CHUNK = 2u * UP_N * UM_KC * 4, B_STAGE = UM_SEG * B_CHUNK;  // per chunk: hi then lo
-    constexpr uint32_t RAW_STAGE = (uint32_t)NC * UM_RAWROW;
-    constexpr uint32_t A_COL = UM_M * EB, A_STAGE = KQ * A_COL;
+    constexpr uint32_t RAW_ROW = up_raw_row<TMA>(), RAW_STAGE = (uint32_t)NC * RAW_ROW;
+    constexpr uint32_t A_STAGE = KQ * UM_M * EB;
+    const uint32_t A_COL = (uint32_t)g.pitch;
     constexpr uint32_t COL_A = 2 * UP_N;  // tensor memory: two accumulators, then the coupling stages
     extern __shared__ __align__(128) unsigned char um_smem[];
     constexpr int UP_AR = up_ar<W>();
-    __shared__ uint64_t full[UP_NS], empty[UP_NS], ar_full[UP_AR], ar_empty[UP_AR];
+    __shared__ uint64_t full[UP_NS], empty[UP_NS], ar_full[UP_AR], ar_empty[UP_AR], br_full[UP_RS], br_empty[UP_RS];
     __shared__ uint64_t acc_full[2], acc_empty[2], it_full[UP_IR], it_empty[UP_IR], fin;
     __shared__ UpItem<NC> rec[UP_IR];
     __shared__ uint32_t tmem_slot;
@@ -937,8 +1000,12 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
             mbar_init(&acc_empty[a], 256);
         }
         for (int a = 0; a < UP_AR; ++a) {
-            mbar_init(&ar_full[a], 64);
+            mbar_init(&ar_full[a], 1);
             mbar_init(&ar_empty[a], 128);
+        }
+        for (int a = 0; a < UP_RS; ++a) {
+            mbar_init(&br_full[a], 1);
+            mbar_init(&br_empty[a], 32);
         }
         for (int a = 0; a < UP_IR; ++a) {
             mbar_init(&it_full[a], 1);
@@ -952,9 +1019,9 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    const uint32_t smem0 = su32(um_smem);
+    const uint32_t smem0 = (su32(um_smem) + 1023u) & ~1023u;
     const uint32_t raw0 = smem0 + UP_NS * B_STAGE;
-    const uint32_t araw0 = raw0 + ((UP_RS * RAW_STAGE + 127u) & ~127u);
+    const uint32_t araw0 = raw0 + ((UP_RS * RAW_STAGE + 1023u) & ~1023u);
     // record n of the ring, for a whole warp; false when the wait gave up
     auto wait = [&](uint64_t *bar, uint32_t parity) -> bool { return up_wait<true>(bar, parity, limit, &abort_s); };
     auto item = [&](int n) -> bool { return wait(&it_full[n % UP_IR], (n / UP_IR) & 1); };
@@ -980,21 +1047,38 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                 const int cc = c + k, st = cc % UP_AR, sg = cc / UM_SEG, s = sg % UP_NS;
                 if (!(run = wait(&ar_full[st], (cc / UP_AR) & 1))) break;
                 const uint32_t src = araw0 + (uint32_t)st * A_STAGE + (uint32_t)row * EB;
-                float v[UM_KC];
+                const uint32_t ta = tl + COL_A + (uint32_t)(s * UM_SEG + grp) * (2u * UM_KC);
+                const int kv = snc - k * KQ;  // values past the block are zeroed (in its last, partial chunk)
 #pragma unroll
-                for (int j = 0; j < KQ; ++j) {
-                    if constexpr (W == 2) {
-                        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-                                     : "=f"(v[2 * j]), "=f"(v[2 * j + 1])
-                                     : "r"(src + (uint32_t)j * A_COL));
-                    } else {
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[j]) : "r"(src + (uint32_t)j * A_COL));
+                for (int h = 0; h < 2; ++h) {  // 16 values at a time
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16 / W; ++j) {
+                        const uint32_t sj = src + (uint32_t)(j + h * 16 / W) * A_COL;
+                        if constexpr (W == 2)
+                            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v[2 * j]), "=f"(v[2 * j + 1]) : "r"(sj));
+                        else
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[j]) : "r"(sj));
                     }
+                    uint32_t hi[16], lo[16];
+                    if (kv < KQ) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            if ((16 * h + e) / W >= kv) v[e] = 0.0f;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) split2(v[e], hi[e], lo[e]);
+                    if (h == 1) {
+                        mbar_arrive(&ar_empty[st]);
+                    } else {
+                        if (sg >= UP_NS && !(run = wait(&empty[s], ((sg / UP_NS) - 1) & 1))) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+                    tmem_st16(ta + 16u * h, hi);
+                    tmem_st16(ta + UM_KC + 16u * h, lo);
                 }
-                mbar_arrive(&ar_empty[st]);
-                if (sg >= UP_NS && !(run = wait(&empty[s], ((sg / UP_NS) - 1) & 1))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                up_store_split<W>(tl + COL_A + (uint32_t)(s * UM_SEG + grp) * (2u * UM_KC), v, snc - k * KQ);
+                if (!run) break;
+                tmem_wait_st();
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 mbar_arrive(&full[s]);
             }
@@ -1006,13 +1090,12 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(UP_REG_B));
         if (warp < UP_COPY) {
             // ---------------- moment warps: B operand into shared memory ----------------
-            // warp bw takes every fourth chunk on its own: copies it one turn ahead, waits for its own
-            // copies only and splits the whole chunk, so nothing but the operand stages ties the warps
+            // warp bw takes every fourth chunk on its own, so nothing but the stages ties the warps
             const int bw = warp - UP_B0;
             constexpr int EV = 16 / EB;  // elements per 16-byte piece
             const uint32_t S = 0x80000000u, s_re = adj ? 0u : S, s_im = adj ? S : 0u;
-            int in = 0, ik = bw, turn = 0;  // copy cursor: record, chunk of it, chunks copied
-            bool run = item(0), more = run;
+            int in = 0, ik = bw, turn = 0;  // copy cursor (cp.async): record, chunk of it, chunks copied
+            bool run = TMA || item(0), more = !TMA && run;
             // moves the cursor to the next record with a chunk for this warp (at once: a record is
             // reused after its last chunk)
             auto enter = [&]() {
@@ -1049,10 +1132,12 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                 ++turn;
                 ik += UP_BW;
             };
-            enter();
-            if (more) copy();
-            enter();
-            cp_commit_group();
+            if constexpr (!TMA) {
+                enter();
+                if (more) copy();
+                enter();
+                cp_commit_group();
+            }
             int c = 0;  // chunks of the records before record n
             for (int n = 0, done = 0; run; ++n) {
                 if (!(run = item(n))) break;
@@ -1060,15 +1145,19 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                 const int nk = it.nk, ncp = up_part<W>(it.ncol);
                 if (nk == 0) break;
                 for (int k = (bw - c) & (UP_BW - 1); k < nk; k += UP_BW, ++done) {
-                    if (more) copy();  // the next turn's, into the stage of the turn before this one
-                    enter();
-                    if (!run) break;
-                    cp_commit_group();
-                    cp_wait_group<1>();
-                    __syncwarp();
-                    const int cc = c + k, sg = cc / UM_SEG, s = sg % UP_NS;
+                    const int cc = c + k, sg = cc / UM_SEG, s = sg % UP_NS, rs = TMA ? cc % UP_RS : 2 * bw + (done & 1);
+                    if constexpr (TMA) {
+                        if (!(run = wait(&br_full[rs], (cc / UP_RS) & 1))) break;
+                    } else {
+                        if (more) copy();  // the next turn's, into the stage of the turn before this one
+                        enter();
+                        if (!run) break;
+                        cp_commit_group();
+                        cp_wait_group<1>();
+                        __syncwarp();
+                    }
                     if (sg >= UP_NS && !(run = wait(&empty[s], ((sg / UP_NS) - 1) & 1))) break;
-                    const uint32_t rb = raw0 + (uint32_t)(2 * bw + (done & 1)) * RAW_STAGE;
+                    const uint32_t rb = raw0 + (uint32_t)rs * RAW_STAGE;
                     const uint32_t hb = smem0 + (uint32_t)s * B_STAGE + (uint32_t)(cc % UM_SEG) * B_CHUNK;
                     const uint32_t lb = hb + UP_N * UM_KC * 4;
                     // lane: column (and column + 32 of a real tile)
@@ -1077,15 +1166,18 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                         const int q = lane + 32 * g2;
                         if (q >= ncp) continue;
                         const uint32_t o0 = goff(q, 0), oi0 = W == 2 ? goff(ncp + q, 0) : 0;
+                        // all of the column's loads before the first store
+                        float w[UM_KG][4];
+#pragma unroll
+                        for (int kg = 0; kg < UM_KG; ++kg)
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(w[kg][0]), "=f"(w[kg][1]), "=f"(w[kg][2]), "=f"(w[kg][3])
+                                         : "r"(rb + (uint32_t)q * RAW_ROW + (uint32_t)(TMA ? kg ^ (q & 7) : kg) * 16));
 #pragma unroll
                         for (int kg = 0; kg < UM_KG; ++kg) {
-                            float w[4];
-                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
-                                         : "r"(rb + (uint32_t)q * UM_RAWROW + (uint32_t)kg * 16));
                             uint32_t h[4], l[4];
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) split2(w[e], h[e], l[e]);
+                            for (int e = 0; e < 4; ++e) split2(w[kg][e], h[e], l[e]);
                             const uint32_t o = o0 + (uint32_t)kg * UM_LBO;
                             if constexpr (W == 1) {
                                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hb + o), "r"(h[0]),
@@ -1108,7 +1200,8 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     mbar_arrive(&full[s]);
-                    __syncwarp();  // the stage of this turn is copied into in the next one
+                    if constexpr (TMA) mbar_arrive(&br_empty[rs]);
+                    else __syncwarp();  // the stage of this turn is copied into in the next one
                 }
                 c += nk;
                 if (run) item_done(n);
@@ -1116,45 +1209,79 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
             if (!run) abort_s = 1;
             asm volatile("cp.async.wait_all;" ::: "memory");
         } else if (warp < UP_MMA) {
-            // ---------------- copy warps: the rows of a chunk's columns, UP_AR chunks ahead ----------------
-            const int cw = warp - UP_COPY;  // this warp copies every other column
-            constexpr int PC = (int)A_COL / 512;  // warp copies (32 x 16 bytes) per column
-            int c = 0;
+            // ---------------- copy warps: coupling columns UP_AR, moments UP_RS chunks ahead ----------------
             bool run = true;
-            for (int n = 0; run; ++n) {
-                if (!(run = item(n))) break;
-                const UpItem<NC> &it = rec[n % UP_IR];
-                const int nk = it.nk, snc = it.snc, ld = it.ld;
-                if (nk == 0) break;
-                const int *kmap = it.perm >= 0 ? m.perm + it.perm : nullptr;
-                const int bytes = it.rows * EB;  // a column's last 16 bytes may reach into its padding
-                const unsigned char *B = reinterpret_cast<const unsigned char *>(blocks + it.blk) + 16 * lane;
-                int col = lane < min(KQ, snc) ? (kmap ? __ldg(kmap + lane) : lane) : 0;
-                for (int k = 0; k < nk; ++k, ++c) {
-                    const int nv = min(KQ, snc - k * KQ), next = (k + 1) * KQ + lane;
-                    // the next chunk's columns, while this one's stage is waited for and filled
-                    const int coln = lane < KQ && next < snc ? (kmap ? __ldg(kmap + next) : next) : 0;
-                    const int st = c % UP_AR;
-                    int off[KQ / 2];  // byte offsets of this warp's columns
+            int c = 0;
+            if (warp == UP_COPY) {
+                for (int n = 0; run; ++n) {
+                    if (!(run = item(n))) break;
+                    const UpItem<NC> &it = rec[n % UP_IR];
+                    const int nk = it.nk, snc = it.snc, col0 = it.col, x0 = it.m0 * W;
+                    if (nk == 0) break;
+                    // lane j: the columns 4 j .. 4 j + 3 of a chunk (past the block: its last one), loaded a
+                    // chunk before they are used
+                    const int *kmap = it.perm >= 0 ? m.perm + it.perm : nullptr;
+                    auto columns = [&](int k) -> int4 {
+                        int r[4];
 #pragma unroll
-                    for (int j = 0; j < KQ / 2; ++j) off[j] = __shfl_sync(0xffffffffu, col, 2 * j + cw) * (ld * EB);
-                    if (c >= UP_AR && !(run = wait(&ar_empty[st], ((c / UP_AR) - 1) & 1))) break;
-                    const uint32_t dst = araw0 + (uint32_t)st * A_STAGE + 16u * lane + (uint32_t)cw * A_COL;
-#pragma unroll
-                    for (int h = 0; h < PC; ++h)
-                        if (16 * lane + 512 * h < bytes) {
-#pragma unroll
-                            for (int j = 0; j < KQ / 2; ++j)
-                                if (2 * j + cw < nv)
-                                    cp16_cg(dst + (uint32_t)(2 * j) * A_COL + 512u * h, B + off[j] + 512 * h, true);
+                        for (int e = 0; e < 4; ++e) {
+                            const int kk = min(k * KQ + 4 * lane + e, snc - 1);
+                            r[e] = kmap ? __ldg(kmap + kk) : kk;
                         }
-                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(su32(&ar_full[st])) : "memory");
-                    col = coln;
+                        return make_int4(r[0], r[1], r[2], r[3]);
+                    };
+                    int4 r = make_int4(0, 0, 0, 0), next = r;
+                    if (lane < KQ / 4) r = columns(0);
+                    for (int k = 0; k < nk; ++k, ++c) {
+                        const int groups = (min(KQ, snc - k * KQ) + 3) / 4, st = c % UP_AR;
+                        if (k + 1 < nk && lane < KQ / 4) next = columns(k + 1);
+                        if (c >= UP_AR && !(run = wait(&ar_empty[st], ((c / UP_AR) - 1) & 1))) break;
+                        if (lane == 0) mbar_expect_tx(&ar_full[st], (uint32_t)(4 * groups) * A_COL);
+                        __syncwarp();
+                        if (lane < groups)
+                            tma_gather4(araw0 + (uint32_t)st * A_STAGE + (uint32_t)lane * (4 * A_COL), &blocks, x0,
+                                        make_int4(r.x + col0, r.y + col0, r.z + col0, r.w + col0), &ar_full[st]);
+                        __syncwarp();
+                        r = next;
+                    }
+                    if (run) item_done(n);
                 }
-                item_done(n);
+                // copies in flight write this CTA's shared memory: all have landed before the CTA can exit
+                for (int cc = max(0, c - UP_AR); cc < c; ++cc) mbar_wait(&ar_full[cc % UP_AR], (cc / UP_AR) & 1, UM_SPIN_FINAL);
+            } else {
+                for (int n = 0; run; ++n) {
+                    if (!(run = item(n))) break;
+                    const UpItem<NC> &it = rec[n % UP_IR];
+                    const int nk = it.nk, rb = TMA ? g.rowbox : 1, groups = (it.ncol + rb - 1) / rb;
+                    if (nk == 0) break;
+                    if constexpr (TMA) {
+                        // lane j: rows j rb .. of the item's columns, in one box of rb rows (rb right-hand sides
+                        // of a pair lie side by side) or, rb = 4, four rows named one by one
+                        int4 r = make_int4(0, 0, 0, 0);
+                        if (lane < groups) {
+                            const int64_t *src = it.src + lane * rb;
+                            r = make_int4((int)src[0], (int)src[1], (int)src[2], (int)src[3]);
+                        }
+                        const uint32_t dst = raw0 + (uint32_t)(lane * rb) * RAW_ROW, bytes = (uint32_t)(groups * rb) * RAW_ROW;
+                        for (int k = 0; k < nk; ++k, ++c) {
+                            const int st = c % UP_RS;
+                            if (c >= UP_RS && !(run = wait(&br_empty[st], ((c / UP_RS) - 1) & 1))) break;
+                            if (lane == 0) mbar_expect_tx(&br_full[st], bytes);
+                            __syncwarp();
+                            if (lane < groups) {
+                                if (rb == 4) tma_gather4(dst + (uint32_t)st * RAW_STAGE, &moments, k * UM_KC, r, &br_full[st]);
+                                else tma_box(dst + (uint32_t)st * RAW_STAGE, &moments, k * UM_KC, r.x, &br_full[st]);
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    if (run) item_done(n);
+                }
+                if constexpr (TMA)
+                    for (int cc = max(0, c - UP_RS); cc < c; ++cc)
+                        mbar_wait(&br_full[cc % UP_RS], (cc / UP_RS) & 1, UM_SPIN_FINAL);
             }
             if (!run) abort_s = 1;
-            asm volatile("cp.async.wait_all;" ::: "memory");
         } else if (warp == UP_MMA) {
             // ---------------- MMA warp: converged, one lane issues ----------------
             int sg = 0;  // segments so far
@@ -1193,36 +1320,42 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
             umma_commit_if(el, &fin);  // products already issued may still read the operands (see the end)
         } else if (warp == UP_SCHED) {
             // ---------------- scheduler: item records ----------------
-            const int items = g.ntiles * g.mt * g.zt;
-            int n = 0;
+            // Column tile z of the tiles with more than z NC / qn pairs (they come first), row tile by row
+            // tile: the grid's stride deals these out evenly. (z, its first item, its tiles) move along.
+            int n = 0, z = 0, first = 0, nz = g.more[0];
             bool run = true;
             for (int id = blockIdx.x; run; id += gridDim.x) {
-                const bool end = id >= items;
-                // column tiles slowest: every tile has a first one, fewer have the later ones, and a stride
-                // of the grid's CTAs meets them evenly
-                const int m0 = (id % g.mt) * UM_M, rest = id / g.mt, t = g.tile0 + rest % g.ntiles, z = rest / g.ntiles;
+                while (nz > 0 && id - first >= nz * g.mt) {
+                    first += nz * g.mt;
+                    const int64_t least = (int64_t)++z * NC / g.qn;
+                    nz = least < PAIR_TILE ? g.more[least] : 0;
+                }
+                const bool end = nz == 0;
+                const int t = g.tile0 + (end ? 0 : (id - first) % nz), m0 = end ? 0 : (id - first) / nz * UM_M;
                 int4 tl = make_int4(0, 0, 0, 0);
                 if (!end) {
                     tl = __ldg(g.tile + t);
-                    if (z * NC >= tl.y * g.qn || m0 >= tl.z) continue;
+                    if (m0 >= tl.z) continue;
                 }
                 UpItem<NC> &it = rec[n % UP_IR];
                 if (n >= UP_IR && !(run = wait(&it_empty[n % UP_IR], ((n / UP_IR) - 1) & 1))) break;
                 if (!end) {
                     const int ncol = min(NC, tl.y * g.qn - z * NC);
-                    for (int c = lane; c < ncol; c += 32) {
-                        const int f = z * NC + c, p = __ldg(g.pair + tl.x + f / g.qn), q = f % g.qn;
-                        it.src[c] = __ldg(r.pair_src + p) * g.nrhs + (int64_t)(g.q0 + q) * tl.w;
-                        it.out[c] = ((int64_t)(p - g.pbase) * g.qn + q) * g.pstride + m0;
+                    for (int c = lane; c < NC; c += 32) {  // past the columns: the last one again
+                        const int f = z * NC + min(c, ncol - 1), q = f % g.qn;
+                        const int4 rc = __ldg(g.rec + tl.x + f / g.qn);
+                        const int64_t src = (int64_t)rc.y << 32 | (uint32_t)rc.x;
+                        it.src[c] = TMA ? src / tl.w * g.nrhs + g.q0 + q : src * g.nrhs + (int64_t)(g.q0 + q) * tl.w;
+                        it.out[c] = ((int64_t)(rc.w - g.pbase) * g.qn + q) * g.pstride + m0;
                     }
                     if (lane == 0) {
                         it.ncol = ncol;
                         it.snc = tl.w;
                         it.rows = min(UM_M, tl.z - m0);
-                        it.ld = up_ld<T>(tl.z);
-                        it.blk = __ldg(g.tile_off + t) + m0;
+                        it.m0 = m0;
+                        it.col = (int)(__ldg(g.tile_off + t) / g.ld);
                         // k -> stored column: the column permutation inverted forward, else the row permutation
-                        const int64_t ps = r.pair_perm ? __ldg(r.pair_perm + __ldg(g.pair + tl.x)) : -1;
+                        const int ps = __ldg(g.rec + tl.x).z;
                         it.perm = ps < 0 ? -1 : ps + (fwd ? 3 * tl.w : tl.w);
                     }
                 }
@@ -1259,17 +1392,17 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                 if (!(run = wait(&acc_full[a], (gs >> 1) & 1))) break;
                 if (mine) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    uint32_t f[16];
-                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part0, f);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) sum[0][e] += (double)__uint_as_float(f[e]);
-                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part1, f);
+                    uint32_t f0[16], f1[16];
+                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part0, f0);
+                    tmem_ld16(tl + (uint32_t)(a * UP_N) + part1, f1);
                     tmem_wait_ld();
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     mbar_arrive(&acc_empty[a]);
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) sum[1][e] += (double)__uint_as_float(f[e]);
+                    for (int e = 0; e < 16; ++e) {
+                        sum[0][e] += (double)__uint_as_float(f0[e]);
+                        sum[1][e] += (double)__uint_as_float(f1[e]);
+                    }
                 } else {
                     mbar_arrive(&acc_empty[a]);
                 }
@@ -1280,7 +1413,7 @@ i2o_umma_pairs_kernel(DMap m, DSide r, UpArgs g, const T *__restrict__ blocks, c
                 for (int e = 0; e < HC; ++e) {
                     const int c = half * HC + e;
                     if (c >= ncol) break;
-                    if constexpr (W == 2) prod[it.out[c] + row] = cdouble{sum[0][e], sum[1][e]};
+                    if constexpr (W == 2) stv(prod + it.out[c] + row, cdouble{sum[0][e], sum[1][e]});
                     else prod[it.out[c] + row] = sum[e / 16][e % 16];
                 }
             }
@@ -1304,8 +1437,30 @@ bool i2o_umma_eligible(bool cplx, int precision, const DMap &m, int nq) {
     return precision == H2B_FP32 && m.coupling_kind == H2B_COUPLING_DENSE && (cplx ? 2 : 1) * nq >= 4;
 }
 
+// A 2-D tensor map of `rows` rows of `inner` FP32 values, `stride` bytes apart, for boxes of `boxrows`
+// rows of `box` values (1: gathers of four rows).
+static cudaError_t up_map(CUtensorMap *map, const void *base, uint64_t inner, uint64_t rows, uint64_t stride,
+                          uint32_t box, uint32_t boxrows, bool swizzle) {
+    static const auto encode = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {inner, rows}, strides[1] = {stride};
+    const cuuint32_t boxes[2] = {box, boxrows}, ones[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims, strides, boxes, ones,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const DSide &src, const int *nodes,
-                            int nnodes, const FarArgs &fa, int maxcoef, cudaStream_t st) {
+                            int nnodes, const FarArgs &fa, int maxcoef, const PairTiles *pt, cudaStream_t st) {
     if (nnodes == 0) return cudaSuccess;
     const int nq = m.ncomp * fa.nrhs;
     const int ntmax = cplx ? UM_NT_MAX_CPLX : UM_NT_MAX_REAL;
@@ -1318,7 +1473,18 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
     // expanded moment stages (hi and lo), the raw moment ring and the coupling column stages
     const size_t eb = cplx ? 8 : 4, kq = cplx ? UM_KC / 2 : UM_KC;
     const size_t raw = ((size_t)UM_RS * qt_max * UM_RAWROW + 127) & ~(size_t)127;
-    const size_t acols = (size_t)UM_AR * ((kq * maxcoef * eb + 127) & ~(size_t)127);
+    // whole columns of stored blocks, one shape, four to a gather: columns of at most 256 FP32 values,
+    // multiples of 32 bytes apart
+    const int W = cplx ? 2 : 1, ld = pt ? pt->nc32 : 0;
+    const int pitch = (ld * W * 4 + 31) / 32 * 32;
+    const bool tma = pt && pt->stored32 && pitch <= 1024;
+    CUtensorMap blocks{};
+    if (tma) {
+        const cudaError_t em = up_map(&blocks, pt->blocks32, (uint64_t)ld * W, (uint64_t)pt->cols32, (uint64_t)ld * W * 4,
+                                      pitch / 4, 1, false);
+        if (em != cudaSuccess) return em;
+    }
+    const size_t acols = (size_t)UM_AR * ((kq * (tma ? (size_t)pitch : maxcoef * eb) + 127) & ~(size_t)127);
     size_t smem = (size_t)UM_NS * 2 * np * UM_KC * 4 + raw;
     // the coupling column stages grow with the block size; blocks whose stages do not fit beside
     // the moment stages are read by the register path instead
@@ -1327,7 +1493,8 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
     if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e0 != cudaSuccess) return e0;
     DMap mm = m;
-    if (mm.cpl_vec && smem + acols + 1024 <= (size_t)optin)
+    const bool fits = smem + acols + 1024 <= (size_t)optin;
+    if ((tma || mm.cpl_vec) && fits)
         smem += acols;
     else
         mm.cpl_vec = 0;
@@ -1335,12 +1502,18 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
     auto go = [&](auto kern, auto *am, auto *dm) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<grid, UM_THREADS, smem, st>>>(mm, recv, src, nodes, fa.mode, fa.nrhs, qt_max, am, dm);
+        kern<<<grid, tma && fits ? UM_THREADS + 32 : UM_THREADS, smem, st>>>(mm, recv, src, nodes, fa.mode, fa.nrhs, qt_max,
+                                                                            am, dm, blocks, pitch, std::max(ld, 1));
         return cudaGetLastError();
     };
-    if (cplx)
-        return go(&i2o_umma_kernel<cfloat>, static_cast<const cfloat *>(fa.am), static_cast<cfloat *>(fa.dm));
-    return go(&i2o_umma_kernel<float>, static_cast<const float *>(fa.am), static_cast<float *>(fa.dm));
+    if (cplx) {
+        const cfloat *am = static_cast<const cfloat *>(fa.am);
+        cfloat *dm = static_cast<cfloat *>(fa.dm);
+        return tma && fits ? go(&i2o_umma_kernel<cfloat, true>, am, dm) : go(&i2o_umma_kernel<cfloat, false>, am, dm);
+    }
+    const float *am = static_cast<const float *>(fa.am);
+    float *dm = static_cast<float *>(fa.dm);
+    return tma && fits ? go(&i2o_umma_kernel<float, true>, am, dm) : go(&i2o_umma_kernel<float, false>, am, dm);
 }
 
 bool i2o_umma_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes) {
@@ -1355,33 +1528,54 @@ cudaError_t launch_i2o_umma_pairs(bool cplx, const DMap &m, const DSide &recv, c
     cudaError_t err = cudaGetDevice(&dev);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (err != cudaSuccess) return err;
-    const int cols = UP_N / (cplx ? 2 : 1);
-    const size_t raw = ((size_t)UP_RS * cols * UM_RAWROW + 127) & ~(size_t)127;
+    const int W = cplx ? 2 : 1, cols = UP_N / W, nc = pt.nc32, snc = pt.snc32;
+    const int ld = cplx ? up_ld<cfloat>(nc) : up_ld<float>(nc);
+    // bytes of a copied block column: 128 rows, or the whole block's in multiples of 32 (four columns to a
+    // gather, whose destination is 128-byte aligned)
+    const int pitch = std::min(UM_M * W, (ld * W + 7) / 8 * 8) * 4;
+    // moment columns of whole 16 bytes are gathered, others copied element by element
+    const bool tma = (snc * W * 4) % 16 == 0;
+    CUtensorMap blocks{}, moments{};
+    err = up_map(&blocks, pt.blocks32, (uint64_t)ld * W, (uint64_t)pt.cols32, (uint64_t)ld * W * 4, pitch / 4, 1, false);
+    // right-hand sides per pass, and how many of one pair's lie side by side in every tile's columns: they
+    // are copied as one box of rows
+    const int qc = (int)std::min<int64_t>(std::min(nq, 1024), (int64_t)fa.prod_bytes / (pt.unit_elems * (cplx ? 16 : 8)));
+    int rowbox = 4;
+    for (int b = cols; b >= 8 && rowbox == 4; b /= 2)
+        if (qc % b == 0 && nq % b == 0) rowbox = b;
+    if (err == cudaSuccess && tma)
+        err = up_map(&moments, fa.am, (uint64_t)snc * W, (uint64_t)pt.src_cols * fa.nrhs, (uint64_t)snc * W * 4, UM_KC,
+                     rowbox == 4 ? 1 : rowbox, true);
+    if (err != cudaSuccess) return err;
+    const size_t raw = ((size_t)UP_RS * cols * (tma ? up_raw_row<true>() : up_raw_row<false>()) + 1023) & ~(size_t)1023;
     const size_t smem = (size_t)UP_NS * UM_SEG * 2 * UP_N * UM_KC * 4 + raw +
-                        (size_t)(cplx ? up_ar<2>() : up_ar<1>()) * UM_KC * 4 * UM_M;
-    auto go = [&](auto kern, const auto *blocks, const auto *am, auto *prod) {
+                        (size_t)(cplx ? up_ar<2>() : up_ar<1>()) * UM_KC * 4 * UM_M + 1024;
+    auto go = [&](auto kern, const auto *am, auto *prod) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        const int64_t unit = pt.unit_elems * (int64_t)sizeof(*prod);
-        const int qc = (int)std::min<int64_t>(std::min(nq, 1024), (int64_t)fa.prod_bytes / unit);
         for (const PairUnit &u : pt.units)
             for (int q0 = 0; q0 < nq; q0 += qc) {
                 const int qn = std::min(qc, nq - q0);
-                UpArgs g{pt.pair, pt.tile32, pt.tile32_off, u.tile32_0, u.ntiles32, (u.maxpairs32 * qn + cols - 1) / cols,
-                         (maxcoef + UM_M - 1) / UM_M, fa.mode, fa.nrhs, q0, qn, u.p0, pt.pstride};
-                const int64_t items = (int64_t)g.ntiles * g.zt * g.mt;
+                UpArgs g{pt.rec, pt.tile32, pt.tile32_off, u.tile32_0, (nc + UM_M - 1) / UM_M, {}, fa.mode, fa.nrhs, q0, qn,
+                         u.p0, pt.pstride, ld, pitch, rowbox};
+                int64_t items = 0;
+                std::copy(u.more32, u.more32 + PAIR_TILE, g.more);
+                for (int64_t z = 0; z * cols / qn < PAIR_TILE; ++z) items += (int64_t)g.more[z * cols / qn] * g.mt;
                 if (items > INT32_MAX) return cudaErrorInvalidValue;
-                kern<<<(unsigned)std::min<int64_t>(nsm, items), UP_THREADS, smem, st>>>(m, recv, g, blocks, am, prod);
+                kern<<<(unsigned)std::min<int64_t>(nsm, items), UP_THREADS, smem, st>>>(m, g, blocks, moments, am, prod);
                 e = launch_i2o_pairs_sum(cplx, H2B_FP32, m, recv, pt, u, fa, maxcoef, q0, qn, st);
                 if (e != cudaSuccess) return e;
             }
         return cudaGetLastError();
     };
-    if (cplx)
-        return go(&i2o_umma_pairs_kernel<cfloat>, static_cast<const cfloat *>(pt.blocks32),
-                  static_cast<const cfloat *>(fa.am), static_cast<cdouble *>(fa.prod));
-    return go(&i2o_umma_pairs_kernel<float>, static_cast<const float *>(pt.blocks32), static_cast<const float *>(fa.am),
-              static_cast<double *>(fa.prod));
+    if (cplx) {
+        const cfloat *am = static_cast<const cfloat *>(fa.am);
+        cdouble *prod = static_cast<cdouble *>(fa.prod);
+        return tma ? go(&i2o_umma_pairs_kernel<cfloat, true>, am, prod) : go(&i2o_umma_pairs_kernel<cfloat, false>, am, prod);
+    }
+    const float *am = static_cast<const float *>(fa.am);
+    double *prod = static_cast<double *>(fa.prod);
+    return tma ? go(&i2o_umma_pairs_kernel<float, true>, am, prod) : go(&i2o_umma_pairs_kernel<float, false>, am, prod);
 }
 
 cudaError_t read_umma_timeouts(unsigned *count) {
