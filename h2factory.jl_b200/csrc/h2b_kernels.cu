@@ -28,13 +28,6 @@ __device__ __forceinline__ int ncoef_of(const DSide &s, int lvl) {
     return s.shape[3 * lvl] * s.shape[3 * lvl + 1] * s.shape[3 * lvl + 2];
 }
 
-// Bound on every intermediate of a separable contraction between levels lp and lp + 1.
-__device__ __forceinline__ int sep_bound(const DSide &s, int lp) {
-    int b = 1;
-    for (int d = 0; d < 3; ++d) b *= max(s.shape[3 * lp + d], s.shape[3 * (lp + 1) + d]);
-    return b;
-}
-
 // ---------------------------------------------------------------------------------------------
 // Per-node small products on all right-hand sides at once: acc (+)= op(M) X over a tile of at most
 // TG_M output rows and TG_Q right-hand sides. op(M)[i, k] = M[i + k*ldm] (trans = false) or
@@ -230,18 +223,6 @@ __device__ __forceinline__ void warp_acc_store(const double (&acc)[8][2][2], int
             }
 }
 
-// op(M)[i, k] = M[i + k*ldm] (trans = false) or M[k + i*ldm] (trans = true), conjugated when cjg.
-template <class T, class A, class XLoad>
-__device__ __forceinline__ void tile_gemm(const T *__restrict__ M, int64_t ldm, bool trans, bool cjg, int m0,
-                                          int mt, int kk, int nq, XLoad xload, A *Ms, A *Xs, A (&acc)[TG_O]) {
-    if (trans)
-        tile_gemm_l(true, m0, mt, kk, nq, [&](int i, int k) -> A { return wide(cj(M[k + (int64_t)i * ldm], cjg)); },
-                    xload, Ms, Xs, acc);
-    else
-        tile_gemm_l(false, m0, mt, kk, nq, [&](int i, int k) -> A { return wide(cj(M[i + (int64_t)k * ldm], cjg)); },
-                    xload, Ms, Xs, acc);
-}
-
 template <class A>
 __device__ __forceinline__ void tile_zero(A (&acc)[TG_O]) {
 #pragma unroll
@@ -253,10 +234,61 @@ template <class A>
 constexpr size_t tile_smem() { return (size_t)(TG_M * TG_LD + TG_K * TG_Q) * sizeof(A); }
 
 // ---------------------------------------------------------------------------------------------
-// A1: m_leaf[c][r] = op(C_c) x[values]   (op = conj for adjoint maps with conjugating leaves);
-// RCH right-hand sides share each pass over the collection
+// A1: m_leaf[c][r] = op(C_c) x[values]   (op = conj for adjoint maps with conjugating leaves).
+//
+// One right-hand side: each collection entry is read once and used once, so a CTA streams its leaf's
+// columns: threads over the rows (contiguous), the columns dealt to the CTA's row groups, eight loads
+// in flight per thread, x in shared memory. Bound: HBM.
 // ---------------------------------------------------------------------------------------------
-template <class T, class V, bool MMA>
+constexpr int LEAF_XS = 256;  // values of x staged at a time
+
+template <class T, class V>
+__global__ void __launch_bounds__(256)
+leaf_aggregate_vec_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, const V *__restrict__ x,
+                          T *__restrict__ am) {
+    using A = typename ScalarTraits<T>::Acc;  // == V
+    __shared__ __align__(16) A xs[LEAF_XS], part[256];
+    const int leaf = leaves[blockIdx.x];
+    const int nc = ncoef_of(s, s.level[leaf]);
+    const int v0 = s.value_ptr[leaf], nv = s.value_ptr[leaf + 1] - v0;
+    const T *C = static_cast<const T *>(s.coll) + s.coll_off[leaf];
+    T *mom = am + s.mom_off[leaf];
+    const int rows = min(256, (nc + 31) / 32 * 32), groups = 256 / rows;
+    const int g = threadIdx.x / rows, r = threadIdx.x - g * rows;
+    for (int c = 0; c < m.ncomp; ++c)
+        for (int m0 = 0; m0 < nc; m0 += rows) {
+            const T *Cc = C + (int64_t)c * nc * nv + m0 + r;
+            const bool live = g < groups && m0 + r < nc;
+            A acc = sc_zero<A>();
+            for (int k0 = 0; k0 < nv; k0 += LEAF_XS) {
+                const int kn = min(LEAF_XS, nv - k0);
+                __syncthreads();
+                for (int k = threadIdx.x; k < kn; k += 256) xs[k] = x[s.value[v0 + k0 + k]];
+                __syncthreads();
+                if (live) {
+                    int k = g;
+                    for (; k + 7 * groups < kn; k += 8 * groups) {
+                        T v[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) v[u] = ldv(Cc + (int64_t)(k0 + k + u * groups) * nc);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) acc = acc + wide(cj(v[u], conjc)) * ldv(xs + k + u * groups);
+                    }
+                    for (; k < kn; k += groups) acc = acc + wide(cj(ldv(Cc + (int64_t)(k0 + k) * nc), conjc)) * ldv(xs + k);
+                }
+            }
+            if (groups > 1) {
+                part[threadIdx.x] = acc;
+                __syncthreads();
+                if (g == 0)
+                    for (int u = 1; u < groups; ++u) acc = acc + part[u * rows + r];
+            }
+            if (g == 0 && live) narrow(acc, mom[(int64_t)c * nc + m0 + r]);
+        }
+}
+
+// Blocks of right-hand sides: 64 x 16 tiles on the FP64 tensor cores.
+template <class T, class V>
 __global__ void __launch_bounds__(256)
 leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, int nrhs,
                       const V *__restrict__ x, int64_t ldx, T *__restrict__ am) {
@@ -274,19 +306,6 @@ leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conj
             for (int m0 = 0; m0 < nc; m0 += TG_M) {
                 const int mt = min(TG_M, nc - m0);
                 const T *Cc = C + (int64_t)c * nc * nv;
-                if constexpr (!MMA) {  // one right-hand side: FMA tile (an MMA would idle 7 of 8 columns)
-                    A acc[TG_O];
-                    tile_zero(acc);
-                    tile_gemm(Cc, nc, false, conjc, m0, mt, nv, nq,
-                              [&](int k, int q) -> A { return x[(int64_t)(q0 + q) * ldx + s.value[v0 + k]]; },
-                              Ms, Xs, acc);
-#pragma unroll
-                    for (int j = 0; j < TG_O; ++j) {
-                        const int o = threadIdx.x + j * blockDim.x;
-                        if (o < mt * nq)
-                            narrow(acc[j], mom[((int64_t)c * nrhs + q0 + o / mt) * nc + m0 + o % mt]);
-                    }
-                } else {
                 MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
                 acc.zero();
                 tile_gemm_mma_l(false, m0, mt, nv, nq,
@@ -296,75 +315,31 @@ leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conj
                 mma_store(acc, mt, nq, [&](int i, int q, A v) {
                     narrow(v, mom[((int64_t)c * nrhs + q0 + q) * nc + m0 + i]);
                 });
-                }
             }
         }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Separable contraction of one moment component in shared memory: out (+)= op(M_dim..M_1) in,
-// axes from `dim` down to 1 (src/maps/leveltranslator.jl:200-265). op: transposed factors when
-// `tr`, conjugated when `cjg`. Factor ax is stored sp[ax] x sc[ax] (parent x child), column-major.
-// Buffers a, b hold max(prod(fin), prod(fout)) elements; in is consumed from `a`.
-// ---------------------------------------------------------------------------------------------
-template <class T, class A, class O>
-__device__ void separable_block(const T *M, const int *sp, const int *sc, int dim, bool up, bool cjg,
-                                A *a, A *b, O *out, bool accumulate) {
-    int cur[3], fin[3], fout[3];
-    for (int d = 0; d < 3; ++d) {
-        fin[d] = up ? sc[d] : sp[d];
-        fout[d] = up ? sp[d] : sc[d];
-        cur[d] = fin[d];
-    }
-    const T *fac[3];
-    int64_t o = 0;
-    for (int d = 0; d < dim; ++d) {
-        fac[d] = M + o;
-        o += (int64_t)sp[d] * sc[d];
-    }
-    for (int ax = dim - 1; ax >= 0; --ax) {
-        int nxt[3] = {cur[0], cur[1], cur[2]};
-        nxt[ax] = fout[ax];
-        const int total = nxt[0] * nxt[1] * nxt[2];
-        const int ld = sp[ax];
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-            int idx[3] = {e % nxt[0], (e / nxt[0]) % nxt[1], e / (nxt[0] * nxt[1])};
-            const int row = idx[ax];
-            A acc = sc_zero<A>();
-            for (int k = 0; k < cur[ax]; ++k) {
-                int src[3] = {idx[0], idx[1], idx[2]};
-                src[ax] = k;
-                // up: op(M)[row,k] = M[row + k*ld]; down: M^T[row,k] = M[k + row*ld]
-                const T mk = up ? fac[ax][row + k * ld] : fac[ax][k + row * ld];
-                acc = acc + wide(cj(mk, cjg)) * a[src[0] + cur[0] * (src[1] + cur[1] * src[2])];
-            }
-            b[e] = acc;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < total; e += blockDim.x) a[e] = b[e];
-        __syncthreads();
-        cur[0] = nxt[0]; cur[1] = nxt[1]; cur[2] = nxt[2];
-    }
-    const int total = fout[0] * fout[1] * fout[2];
-    for (int e = threadIdx.x; e < total; e += blockDim.x) narrow(accumulate ? wide(out[e]) + a[e] : a[e], out[e]);
-    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------------------------
 // Separable level transfers (SeparableI2I, src/maps/leveltranslator.jl:168-265) on blocks of
-// right-hand sides: one CTA per parent (upward: m_p = sum over children of op(T_c) m_c, first child
-// overwriting) or per child (downward: l_c (+)= op(T_c)^T l_p, accumulating where the child already
-// received I2O contributions). A chunk of `qc` moment columns is contracted axis by axis in
-// shared memory (axes dim .. 1, one barrier per axis, ping-pong buffers); each thread computes
-// whole output elements of the axis pass, so the work of one barrier is qc times that of one column.
+// right-hand sides: one CTA per (parent, chunk of moment columns) upward (m_p = sum over children of
+// op(T_c) m_c in child order, first child overwriting), per (child, chunk) downward (l_c (+)=
+// op(T_c)^T l_p, accumulating where the child already received I2O contributions). Upward, every
+// child's columns are contracted side by side, so an axis pass (dim .. 1, ping-pong buffers in shared
+// memory, one barrier each) is shared by all of them; the children are summed at the end.
+//
+// What bounds it: the chain of a level's axis passes, each one barrier and one column of factor and
+// moment loads from shared memory, and the levels after one another. Measured upward on the level of
+// 64 parents, 216 complex coefficients, FP64: 1 right-hand side 41 us when children and column chunks
+// followed one another in one CTA per parent.
 // ---------------------------------------------------------------------------------------------
+constexpr int SEP_CHILDREN = 64;  // children contracted side by side at most
+
 template <class T, bool UP>
 __global__ void __launch_bounds__(256)
 transfer_sep_kernel(DMap m, DSide s, const int *__restrict__ nodes, const uint8_t *__restrict__ received,
-                    bool conjt, int nrhs, T *__restrict__ mom, int qc_max, int bufsz) {
+                    bool conjt, int nrhs, T *__restrict__ mom, int qbase, int qc_max, int cg, int bufsz) {
     using A = typename ScalarTraits<T>::Acc;
-    extern __shared__ unsigned char smem_raw[];
-    A *X = reinterpret_cast<A *>(smem_raw), *Y = X + (size_t)qc_max * bufsz, *Acc = Y + (size_t)qc_max * bufsz;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int node = nodes[blockIdx.x];
     const int lp = UP ? s.level[node] : s.level[node] - 1, lc = lp + 1;
     const int *sp = &s.shape[3 * lp], *sc = &s.shape[3 * lc];
@@ -374,72 +349,70 @@ transfer_sep_kernel(DMap m, DSide s, const int *__restrict__ nodes, const uint8_
         fout[d] = UP ? sp[d] : sc[d];
     }
     const int nin = fin[0] * fin[1] * fin[2], nout = fout[0] * fout[1] * fout[2];
-    const int nq = m.ncomp * nrhs;
+    const int nq = m.ncomp * nrhs, q0 = qbase + blockIdx.y * qc_max, qc = min(qc_max, nq - q0);
     const int c0 = UP ? s.child_ptr[node] : 0, c1 = UP ? s.child_ptr[node + 1] : 1;
-    T *dst = mom + s.mom_off[node] * nrhs;
+    A *bufs = reinterpret_cast<A *>(smem_raw), *Acc = bufs + 2 * (size_t)cg * qc_max * bufsz;
+    __shared__ const T *fac[3][SEP_CHILDREN];   // per child: its factor along each axis
+    __shared__ const T *from[SEP_CHILDREN];     // per child: the columns it contributes
+    T *dst = mom + s.mom_off[node] * nrhs + (int64_t)q0 * nout;
     const bool acc_dst = !UP && received[node] != 0;
-    for (int q0 = 0; q0 < nq; q0 += qc_max) {
-        const int qc = min(qc_max, nq - q0);
-        A *res = X;
-        for (int k = c0; k < c1; ++k) {
-            const int ch = UP ? s.child[k] : node;  // the transfer belongs to the child
-            const T *src = UP ? mom + s.mom_off[ch] * nrhs : mom + s.mom_off[s.parent[node]] * nrhs;
+    for (int k0 = c0; k0 < c1; k0 += cg) {  // cg children at a time: all of them unless they are large
+        const int nch = min(cg, c1 - k0);
+        A *X = bufs, *Y = X + (size_t)cg * qc_max * bufsz;
+        int cur[3] = {fin[0], fin[1], fin[2]};
+        if (threadIdx.x < nch) {
+            const int ch = UP ? s.child[k0 + threadIdx.x] : node;  // the transfer belongs to the child
             const T *M = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
-            const T *fac[3];
-            int64_t o = 0;
             for (int d = 0; d < m.dim; ++d) {
-                fac[d] = M + o;
-                o += (int64_t)sp[d] * sc[d];
+                fac[d][threadIdx.x] = M;
+                M += sp[d] * sc[d];
             }
-            for (int e = threadIdx.x; e < qc * nin; e += blockDim.x) {
-                const int q = e / nin, i = e - q * nin;
-                X[q * bufsz + i] = wide(src[(int64_t)(q0 + q) * nin + i]);
+            from[threadIdx.x] = mom + s.mom_off[UP ? ch : s.parent[node]] * nrhs + (int64_t)q0 * nin;
+        }
+        __syncthreads();
+        const int ncol = nch * qc;  // column q of child k: k qc + q
+        for (int e = threadIdx.x; e < ncol * nin; e += blockDim.x) {
+            const int c = e / nin, i = e - c * nin, k = c / qc;
+            stv(X + c * bufsz + i, wide(ldv(from[k] + (int64_t)(c - k * qc) * nin + i)));
+        }
+        __syncthreads();
+        for (int ax = m.dim - 1; ax >= 0; --ax) {
+            int nxt[3] = {cur[0], cur[1], cur[2]};
+            nxt[ax] = fout[ax];
+            const int tot = nxt[0] * nxt[1] * nxt[2], ld = sp[ax], kk = cur[ax];
+            const int sstr = ax == 0 ? 1 : (ax == 1 ? cur[0] : cur[0] * cur[1]);  // input stride along ax
+            for (int e = threadIdx.x; e < ncol * tot; e += blockDim.x) {
+                const int c = e / tot, f = e - c * tot;
+                const int i0 = f % nxt[0], r = f / nxt[0], i1 = r % nxt[1], i2 = r / nxt[1];
+                const int row = ax == 0 ? i0 : (ax == 1 ? i1 : i2);
+                // the input index with i[ax] = 0
+                const A *in = X + c * bufsz + i0 + cur[0] * (i1 + cur[1] * i2) - row * sstr;
+                const T *F = fac[ax][UP ? c / qc : 0];
+                A acc = sc_zero<A>();
+                for (int j = 0; j < kk; ++j) {
+                    // up: op(M)[row, j] = M[row + j ld]; down: M^T[row, j] = M[j + row ld]
+                    const T mk = ldv(UP ? F + row + j * ld : F + j + row * ld);
+                    acc = acc + wide(cj(mk, conjt)) * ldv(in + j * sstr);
+                }
+                stv(Y + c * bufsz + f, acc);
             }
             __syncthreads();
-            int cur[3] = {fin[0], fin[1], fin[2]};
-            A *a = X, *b = Y;
-            for (int ax = m.dim - 1; ax >= 0; --ax) {
-                int nxt[3] = {cur[0], cur[1], cur[2]};
-                nxt[ax] = fout[ax];
-                const int tot = nxt[0] * nxt[1] * nxt[2], ld = sp[ax], kk = cur[ax];
-                const int sstr = ax == 0 ? 1 : (ax == 1 ? cur[0] : cur[0] * cur[1]);  // input stride along ax
-                for (int e = threadIdx.x; e < qc * tot; e += blockDim.x) {
-                    const int q = e / tot, f = e - q * tot;
-                    const int i0 = f % nxt[0], i1 = (f / nxt[0]) % nxt[1], i2 = f / (nxt[0] * nxt[1]);
-                    const int row = ax == 0 ? i0 : (ax == 1 ? i1 : i2);
-                    int base = i0 + cur[0] * (i1 + cur[1] * i2);  // the input index with i[ax] = 0
-                    base -= row * sstr;
-                    const A *in = a + q * bufsz + base;
-                    A acc = sc_zero<A>();
-                    for (int j = 0; j < kk; ++j) {
-                        // up: op(M)[row, j] = M[row + j ld]; down: M^T[row, j] = M[j + row ld]
-                        const T mk = UP ? fac[ax][row + j * ld] : fac[ax][j + row * ld];
-                        acc = acc + wide(cj(mk, conjt)) * in[j * sstr];
-                    }
-                    b[q * bufsz + f] = acc;
-                }
-                __syncthreads();
-                A *t = a;
-                a = b;
-                b = t;
-                cur[0] = nxt[0];
-                cur[1] = nxt[1];
-                cur[2] = nxt[2];
-            }
-            res = a;
-            if (UP && c1 - c0 > 1) {
-                for (int e = threadIdx.x; e < qc * nout; e += blockDim.x) {
-                    const int q = e / nout, i = e - q * nout;
-                    Acc[q * bufsz + i] = (k == c0 ? sc_zero<A>() : Acc[q * bufsz + i]) + a[q * bufsz + i];
-                }
-                res = Acc;
-                __syncthreads();
-            }
+            A *t = X;
+            X = Y;
+            Y = t;
+            cur[ax] = nxt[ax];
         }
         for (int e = threadIdx.x; e < qc * nout; e += blockDim.x) {
             const int q = e / nout, i = e - q * nout;
-            T *o = dst + (int64_t)(q0 + q) * nout + i;
-            narrow(acc_dst ? wide(*o) + res[q * bufsz + i] : res[q * bufsz + i], *o);
+            A sum = k0 == c0 ? ldv(X + q * bufsz + i) : ldv(Acc + e) + ldv(X + q * bufsz + i);
+            for (int k = 1; k < nch; ++k) sum = sum + ldv(X + (k * qc + q) * bufsz + i);
+            if (k0 + cg < c1) {
+                stv(Acc + e, sum);  // read back by this thread
+            } else {
+                T v;
+                narrow(acc_dst ? wide(ldv(dst + e)) + sum : sum, v);
+                stv(dst + e, v);
+            }
         }
         __syncthreads();
     }
@@ -450,115 +423,119 @@ cudaError_t launch_transfer_sep(const DMap &m, const DSide &s, const int *nodes,
                                 bool conjt, int nrhs, void *mom, int maxsep, cudaStream_t st) {
     using A = typename ScalarTraits<T>::Acc;
     const int nq = m.ncomp * nrhs;
-    // moment columns per chunk: three buffers of maxsep accumulators each within 48 KB
-    const int qc = std::max(1, std::min(nq, (int)((48 * 1024) / (3 * (size_t)maxsep * sizeof(A)))));
-    const size_t sm = 3 * (size_t)qc * maxsep * sizeof(A);
-    transfer_sep_kernel<T, UP><<<nnodes, 256, sm, st>>>(m, s, nodes, received, conjt, nrhs, static_cast<T *>(mom),
-                                                        qc, maxsep);
+    // two buffers of every child's columns per CTA, as many columns as fit 56 KB (four CTAs an SM, and
+    // eight children's 216 complex coefficients fit), at least one; fewer children at a time, with their
+    // sum in a third buffer, where even one column of all of them exceeds an SM's shared memory
+    const size_t one = (size_t)maxsep * sizeof(A);
+    int cg = UP ? std::min(m.nsectors, SEP_CHILDREN) : 1;
+    const int qc = std::max(1, std::min(nq, (int)((56 * 1024) / (2 * cg * one))));
+    while (cg > 1 && (2 * cg + 1) * qc * one > 200 * 1024) --cg;
+    const size_t sm = (2 * cg + 1) * qc * one;
+    auto kern = &transfer_sep_kernel<T, UP>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    for (int q0 = 0; q0 < nq; q0 += 65535 * qc)
+        kern<<<dim3(nnodes, std::min(65535, (nq - q0 + qc - 1) / qc)), 256, sm, st>>>(
+            m, s, nodes, received, conjt, nrhs, static_cast<T *>(mom), q0, qc, cg, maxsep);
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------
 // A2: m_p = sum over children of op(T_{level(c), sector(c)}) m_c, first child overwriting.
+//
+// One moment column: a CTA per parent, its threads over the rows and the children dealt to its row
+// groups; a chunk of every child's moments in shared memory, sixteen transfer loads in flight per
+// thread. Bound: the loads' latency (the transfers of a level are a few hundred KB in L2). 64 parents
+// of 64 coefficients, FP64: 21 us with the moments read from global memory beside each transfer entry.
 // ---------------------------------------------------------------------------------------------
-template <class T, bool MMA>
+constexpr int UPV_THREADS = 512;
+constexpr int UPV_CHILDREN = 8, UPV_CHUNK = 128;  // children at a time, coefficients of each staged at a time
+
+template <class T>
+__global__ void __launch_bounds__(UPV_THREADS, 2)
+transfer_up_vec_kernel(DMap m, DSide s, const int *__restrict__ nodes, bool conjt, T *__restrict__ am) {
+    using A = typename ScalarTraits<T>::Acc;
+    __shared__ __align__(16) A ms[UPV_CHILDREN][UPV_CHUNK], part[UPV_THREADS];
+    const int p = nodes[blockIdx.x];
+    const int lp = s.level[p], lc = lp + 1;
+    const int nout = ncoef_of(s, lp), nin = ncoef_of(s, lc);
+    const int c0 = s.child_ptr[p], c1 = s.child_ptr[p + 1];
+    const int rows = min(UPV_THREADS, (nout + 31) / 32 * 32), groups = UPV_THREADS / rows;
+    const int g = threadIdx.x / rows, r = threadIdx.x - g * rows;
+    for (int a0 = 0; a0 < nout; a0 += rows) {
+        const int a = a0 + r;
+        const bool live = g < groups && a < nout;
+        A acc = sc_zero<A>();
+        for (int k0 = c0; k0 < c1; k0 += UPV_CHILDREN)
+            for (int b0 = 0; b0 < nin; b0 += UPV_CHUNK) {
+                const int nch = min(UPV_CHILDREN, c1 - k0), nb = min(UPV_CHUNK, nin - b0);
+                __syncthreads();
+                for (int e = threadIdx.x; e < nch * nb; e += UPV_THREADS) {
+                    const int k = e / nb, b = e - k * nb;
+                    stv(&ms[k][b], wide(ldv(am + s.mom_off[s.child[k0 + k]] + b0 + b)));
+                }
+                __syncthreads();
+                if (live)
+                    for (int k = g; k < nch; k += groups) {
+                        const int ch = s.child[k0 + k];
+                        const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]] +
+                                      (int64_t)b0 * nout + a;
+                        int b = 0;
+                        for (; b + 16 <= nb; b += 16) {
+                            T v[16];
+#pragma unroll
+                            for (int u = 0; u < 16; ++u) v[u] = ldv(Tk + (int64_t)(b + u) * nout);
+#pragma unroll
+                            for (int u = 0; u < 16; ++u) acc = acc + wide(cj(v[u], conjt)) * ldv(&ms[k][b + u]);
+                        }
+                        for (; b < nb; ++b) acc = acc + wide(cj(ldv(Tk + (int64_t)b * nout), conjt)) * ldv(&ms[k][b]);
+                    }
+            }
+        if (groups > 1) {
+            __syncthreads();
+            stv(part + threadIdx.x, acc);
+            __syncthreads();
+            if (g == 0)
+                for (int u = 1; u < groups; ++u) acc = acc + ldv(part + u * rows + r);
+        }
+        if (g == 0 && live) {
+            T v;
+            narrow(acc, v);
+            stv(am + s.mom_off[p] + a, v);
+        }
+    }
+}
+
+// Blocks of moment columns: 64 x 16 tiles on the FP64 tensor cores.
+template <class T>
 __global__ void transfer_up_kernel(DMap m, DSide s, const int *__restrict__ nodes, bool conjt,
                                    int nrhs, T *__restrict__ am) {
     using A = typename ScalarTraits<T>::Acc;
     extern __shared__ unsigned char smem_raw[];
-    A *sm = reinterpret_cast<A *>(smem_raw);
     const int p = nodes[blockIdx.x];
     const int lp = s.level[p], lc = lp + 1;
     const int nout = ncoef_of(s, lp), nin = ncoef_of(s, lc);
     T *mp = am + s.mom_off[p] * nrhs;
     const int c0 = s.child_ptr[p], c1 = s.child_ptr[p + 1];
     const int nq = m.ncomp * nrhs;
-    if (m.transfer_kind == H2B_TRANSFER_DENSE && nq == 1) {
-        // one right-hand side: children split over `ns` thread groups of `npad` threads reading
-        // their transfers directly (coalesced over the output row), partial sums reduced in smem
-        const int npad = ((nout + 31) / 32) * 32;
-        const int ns = npad <= (int)blockDim.x ? (int)blockDim.x / npad : 1;
-        const int sidx = threadIdx.x / npad;
-        for (int a0 = 0; a0 < nout; a0 += (ns > 1 ? npad : (int)blockDim.x)) {
-            const int a = a0 + (ns > 1 ? (int)threadIdx.x % npad : (int)threadIdx.x);
-            A acc = sc_zero<A>();
-            if (sidx < ns && a < nout)
-                for (int k = c0 + sidx; k < c1; k += ns) {
-                    const int ch = s.child[k];
-                    const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
-                    const T *mc = am + s.mom_off[ch] * nrhs;
-#pragma unroll 4
-                    for (int b = 0; b < nin; ++b) acc = acc + wide(cj(Tk[a + (int64_t)b * nout], conjt)) * wide(mc[b]);
-                }
-            if (ns > 1) {
-                if (sidx < ns) sm[sidx * npad + (threadIdx.x % npad)] = acc;
-                __syncthreads();
-                if (threadIdx.x < npad && a0 + threadIdx.x < nout) {
-                    A sum = sm[threadIdx.x];
-                    for (int w = 1; w < ns; ++w) sum = sum + sm[w * npad + threadIdx.x];
-                    narrow(sum, mp[a0 + threadIdx.x]);
-                }
-                __syncthreads();
-            } else if (a < nout) {
-                narrow(acc, mp[a]);
+    A *Ms = reinterpret_cast<A *>(smem_raw), *Xs = Ms + TG_M * TG_LD;
+    for (int q0 = 0; q0 < nq; q0 += TG_Q) {
+        const int nqc = min(TG_Q, nq - q0);
+        for (int m0 = 0; m0 < nout; m0 += TG_M) {
+            const int mt = min(TG_M, nout - m0);
+            MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
+            acc.zero();
+            for (int k = c0; k < c1; ++k) {
+                const int ch = s.child[k];
+                const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
+                const T *mc = am + s.mom_off[ch] * nrhs;
+                tile_gemm_mma_l(false, m0, mt, nin, nqc,
+                                [&](int i, int kk) -> A { return wide(cj(Tk[i + (int64_t)kk * nout], conjt)); },
+                                [&](int kk, int q) -> A { return wide(mc[(int64_t)(q0 + q) * nin + kk]); },
+                                Ms, Xs, acc);
             }
+            mma_store(acc, mt, nqc, [&](int i, int q, A v) { narrow(v, mp[(int64_t)(q0 + q) * nout + m0 + i]); });
         }
-        return;
-    }
-    if (m.transfer_kind == H2B_TRANSFER_DENSE) {
-        A *Ms = sm, *Xs = sm + TG_M * TG_LD;
-        for (int q0 = 0; q0 < nq; q0 += TG_Q) {
-            const int nqc = min(TG_Q, nq - q0);
-            for (int m0 = 0; m0 < nout; m0 += TG_M) {
-                const int mt = min(TG_M, nout - m0);
-                if constexpr (MMA) {
-                    MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
-                    acc.zero();
-                    for (int k = c0; k < c1; ++k) {
-                        const int ch = s.child[k];
-                        const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
-                        const T *mc = am + s.mom_off[ch] * nrhs;
-                        tile_gemm_mma_l(false, m0, mt, nin, nqc,
-                                        [&](int i, int kk) -> A { return wide(cj(Tk[i + (int64_t)kk * nout], conjt)); },
-                                        [&](int kk, int q) -> A { return wide(mc[(int64_t)(q0 + q) * nin + kk]); },
-                                        Ms, Xs, acc);
-                    }
-                    mma_store(acc, mt, nqc, [&](int i, int q, A v) { narrow(v, mp[(int64_t)(q0 + q) * nout + m0 + i]); });
-                } else {
-                    A acc[TG_O];
-                    tile_zero(acc);
-                    for (int k = c0; k < c1; ++k) {
-                        const int ch = s.child[k];
-                        const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
-                        const T *mc = am + s.mom_off[ch] * nrhs;
-                        tile_gemm(Tk, nout, false, conjt, m0, mt, nin, nqc,
-                                  [&](int kk, int q) -> A { return wide(mc[(int64_t)(q0 + q) * nin + kk]); }, Ms, Xs,
-                                  acc);
-                    }
-#pragma unroll
-                    for (int j = 0; j < TG_O; ++j) {
-                        const int o = threadIdx.x + j * blockDim.x;
-                        if (o < mt * nqc) narrow(acc[j], mp[(int64_t)(q0 + o / mt) * nout + m0 + o % mt]);
-                    }
-                }
-            }
-        }
-        return;
-    }
-    const int mx = sep_bound(s, lp);
-    A *bufa = sm, *bufb = sm + mx, *acc = sm + 2 * mx;
-    for (int q = 0; q < nq; ++q) {
-        for (int k = c0; k < c1; ++k) {
-            const int ch = s.child[k];
-            const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[ch]];
-            const T *mc = am + s.mom_off[ch] * nrhs + (int64_t)q * nin;
-            for (int e = threadIdx.x; e < nin; e += blockDim.x) bufa[e] = wide(mc[e]);
-            __syncthreads();
-            separable_block(Tk, &s.shape[3 * lp], &s.shape[3 * lc], m.dim, true, conjt, bufa, bufb,
-                            acc, k != c0);
-        }
-        for (int e = threadIdx.x; e < nout; e += blockDim.x) narrow(acc[e], mp[(int64_t)q * nout + e]);
-        __syncthreads();
     }
 }
 
@@ -1336,15 +1313,81 @@ i2o_slot_kernel(DMap m, DSide r, SibGroups g, int mode, int nrhs,
 }
 
 // ---------------------------------------------------------------------------------------------
-// C1: l_c = [l_c +] op(T_{level(c), sector(c)}) l_parent, op = transpose (adjoint for adjoint maps)
+// Sums down the columns of a stored matrix for one vector: f(j, sum over i of op(C[i + j ld]) v[i]) on
+// one lane each, for j < n, i < k, by the eight warps of a CTA. A warp takes four columns at a time,
+// lanes along the contiguous rows: one vector load serves four entries.
 // ---------------------------------------------------------------------------------------------
-template <class T, bool MMA>
+template <class A> __device__ __forceinline__ A lane_sum(A v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if constexpr (sizeof(A) == sizeof(double)) v = v + __shfl_xor_sync(0xffffffffu, v, o);
+        else v = v + A{__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)};
+    }
+    return v;
+}
+
+// `parts` matrices of n columns (n k entries apart) with vectors k entries apart are summed.
+template <class T, class F>
+__device__ __forceinline__ void column_sums(const T *__restrict__ C, const T *__restrict__ v, int k, int n, int parts,
+                                            bool conj, F f) {
+    using A = typename ScalarTraits<T>::Acc;
+    constexpr int U = 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int j0 = U * warp; j0 < n; j0 += U * 8) {
+        A acc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc[u] = sc_zero<A>();
+        for (int c = 0; c < parts; ++c) {
+            const T *Cc = C + ((int64_t)c * n + j0) * k;
+            const T *vc = v + (int64_t)c * k;
+#pragma unroll 2
+            for (int i = lane; i < k; i += 32) {
+                const A vi = wide(ldv(vc + i));
+                T e[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) e[u] = ldv(Cc + (int64_t)min(u, n - 1 - j0) * k + i);
+#pragma unroll
+                for (int u = 0; u < U; ++u) acc[u] = acc[u] + wide(cj(e[u], conj)) * vi;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const A sum = lane_sum(acc[u]);
+            if (lane == u && j0 + u < n) f(j0 + u, sum);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// C1: l_c = [l_c +] op(T_{level(c), sector(c)}) l_parent, op = transpose (adjoint for adjoint maps).
+// Stored T is nin x nout (parent x child): op(T) = T^T (or T^H), contiguous along the parent's
+// coefficients. One moment column: column sums, a CTA per child.
+// ---------------------------------------------------------------------------------------------
+template <class T>
+__global__ void __launch_bounds__(256)
+transfer_down_vec_kernel(DMap m, DSide s, const int *__restrict__ nodes, const uint8_t *__restrict__ received, bool conjt,
+                         T *dm) {
+    using A = typename ScalarTraits<T>::Acc;
+    const int c = nodes[blockIdx.x];
+    const int lc = s.level[c], lp = lc - 1;
+    const bool acc0 = received[c] != 0;
+    const T *Tk = static_cast<const T *>(s.tr) + s.tr_off[lc * m.nsectors + s.sector[c]];
+    T *mc = dm + s.mom_off[c];
+    column_sums(Tk, static_cast<const T *>(dm + s.mom_off[s.parent[c]]), ncoef_of(s, lp), ncoef_of(s, lc), 1, conjt,
+                [&](int j, A sum) {
+                    T v;
+                    narrow(acc0 ? wide(ldv(mc + j)) + sum : sum, v);
+                    stv(mc + j, v);
+                });
+}
+
+// Blocks of moment columns: 64 x 16 tiles on the FP64 tensor cores.
+template <class T>
 __global__ void transfer_down_kernel(DMap m, DSide s, const int *__restrict__ nodes,
                                      const uint8_t *__restrict__ received, bool conjt, int nrhs,
                                      T *__restrict__ dm) {
     using A = typename ScalarTraits<T>::Acc;
     extern __shared__ unsigned char smem_raw[];
-    A *sm = reinterpret_cast<A *>(smem_raw);
     const int c = nodes[blockIdx.x];
     const int lc = s.level[c], lp = lc - 1;
     const int par = s.parent[c];
@@ -1354,55 +1397,45 @@ __global__ void transfer_down_kernel(DMap m, DSide s, const int *__restrict__ no
     T *mc = dm + s.mom_off[c] * nrhs;
     const T *mp = dm + s.mom_off[par] * nrhs;
     const int nq = m.ncomp * nrhs;
-    if (m.transfer_kind == H2B_TRANSFER_DENSE) {
-        // stored T is nin x nout (parent x child): op(T) = T^T (or T^H), column-contiguous in k
-        A *Ms = sm, *Xs = sm + TG_M * TG_LD;
-        for (int q0 = 0; q0 < nq; q0 += TG_Q) {
-            const int nqc = min(TG_Q, nq - q0);
-            for (int m0 = 0; m0 < nout; m0 += TG_M) {
-                const int mt = min(TG_M, nout - m0);
-                if constexpr (!MMA) {  // one right-hand side: FMA tile (an MMA would idle 7 of 8 columns)
-                    A acc[TG_O];
-                    tile_zero(acc);
-                    tile_gemm(Tk, nin, true, conjt, m0, mt, nin, nqc,
-                              [&](int kk, int q) -> A { return wide(mp[(int64_t)(q0 + q) * nin + kk]); }, Ms, Xs, acc);
-#pragma unroll
-                    for (int j = 0; j < TG_O; ++j) {
-                        const int o = threadIdx.x + j * blockDim.x;
-                        if (o < mt * nqc) {
-                            T *dst = &mc[(int64_t)(q0 + o / mt) * nout + m0 + o % mt];
-                            narrow(acc0 ? wide(*dst) + acc[j] : acc[j], *dst);
-                        }
-                    }
-                } else {
-                MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
-                acc.zero();
-                tile_gemm_mma_l(true, m0, mt, nin, nqc,
-                                [&](int i, int kk) -> A { return wide(cj(Tk[kk + (int64_t)i * nin], conjt)); },
-                                [&](int kk, int q) -> A { return wide(mp[(int64_t)(q0 + q) * nin + kk]); }, Ms, Xs, acc);
-                mma_store(acc, mt, nqc, [&](int i, int q, A v) {
-                    T *dst = &mc[(int64_t)(q0 + q) * nout + m0 + i];
-                    narrow(acc0 ? wide(*dst) + v : v, *dst);
-                });
-                }
-            }
+    A *Ms = reinterpret_cast<A *>(smem_raw), *Xs = Ms + TG_M * TG_LD;
+    for (int q0 = 0; q0 < nq; q0 += TG_Q) {
+        const int nqc = min(TG_Q, nq - q0);
+        for (int m0 = 0; m0 < nout; m0 += TG_M) {
+            const int mt = min(TG_M, nout - m0);
+            MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
+            acc.zero();
+            tile_gemm_mma_l(true, m0, mt, nin, nqc,
+                            [&](int i, int kk) -> A { return wide(cj(Tk[kk + (int64_t)i * nin], conjt)); },
+                            [&](int kk, int q) -> A { return wide(mp[(int64_t)(q0 + q) * nin + kk]); }, Ms, Xs, acc);
+            mma_store(acc, mt, nqc, [&](int i, int q, A v) {
+                T *dst = &mc[(int64_t)(q0 + q) * nout + m0 + i];
+                narrow(acc0 ? wide(*dst) + v : v, *dst);
+            });
         }
-        return;
-    }
-    const int mx = sep_bound(s, lp);
-    A *bufa = sm, *bufb = sm + mx;
-    for (int q = 0; q < nq; ++q) {
-        for (int e = threadIdx.x; e < nin; e += blockDim.x) bufa[e] = wide(mp[(int64_t)q * nin + e]);
-        __syncthreads();
-        separable_block(Tk, &s.shape[3 * lp], &s.shape[3 * lc], m.dim, false, conjt, bufa, bufb,
-                        mc + (int64_t)q * nout, acc0);
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // C2: y[values] = alpha * sum_c op(C_c)^T l_c + beta * y[values]  (beta == 0 overwrites)
+//
+// One right-hand side: column sums, a CTA per leaf. Bound: HBM (each collection entry is used once).
 // ---------------------------------------------------------------------------------------------
-template <class T, class V, bool MMA>
+template <class T, class V>
+__global__ void __launch_bounds__(256)
+leaf_disaggregate_vec_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, const T *__restrict__ dm,
+                             V alpha, V beta, bool beta_zero, V *__restrict__ y) {
+    const int leaf = leaves[blockIdx.x];
+    const int v0 = s.value_ptr[leaf], nv = s.value_ptr[leaf + 1] - v0;
+    column_sums(static_cast<const T *>(s.coll) + s.coll_off[leaf], dm + s.mom_off[leaf], ncoef_of(s, s.level[leaf]), nv,
+                m.ncomp, conjc, [&](int j, V sum) {
+                    V *dst = &y[s.value[v0 + j]];
+                    const V v = alpha * sum;
+                    *dst = beta_zero ? v : v + beta * *dst;
+                });
+}
+
+// Blocks of right-hand sides: 64 x 16 tiles on the FP64 tensor cores.
+template <class T, class V>
 __global__ void __launch_bounds__(256)
 leaf_disaggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, int nrhs,
                          const T *__restrict__ dm, V alpha, V beta, bool beta_zero, V *__restrict__ y,
@@ -1419,23 +1452,6 @@ leaf_disaggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool c
         const int nq = min(TG_Q, nrhs - q0);
         for (int m0 = 0; m0 < nv; m0 += TG_M) {
             const int mt = min(TG_M, nv - m0);
-            if constexpr (!MMA) {  // one right-hand side: FMA tile
-                A acc[TG_O];
-                tile_zero(acc);
-                for (int c = 0; c < m.ncomp; ++c)
-                    tile_gemm(C + (int64_t)c * nc * nv, nc, true, conjc, m0, mt, nc, nq,
-                              [&](int k, int q) -> A { return wide(mom[((int64_t)c * nrhs + q0 + q) * nc + k]); },
-                              Ms, Xs, acc);
-#pragma unroll
-                for (int j = 0; j < TG_O; ++j) {
-                    const int o = threadIdx.x + j * blockDim.x;
-                    if (o < mt * nq) {
-                        V *dst = &y[(int64_t)(q0 + o / mt) * ldy + s.value[v0 + m0 + o % mt]];
-                        const V v = alpha * acc[j];
-                        *dst = beta_zero ? v : v + beta * *dst;
-                    }
-                }
-            } else {
             MmaAcc<A> acc;  // FP64 tensor cores (256 threads: 8 warps x 8 rows)
             acc.zero();
             for (int c = 0; c < m.ncomp; ++c) {
@@ -1450,7 +1466,6 @@ leaf_disaggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool c
                 const V w = alpha * v;
                 *dst = beta_zero ? w : w + beta * *dst;
             });
-            }
         }
     }
 }
@@ -1510,7 +1525,12 @@ cudaError_t launch_leaf_aggregate(bool cplx, int precision, const DMap &m, const
                     m, s, leaves, nleaves, fa.nrhs, static_cast<const double *>(x), ldx, static_cast<T *>(fa.am));
                 break;
             }
-            auto kern = fa.nrhs > 1 ? &leaf_aggregate_kernel<T, double, true> : &leaf_aggregate_kernel<T, double, false>;
+            if (fa.nrhs == 1) {
+                leaf_aggregate_vec_kernel<T, double><<<nleaves, 256, 0, st>>>(m, s, leaves, conjc, static_cast<const double *>(x),
+                                                                              static_cast<T *>(fa.am));
+                break;
+            }
+            auto kern = &leaf_aggregate_kernel<T, double>;
             err = allow_smem(kern, tile_smem<double>());
             if (err == cudaSuccess)
                 kern<<<nleaves, 256, tile_smem<double>(), st>>>(
@@ -1518,7 +1538,13 @@ cudaError_t launch_leaf_aggregate(bool cplx, int precision, const DMap &m, const
         });
     } else {
         H2B_DISPATCH_CPLX(precision, {
-            auto kern = fa.nrhs > 1 ? &leaf_aggregate_kernel<T, cdouble, true> : &leaf_aggregate_kernel<T, cdouble, false>;
+            if (fa.nrhs == 1) {
+                leaf_aggregate_vec_kernel<T, cdouble><<<nleaves, 256, 0, st>>>(m, s, leaves, conjc,
+                                                                               static_cast<const cdouble *>(x),
+                                                                               static_cast<T *>(fa.am));
+                break;
+            }
+            auto kern = &leaf_aggregate_kernel<T, cdouble>;
             err = allow_smem(kern, tile_smem<cdouble>());
             if (err == cudaSuccess)
                 kern<<<nleaves, 256, tile_smem<cdouble>(), st>>>(
@@ -1539,7 +1565,6 @@ cudaError_t launch_transfer_up(bool cplx, int precision, const DMap &m, const DS
                                               : warp_transfer_up<float>(m, s, nodes, nnodes, fa.nrhs, fa.am, st);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    const int bs = m.transfer_kind == H2B_TRANSFER_DENSE ? 256 : block_for(maxcoef);
     cudaError_t err = cudaSuccess;
     if (m.transfer_kind == H2B_TRANSFER_SEPARABLE) {
         H2B_DISPATCH_T(cplx, precision, {
@@ -1549,13 +1574,16 @@ cudaError_t launch_transfer_up(bool cplx, int precision, const DMap &m, const DS
     }
     H2B_DISPATCH_T(cplx, precision, {
         using A = typename ScalarTraits<T>::Acc;
-        const size_t sm = m.transfer_kind == H2B_TRANSFER_DENSE ? tile_smem<A>()
-                                                                 : 3 * (size_t)maxsep * sizeof(A);
+        const size_t sm = tile_smem<A>();
         const int nq = m.ncomp * fa.nrhs;
-        auto kern = nq > 1 ? &transfer_up_kernel<T, true> : &transfer_up_kernel<T, false>;
+        if (nq == 1) {
+            transfer_up_vec_kernel<T><<<nnodes, UPV_THREADS, 0, st>>>(m, s, nodes, conjt, static_cast<T *>(fa.am));
+            break;
+        }
+        auto kern = &transfer_up_kernel<T>;
         err = allow_smem(kern, sm);
         if (err == cudaSuccess)
-            kern<<<nnodes, bs, sm, st>>>(m, s, nodes, conjt, fa.nrhs, static_cast<T *>(fa.am));
+            kern<<<nnodes, 256, sm, st>>>(m, s, nodes, conjt, fa.nrhs, static_cast<T *>(fa.am));
     });
     return err != cudaSuccess ? err : cudaGetLastError();
 }
@@ -1732,7 +1760,6 @@ cudaError_t launch_transfer_down(bool cplx, int precision, const DMap &m, const 
         else warp_transfer_down<float>(m, s, nodes, nnodes, received, fa.nrhs, fa.dm, st);
         return cudaGetLastError();
     }
-    const int bs = m.transfer_kind == H2B_TRANSFER_DENSE ? 256 : block_for(maxcoef, 64, 256);
     const bool conjt = fa.mode == H2B_ADJOINT;
     cudaError_t err = cudaSuccess;
     if (m.transfer_kind == H2B_TRANSFER_SEPARABLE) {
@@ -1743,13 +1770,16 @@ cudaError_t launch_transfer_down(bool cplx, int precision, const DMap &m, const 
     }
     H2B_DISPATCH_T(cplx, precision, {
         using A = typename ScalarTraits<T>::Acc;
-        const size_t sm = m.transfer_kind == H2B_TRANSFER_DENSE ? tile_smem<A>()
-                                                                 : 2 * (size_t)maxsep * sizeof(A);
+        const size_t sm = tile_smem<A>();
         const int nq = m.ncomp * fa.nrhs;
-        auto kern = nq > 1 ? &transfer_down_kernel<T, true> : &transfer_down_kernel<T, false>;
+        if (nq == 1) {
+            transfer_down_vec_kernel<T><<<nnodes, 256, 0, st>>>(m, s, nodes, received, conjt, static_cast<T *>(fa.dm));
+            break;
+        }
+        auto kern = &transfer_down_kernel<T>;
         err = allow_smem(kern, sm);
         if (err == cudaSuccess)
-            kern<<<nnodes, bs, sm, st>>>(m, s, nodes, received, conjt, fa.nrhs,
+            kern<<<nnodes, 256, sm, st>>>(m, s, nodes, received, conjt, fa.nrhs,
                                                            static_cast<T *>(fa.dm));
     });
     return err != cudaSuccess ? err : cudaGetLastError();
@@ -1771,7 +1801,12 @@ cudaError_t launch_leaf_disaggregate(bool cplx, int precision, const DMap &m, co
                     static_cast<double *>(y), ldy);
                 break;
             }
-            auto kern = fa.nrhs > 1 ? &leaf_disaggregate_kernel<T, double, true> : &leaf_disaggregate_kernel<T, double, false>;
+            if (fa.nrhs == 1) {
+                leaf_disaggregate_vec_kernel<T, double><<<nleaves, 256, 0, st>>>(
+                    m, s, leaves, conjc, static_cast<const T *>(fa.dm), alpha.x, beta.x, bz, static_cast<double *>(y));
+                break;
+            }
+            auto kern = &leaf_disaggregate_kernel<T, double>;
             err = allow_smem(kern, tile_smem<double>());
             if (err == cudaSuccess)
                 kern<<<nleaves, bs, tile_smem<double>(), st>>>(
@@ -1781,7 +1816,12 @@ cudaError_t launch_leaf_disaggregate(bool cplx, int precision, const DMap &m, co
     } else {
         const bool bz = beta.x == 0.0 && beta.y == 0.0;
         H2B_DISPATCH_CPLX(precision, {
-            auto kern = fa.nrhs > 1 ? &leaf_disaggregate_kernel<T, cdouble, true> : &leaf_disaggregate_kernel<T, cdouble, false>;
+            if (fa.nrhs == 1) {
+                leaf_disaggregate_vec_kernel<T, cdouble><<<nleaves, 256, 0, st>>>(
+                    m, s, leaves, conjc, static_cast<const T *>(fa.dm), alpha, beta, bz, static_cast<cdouble *>(y));
+                break;
+            }
+            auto kern = &leaf_disaggregate_kernel<T, cdouble>;
             err = allow_smem(kern, tile_smem<cdouble>());
             if (err == cudaSuccess)
                 kern<<<nleaves, bs, tile_smem<cdouble>(), st>>>(
