@@ -289,8 +289,11 @@ i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTrai
 // its pairs' columns, read through each pair's row permutation. Loads of eight pairs are in flight
 // per thread; the sum runs in list order. (Columns copied to shared memory as they lie and permuted on
 // the reads from there were slower everywhere, 65,536-point sphere, 32 right-hand sides: 2.4 -> 5 ms.)
+// Bound: the loads in flight, so the registers leave room for ten blocks an SM of complex maps (48
+// each; 56 before: FP32 sphere, I2O of 32 right-hand sides 12.65 -> 12.30 ms, of 8 3.78 -> 3.72), twelve
+// of real ones (40, what the compiler took by itself).
 template <class T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, ScalarTraits<T>::is_complex ? 10 : 12)
 i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, int nrhs, int q0, int qn, int pbase,
                      int pstride, const typename ScalarTraits<T>::Acc *__restrict__ prod, T *__restrict__ dm) {
     using A = typename ScalarTraits<T>::Acc;
