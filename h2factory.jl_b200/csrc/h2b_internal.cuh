@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
 #include <vector>
 
 #include "../../include/h2b200.h"
@@ -91,6 +92,32 @@ template <> __device__ __forceinline__ cfloat ldv(const cfloat *p) {
 template <class T> __device__ __forceinline__ void stv(T *p, T v) { *p = v; }
 template <> __device__ __forceinline__ void stv(cdouble *p, cdouble v) { *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y); }
 template <> __device__ __forceinline__ void stv(cfloat *p, cfloat v) { *reinterpret_cast<float2 *>(p) = make_float2(v.x, v.y); }
+
+// ---------------------------------------------------------------------------------------------
+// The far passes of one column are a chain of short launches, each reading what the one before wrote.
+// A kernel that calls chain_wait() before its first access to moments or pair products (reads and
+// writes alike) may be launched ahead: its blocks then start, and read the map's own arrays, while the
+// last blocks of the kernel before it in the stream still run. chain_wait() returns when that kernel
+// has completed, and lets the next one start in turn; the pointers that it guards carry no
+// __restrict__, so no load of theirs is an invariant one that could move above it. At least one
+// thread of a launch must reach it. (After any other stream operation the launch is an ordinary one.)
+//
+// Which launches go ahead: those of one column, of dense and diagonal couplings, of up to 16 blocks
+// an SM. Blocks that wait hold their places on the SMs, where the near field's kernels run meanwhile.
+// Per product, us, ordinary -> ahead: Laplace maps of 2,048 points 41 -> 38, of 8,192 points 98 -> 88,
+// Helmholtz ellipsoid of 20,011 points 420 -> 409, sphere of 65,536 points 1288 -> 1267 (1290 without
+// the limit on blocks). Slower, so left out: Toeplitz maps (262,144 points, 1027 -> 1080) and several
+// columns (12,289 points, three right-hand sides, 449 -> 456; 7,189 points, fourteen, 254 -> 266).
+// ---------------------------------------------------------------------------------------------
+constexpr int CHAIN_BLOCKS = 16 * 148;
+
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// The first kernel of a chain, launched the ordinary way, only lets the next one start.
+__device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------
 // Device-resident side of a core (all pointers device memory).
@@ -206,6 +233,24 @@ struct PairTiles {
     int64_t unit_elems = 0;
     int pstride = 1;              // scalars per pair and right-hand side
 };
+
+inline bool chain_ahead(const DMap &m, int nq) { return nq == 1 && m.coupling_kind != H2B_COUPLING_TOEPLITZ; }
+
+template <class... P, class... A>
+cudaError_t launch_chain(bool ahead, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                         A &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ahead && (int64_t)grid.x * grid.y * grid.z <= CHAIN_BLOCKS ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // Per-call arguments of the far passes.
 struct FarArgs {

@@ -246,6 +246,7 @@ template <class T, class V>
 __global__ void __launch_bounds__(256)
 leaf_aggregate_vec_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, const V *__restrict__ x,
                           T *__restrict__ am) {
+    chain_open();
     using A = typename ScalarTraits<T>::Acc;  // == V
     __shared__ __align__(16) A xs[LEAF_XS], part[256];
     const int leaf = leaves[blockIdx.x];
@@ -292,6 +293,7 @@ template <class T, class V>
 __global__ void __launch_bounds__(256)
 leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, int nrhs,
                       const V *__restrict__ x, int64_t ldx, T *__restrict__ am) {
+    chain_open();
     using A = typename ScalarTraits<T>::Acc;  // == V
     extern __shared__ unsigned char smem_raw[];
     A *Ms = reinterpret_cast<A *>(smem_raw), *Xs = Ms + TG_M * TG_LD;
@@ -337,7 +339,8 @@ constexpr int SEP_CHILDREN = 64;  // children contracted side by side at most
 template <class T, bool UP>
 __global__ void __launch_bounds__(256)
 transfer_sep_kernel(DMap m, DSide s, const int *__restrict__ nodes, const uint8_t *__restrict__ received,
-                    bool conjt, int nrhs, T *__restrict__ mom, int qbase, int qc_max, int cg, int bufsz) {
+                    bool conjt, int nrhs, T *mom, int qbase, int qc_max, int cg, int bufsz) {
+    chain_wait();
     using A = typename ScalarTraits<T>::Acc;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int node = nodes[blockIdx.x];
@@ -434,10 +437,10 @@ cudaError_t launch_transfer_sep(const DMap &m, const DSide &s, const int *nodes,
     auto kern = &transfer_sep_kernel<T, UP>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    for (int q0 = 0; q0 < nq; q0 += 65535 * qc)
-        kern<<<dim3(nnodes, std::min(65535, (nq - q0 + qc - 1) / qc)), 256, sm, st>>>(
-            m, s, nodes, received, conjt, nrhs, static_cast<T *>(mom), q0, qc, cg, maxsep);
-    return cudaGetLastError();
+    for (int q0 = 0; q0 < nq && e == cudaSuccess; q0 += 65535 * qc)
+        e = launch_chain(chain_ahead(m, nq), kern, dim3(nnodes, std::min(65535, (nq - q0 + qc - 1) / qc)), 256, sm, st, m, s, nodes,
+                         received, conjt, nrhs, static_cast<T *>(mom), q0, qc, cg, maxsep);
+    return e;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -453,7 +456,8 @@ constexpr int UPV_CHILDREN = 8, UPV_CHUNK = 128;  // children at a time, coeffic
 
 template <class T>
 __global__ void __launch_bounds__(UPV_THREADS, 2)
-transfer_up_vec_kernel(DMap m, DSide s, const int *__restrict__ nodes, bool conjt, T *__restrict__ am) {
+transfer_up_vec_kernel(DMap m, DSide s, const int *__restrict__ nodes, bool conjt, T *am) {
+    chain_wait();
     using A = typename ScalarTraits<T>::Acc;
     __shared__ __align__(16) A ms[UPV_CHILDREN][UPV_CHUNK], part[UPV_THREADS];
     const int p = nodes[blockIdx.x];
@@ -1367,6 +1371,7 @@ template <class T>
 __global__ void __launch_bounds__(256)
 transfer_down_vec_kernel(DMap m, DSide s, const int *__restrict__ nodes, const uint8_t *__restrict__ received, bool conjt,
                          T *dm) {
+    chain_wait();
     using A = typename ScalarTraits<T>::Acc;
     const int c = nodes[blockIdx.x];
     const int lc = s.level[c], lp = lc - 1;
@@ -1577,7 +1582,8 @@ cudaError_t launch_transfer_up(bool cplx, int precision, const DMap &m, const DS
         const size_t sm = tile_smem<A>();
         const int nq = m.ncomp * fa.nrhs;
         if (nq == 1) {
-            transfer_up_vec_kernel<T><<<nnodes, UPV_THREADS, 0, st>>>(m, s, nodes, conjt, static_cast<T *>(fa.am));
+            err = launch_chain(chain_ahead(m, nq), transfer_up_vec_kernel<T>, nnodes, UPV_THREADS, 0, st, m, s, nodes, conjt,
+                               static_cast<T *>(fa.am));
             break;
         }
         auto kern = &transfer_up_kernel<T>;
@@ -1773,7 +1779,8 @@ cudaError_t launch_transfer_down(bool cplx, int precision, const DMap &m, const 
         const size_t sm = tile_smem<A>();
         const int nq = m.ncomp * fa.nrhs;
         if (nq == 1) {
-            transfer_down_vec_kernel<T><<<nnodes, 256, 0, st>>>(m, s, nodes, received, conjt, static_cast<T *>(fa.dm));
+            err = launch_chain(chain_ahead(m, nq), transfer_down_vec_kernel<T>, nnodes, 256, 0, st, m, s, nodes, received, conjt,
+                               static_cast<T *>(fa.dm));
             break;
         }
         auto kern = &transfer_down_kernel<T>;

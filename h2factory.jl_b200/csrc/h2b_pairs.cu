@@ -240,7 +240,7 @@ __device__ __forceinline__ void pk_tile(const DMap &m, const PkArgs &g, const T 
 // at prod[((p - pbase) qn + q) pstride].
 template <class T, bool FWD>
 __global__ void __launch_bounds__(PK_THREADS, PkGeom<T>::CTAS)
-i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTraits<T>::Acc *__restrict__ prod) {
+i2o_pairs_kernel(DMap m, PkArgs g, const T *am, typename ScalarTraits<T>::Acc *prod) {
     extern __shared__ __align__(16) unsigned char pk_smem[];
     __shared__ int64_t col_src[PK_N], col_out[PK_N];  // per column: its moments and its product
     __shared__ int col_perm[PK_N];                    // the permutation its moments are read through, -1: none
@@ -263,6 +263,7 @@ i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTrai
         // block's columns (x read through colperm), transposed ones over its rows (rowperm)
         col_perm[c] = rc.z < 0 ? -1 : rc.z + (FWD ? 2 * kk : 0);
     }
+    chain_wait();
     __syncthreads();
     // 8 x 8 blocks per warp: wide tiles one column block per warp with all row blocks, or, for real
     // tiles of 64 rows, two column blocks with half the row blocks (six loads for eight products
@@ -295,7 +296,7 @@ i2o_pairs_kernel(DMap m, PkArgs g, const T *__restrict__ am, typename ScalarTrai
 template <class T>
 __global__ void __launch_bounds__(128, ScalarTraits<T>::is_complex ? 10 : 12)
 i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, int nrhs, int q0, int qn, int pbase,
-                     int pstride, const typename ScalarTraits<T>::Acc *__restrict__ prod, T *__restrict__ dm) {
+                     int pstride, const typename ScalarTraits<T>::Acc *prod, T *dm) {
     using A = typename ScalarTraits<T>::Acc;
     constexpr int U = 8;
     const int node = nodes[blockIdx.x];
@@ -307,6 +308,7 @@ i2o_pairs_sum_kernel(DMap m, DSide r, const int *__restrict__ nodes, bool fwd, i
     // forward: out[i] += Y[rowperm^-1[i]]; transposed: out[j] += Y[colperm^-1[j]]
     const int set = fwd ? nc : 3 * nc;
     A sum = sc_zero<A>();
+    chain_wait();
     for (int p = p0; p < p1; p += U) {
         A v[U];
 #pragma unroll
@@ -330,9 +332,8 @@ cudaError_t launch_sum_t(const DMap &m, const DSide &r, const PairTiles &pt, con
                          int q0, int qn, cudaStream_t st) {
     using A = typename ScalarTraits<T>::Acc;
     const dim3 grid(u.nrcv, (unsigned)(((int64_t)maxcoef * qn + 127) / 128));
-    i2o_pairs_sum_kernel<T><<<grid, 128, 0, st>>>(m, r, pt.rcv + u.rcv0, fa.mode == H2B_FORWARD, fa.nrhs, q0, qn, u.p0,
-                                                  pt.pstride, static_cast<const A *>(fa.prod), static_cast<T *>(fa.dm));
-    return cudaGetLastError();
+    return launch_chain(chain_ahead(m, m.ncomp * fa.nrhs), i2o_pairs_sum_kernel<T>, grid, 128, 0, st, m, r, pt.rcv + u.rcv0, fa.mode == H2B_FORWARD, fa.nrhs, q0,
+                        qn, u.p0, pt.pstride, static_cast<const A *>(fa.prod), static_cast<T *>(fa.dm));
 }
 
 template <class T>
@@ -356,7 +357,8 @@ cudaError_t launch_pairs_t(const DMap &m, const DSide &r, const PairTiles &pt, c
             const int qn = std::min(qc, nq - q0);
             const dim3 grid(u.ntiles, mtiles, (u.maxpairs * qn + PK_N - 1) / PK_N);
             const PkArgs g{pt.rec, pt.tile, pt.tile_off, u.tile0, fa.nrhs, q0, qn, u.p0, pt.pstride, adj};
-            kern<<<grid, PK_THREADS, sm, st>>>(m, g, static_cast<const T *>(fa.am), prod);
+            err = launch_chain(chain_ahead(m, nq), kern, grid, PK_THREADS, sm, st, m, g, static_cast<const T *>(fa.am), prod);
+            if (err != cudaSuccess) return err;
             err = launch_sum_t<T>(m, r, pt, u, fa, maxcoef, q0, qn, st);
             if (err != cudaSuccess) return err;
         }
