@@ -488,9 +488,15 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
 // with: plans whose units take at most these shares of it per right-hand side, so that a wide block
 // runs all its right-hand sides in one pass over smaller units. The last one is also what
 // h2b_farmul_noalloc's buffer holds.
-constexpr int64_t PAIR_BUFFER_BYTES = 256ll << 20;
-constexpr int PAIR_PLANS[] = {1, 4, 16, 64};
-constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 64;
+//
+// Why 512 MiB: every unit ends in a wave of tiles that leaves SMs idle, and the fewer receivers a unit
+// has, the fewer pairs of it share a block. I2O per product at 64, 128, 256, 512 and 1024 MiB, ms:
+// 65,536-point sphere, FP32, 8 right-hand sides 5.3, 4.3, 3.7, 3.2, 3.1, and 32 16.4, 13.5, 12.2, 11.3, 11.4;
+// 262,144 points, FP64, 32 right-hand sides 154, 122, 112, 104, 103. Five plans: a core of 30,011
+// points takes 73 ms to make with them, 70 with four, 86 with eight.
+constexpr int64_t PAIR_BUFFER_BYTES = 512ll << 20;
+constexpr int PAIR_PLANS[] = {1, 8, 16, 32, 128};
+constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 128;
 
 // Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of one side, a
 // plan for each share of PAIR_PLANS that cuts them differently. A plan is left out when one receiving
@@ -537,8 +543,27 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         const Key &x = keys[a], &y = keys[b];
         return std::tie(x.off, x.nc, x.snc, x.perm, a) < std::tie(y.off, y.nc, y.snc, y.perm, b);
     });
-    for (size_t i = 0; i < keys.size(); ++i) rank[order[i]] = (int)i;
+    {
+        std::vector<Key> sorted(keys.size());
+        for (size_t i = 0; i < keys.size(); ++i) {
+            rank[order[i]] = (int)i;
+            sorted[i] = keys[order[i]];
+        }
+        keys.swap(sorted);
+    }
     for (int p = 0; p < np; ++p) key[p] = rank[key[p]];
+    // runs of keys: of one block, and of one block and permutation
+    std::vector<int> block_run(keys.size()), perm_run(keys.size());
+    for (size_t i = 1; i < keys.size(); ++i) {
+        const bool same = same_block(keys[i], keys[i - 1]);
+        block_run[i] = block_run[i - 1] + !same;
+        perm_run[i] = perm_run[i - 1] + !(same && keys[i].perm == keys[i - 1].perm);
+    }
+    // the pairs by key, in list order within a key: a plan deals them out to its units
+    std::vector<int> by_key(np), key_at(keys.size() + 1);
+    for (int p = 0; p < np; ++p) ++key_at[key[p] + 1];
+    for (size_t k = 0; k < keys.size(); ++k) key_at[k + 1] += key_at[k];
+    for (int p = 0; p < np; ++p) by_key[key_at[key[p]]++] = p;
 
     // the FP32 form's tensor-core tiles: blocks of one shape (one tensor map names the columns of all of
     // them, another those of the moments) whose chunks of 32 FP32 values of K pair up into accumulation
@@ -562,12 +587,12 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         base.blocks32 = test_side ? c->dmap.cpl : c->dmap.cpl_t;
         base.cols32 = d.coupling_len / W / base.nc32;
         base.stored32 = true;
-        for (size_t i = 0; i < keys.size(); ++i) off32[i] = keys[order[i]].off;
+        for (size_t i = 0; i < keys.size(); ++i) off32[i] = keys[i].off;
     } else if (tensor) {
         std::vector<float> blocks;
         for (size_t i = 0; i < keys.size(); ++i) {
-            const Key &k = keys[order[i]];
-            if (i > 0 && same_block(k, keys[order[i - 1]])) {
+            const Key &k = keys[i];
+            if (i > 0 && block_run[i] == block_run[i - 1]) {
                 off32[i] = off32[i - 1];
                 continue;
             }
@@ -604,56 +629,57 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         const int64_t max_pairs = PAIR_BUFFER_BYTES / share / (8 * W * (int64_t)pstride);
         if (!plans.empty() && plans.back().units.size() == 1 && np <= max_pairs) continue;  // the same plan again
         PairTiles out = base;
-        std::vector<int> pair(np), count;
-        std::vector<int4> tile, tile32;
-        std::vector<int64_t> tile_off, tile32_off;
-        int64_t most = 0;
-        bool fits = true;
+        // units: as many receiving nodes as their pairs fit
+        std::vector<int> first{0}, at, unit(np), pair(np);  // units' first receiving nodes and pairs; pairs by unit and key
         for (size_t i = 0; i < recv.size();) {
-            const size_t i0 = i;
             const int p0 = s.i2o_ptr[recv[i]];
             while (i < recv.size() && s.i2o_ptr[recv[i] + 1] - p0 <= max_pairs) ++i;
-            if (!(fits = i > i0)) break;
-            const int p1 = s.i2o_ptr[recv[i - 1] + 1];
+            if ((int)i == first.back()) break;
+            std::fill(unit.begin() + p0, unit.begin() + s.i2o_ptr[recv[i - 1] + 1], (int)at.size());
+            at.push_back(p0);
+            first.push_back((int)i);
+        }
+        if (first.back() < (int)recv.size()) break;  // nor will smaller units hold that receiving node
+        for (int p : by_key) pair[at[unit[p]]++] = p;  // at: now the units' ends
+        std::vector<int4> tile, tile32;
+        std::vector<int64_t> tile_off, tile32_off;
+        std::vector<std::pair<int4, int>> cuts, tiles;
+        int64_t most = 0;
+        for (size_t n = 0; n < at.size(); ++n) {
+            const int p0 = s.i2o_ptr[recv[first[n]]], p1 = at[n];
             most = std::max<int64_t>(most, p1 - p0);
-            // the unit's pairs by key, in list order within a key
-            if ((size_t)(p1 - p0) >= keys.size() / 8) {
-                count.assign(keys.size() + 1, 0);
-                for (int p = p0; p < p1; ++p) ++count[key[p] + 1];
-                for (size_t k = 0; k < keys.size(); ++k) count[k + 1] += count[k];
-                for (int p = p0; p < p1; ++p) pair[p0 + count[key[p]]++] = p;
-            } else {
-                for (int p = p0; p < p1; ++p) pair[p] = p;
-                std::sort(pair.begin() + p0, pair.begin() + p1,
-                          [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
-            }
-            PairUnit u{(int)tile.size(), 0, 0, (int)tile32.size(), {}, (int)i0, (int)(i - i0), p0};
-            // runs of pairs for which same(other, first) holds, each cut into whole tiles and a rest (tiles of
-            // equal pairs kept more column blocks busy: 514 pairs are 8.25 tiles' work that way, 9 the other),
-            // the tiles with more pairs first: {tile, its first pair's key}
-            std::vector<std::pair<int4, int>> cuts;
-            auto cut = [&](auto same) {
-                cuts.clear();
+            PairUnit u{(int)tile.size(), 0, 0, (int)tile32.size(), {}, first[n], first[n + 1] - first[n], p0};
+            // the pairs of each run of keys, cut into whole tiles and a rest (tiles of equal pairs kept more
+            // column blocks busy: 514 pairs are 8.25 tiles' work that way, 9 the other), the tiles with more
+            // pairs first: {tile, its first pair's key}
+            auto cut = [&](const std::vector<int> &run) {
+                int count[PAIR_TILE + 1] = {};
+                tiles.clear();
                 for (int a = p0; a < p1;) {
                     const int ka = key[pair[a]];
-                    const Key &k = keys[order[ka]];
                     int b = a + 1;
-                    while (b < p1 && (key[pair[b]] == ka || same(keys[order[key[pair[b]]]], k))) ++b;
-                    for (; a < b; a += PAIR_TILE) cuts.emplace_back(make_int4(a, std::min(PAIR_TILE, b - a), k.nc, k.snc), ka);
+                    while (b < p1 && run[key[pair[b]]] == run[ka]) ++b;
+                    for (; a < b; a += PAIR_TILE) {
+                        const int n = std::min(PAIR_TILE, b - a);
+                        tiles.emplace_back(make_int4(a, n, keys[ka].nc, keys[ka].snc), ka);
+                        ++count[n];
+                    }
                     a = b;
                 }
-                std::stable_sort(cuts.begin(), cuts.end(),
-                                 [](const auto &x, const auto &y) { return x.first.y > y.first.y; });
+                int start = 0;
+                for (int n = PAIR_TILE; n > 0; --n) start += std::exchange(count[n], start);
+                cuts.resize(tiles.size());
+                for (const auto &t : tiles) cuts[count[t.first.y]++] = t;
             };
-            cut(same_block);
+            cut(block_run);
             for (const auto &t : cuts) {
                 tile.push_back(t.first);
-                tile_off.push_back(keys[order[t.second]].off);
+                tile_off.push_back(keys[t.second].off);
             }
             u.ntiles = (int)cuts.size();
             u.maxpairs = cuts[0].first.y;
             if (tensor) {
-                cut([&](const Key &x, const Key &y) { return same_block(x, y) && x.perm == y.perm; });
+                cut(perm_run);
                 for (const auto &t : cuts) {
                     tile32.push_back(t.first);
                     tile32_off.push_back(off32[t.second]);
@@ -662,11 +688,10 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
             }
             out.units.push_back(u);
         }
-        if (!fits) break;  // nor will smaller units hold that receiving node
         std::vector<int4> rec(np);
         for (int i = 0; i < np; ++i) {
             const int p = pair[i];
-            const int64_t src = other_mom_off[s.i2o_src[p]], ps = keys[order[key[p]]].perm;
+            const int64_t src = other_mom_off[s.i2o_src[p]], ps = keys[key[p]].perm;
             rec[i] = make_int4((int)(uint32_t)src, (int)(src >> 32), (int)ps, p);
         }
         put(out.rec, rec);
