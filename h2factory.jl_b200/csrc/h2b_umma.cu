@@ -17,9 +17,12 @@
 //     into a tensor-memory stage with tcgen05.st. The MMAs take this operand (A) straight from
 //     tensor memory. Couplings without whole 16-byte columns are read row by row from global
 //     memory into a register ring instead;
-//   * moment warps (4-6): cp.async each chunk's source moments into a raw shared-memory ring four
-//     chunks ahead, then write them as the B operand, TF32 high parts plus remainders, in the
-//     canonical no-swizzle K-major layout (a complex piece is split once for its two rows);
+//   * moment warps (4-6), every third chunk each: cp.async the chunk's source moments into a raw
+//     shared-memory stage a turn ahead, then write them as the B operand, TF32 high parts plus
+//     remainders, in the canonical no-swizzle K-major layout (a complex piece is split once for its
+//     two rows). All three on every chunk, joined by a named barrier, they were what the kernel
+//     waited for: 10,931 points, p = 6 real, 12 right-hand sides, I2O 5.68 -> 4.82 ms (4.45 with the
+//     longest interaction lists first);
 //   * one MMA warp (warp 11): per 8-wide k step the products hi*hi + hi*lo + lo*hi (the lo*lo
 //     term is below FP32 rounding), N = 64 columns each, into an FP32 accumulator in tensor memory;
 //     one commit per chunk releases both operand stages;
@@ -37,7 +40,7 @@
 //
 // Every wait on an mbarrier is bounded: a wait that gives up counts itself in a device counter
 // (h2b_tensor_wait_timeouts) and sets the CTA's abort flag; every role then leaves its loop, the
-// MMA thread waits (with the full bound) for the products it issued, the moment warps for their
+// MMA warp waits (with the full bound) for the products it issued, the moment warps for their
 // copies, and the CTA frees its tensor memory and returns with its output tile unwritten.
 
 #include <cuda.h>
@@ -55,8 +58,6 @@ constexpr int UM_M = 128;         // output rows per tile = tensor-memory lanes
 constexpr int UM_KC = 32;         // FP32 K values per chunk: 8 groups of 16 bytes per B row
 constexpr int UM_KG = UM_KC / 4;
 constexpr int UM_NS = 4;          // operand stages: coupling in tensor memory, moments in shared memory
-constexpr int UM_LAG = 4;         // moment copies issued this many chunks ahead of their expansion
-constexpr int UM_RS = UM_LAG + 2; // raw moment stages (a slot is rewritten two barriers after its last read)
 constexpr uint32_t UM_RAWROW = UM_KC * 4 + 16;  // raw moment row: one chunk's values + 16 bytes of padding
 // chunks per accumulation segment: 64 values of K are summed in FP32 (the tensor cores' own
 // rounding) before the segment is added to the FP64 sum (measured on the 65,536-point sphere:
@@ -73,7 +74,7 @@ constexpr int UM_ALA = 3;         // coupling columns copied this many chunks ah
 // 16K registers then allow up to 170 per thread (a thirteenth warp would cap them at 128)
 constexpr int UM_WARPS = 12;
 constexpr int UM_BW = 3;           // moment warps
-constexpr int UM_BT = UM_BW * 32;  // moment threads
+constexpr int UM_RS = 2 * UM_BW;   // raw moment stages, two per moment warp
 constexpr int UM_THREADS = UM_WARPS * 32;
 constexpr int UM_NT_MAX_REAL = 64;    // right-hand sides per tile, real maps (MMA N = 64)
 constexpr int UM_NT_MAX_CPLX = 32;    // complex maps: Re and Im rows make MMA N = 64
@@ -212,20 +213,6 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, unsign
 }
 
 __device__ __forceinline__ bool warp_aborted(volatile int *flag) { return __any_sync(0xffffffffu, *flag != 0); }
-
-// named barrier 1 over the moment warps with an OR vote: every participant gets the same answer
-__device__ __forceinline__ bool bar_vote_or(bool v) {
-    uint32_t out;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(out)
-        : "r"((uint32_t)v), "n"(UM_BT)
-        : "memory");
-    return out != 0;
-}
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -395,7 +382,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
     if (tid == 0) {
         for (int s = 0; s < UM_NS; ++s) {
             mbar_init(&a_full[s], 128);
-            mbar_init(&b_full[s], UM_BT);
+            mbar_init(&b_full[s], 32);
             mbar_init(&empty[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
@@ -419,6 +406,16 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
         int mine = 0;
         for (int p = p0 + tid; p < p1; p += (int)blockDim.x) mine += (W * um_ncoef(t, t.level[r.i2o_src[p]]) + UM_KC - 1) / UM_KC;
         if (mine) atomicAdd(&nchunks_s, mine);
+        // rows past the right-hand sides' rows (real tiles whose width is not a multiple of 16)
+        // are zero in every stage, written once
+        const int zr = np - W * qt_max;
+        for (int o = tid; o < UM_NS * 2 * zr * UM_KG; o += (int)blockDim.x) {
+            const int rr = W * qt_max + (o / UM_KG) % zr, kg = o % UM_KG, sh = o / (UM_KG * zr);  // sh: stage and hi/lo half
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(su32(um_smem) + (uint32_t)sh * ((uint32_t)np * UM_KC * 4) +
+                                                                         goff(rr, kg)),
+                         "r"(0u));
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
     }
     const int C = nchunks_s;
@@ -599,17 +596,28 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
         }
     } else if (warp < 4 + UM_BW) {
         // ---------------- moment warps: B operand into shared memory ----------------
-        const int bt = tid - 128;
-        // copy cursor (pair cp_, chunk ck); a chunk's raw moments are qt_max rows of 64 bytes, copied
-        // as 16-byte pieces (consecutive threads: consecutive pieces of a row), element by element
-        // where a column is not 16-byte aligned or the chunk runs past the pair's coefficients
-        int cp_ = p0, ck = 0;
+        // warp bw takes every UM_BW-th chunk on its own, so nothing but the stages ties the warps
+        const int bw = warp - 4;
+        // copy cursor (pair cp_, chunk ck; the next pair's operands loaded a pair ahead); a chunk's raw
+        // moments are qt_max rows of 128 bytes, copied as 16-byte pieces (consecutive lanes: consecutive
+        // pieces of a row), element by element where a column is not 16-byte aligned or the chunk
+        // runs past the pair's coefficients
+        int cp_ = p0, ck = bw;
         UmPair<T> cu = um_pair<T>(m, r, t, p0, nc, fwd, nrhs, q0, am);
+        UmPair<T> cn = um_pair<T>(m, r, t, min(p0 + 1, p1 - 1), nc, fwd, nrhs, q0, am);
+        auto settle = [&]() {
+            while (cp_ < p1 && ck >= cu.nk) {
+                ck -= cu.nk;
+                cu = cn;
+                if (++cp_ + 1 < p1) cn = um_pair<T>(m, r, t, cp_ + 1, nc, fwd, nrhs, q0, am);
+            }
+        };
+        settle();
         constexpr int EV = 16 / EB;  // elements per piece
-        auto issue = [&](int ci) {
-            const uint32_t rb = raw0 + (uint32_t)(ci % UM_RS) * raw_stage_bytes;
+        auto issue = [&](int turn) {
+            const uint32_t rb = raw0 + (uint32_t)(2 * bw + (turn & 1)) * raw_stage_bytes;
             const int k0 = ck * KQ;
-            for (int pc = bt; pc < qt_max * UM_KG; pc += UM_BT) {
+            for (int pc = lane; pc < qt_max * UM_KG; pc += 32) {
                 const int q = pc / UM_KG, kg = pc % UM_KG, kp = k0 + kg * EV;
                 const uint32_t dst = rb + (uint32_t)q * UM_RAWROW + (uint32_t)kg * 16;
                 const T *src = cu.X + (int64_t)q * cu.snc + kp;
@@ -623,51 +631,36 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
                     }
                 }
             }
-            if (++ck == cu.nk) {
-                ck = 0;
-                if (++cp_ < p1) cu = um_pair<T>(m, r, t, cp_, nc, fwd, nrhs, q0, am);
-            }
+            ck += UM_BW;
+            settle();
         };
-        for (int c = 0; c < UM_LAG && c < C; ++c) {
-            issue(c);
-            cp_commit_group();
-        }
-        // rows past the right-hand sides' rows (real tiles whose width is not a multiple of 16)
-        // are zero in every stage, written once
-        for (int o = bt; o < UM_NS * 2 * (np - W * qt_max) * UM_KG; o += UM_BT) {
-            const int rr = W * qt_max + (o / UM_KG) % (np - W * qt_max), kg = o % UM_KG;
-            const int sh = o / (UM_KG * (np - W * qt_max));  // stage and hi/lo half
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(smem0 + (uint32_t)sh * ((uint32_t)np * UM_KC * 4) +
-                                                                         goff(rr, kg)),
-                         "r"(0u));
-        }
+        if (bw < C) issue(0);
+        cp_commit_group();
         const int npieces = qt_max * UM_KG;  // 16-byte pieces of the raw tile
-        const int q0p = bt % qt_max, kg0 = bt / qt_max;
-        for (int c = 0; c < C; ++c) {
-            const int ci = c + UM_LAG;
-            if (ci < C) issue(ci);
+        const int q0p = lane % qt_max, kg0 = lane / qt_max;
+        for (int c = bw, turn = 0; c < C; c += UM_BW, ++turn) {
+            if (c + UM_BW < C) issue(turn + 1);  // into the stage of the turn before this one
             cp_commit_group();
-            cp_wait_group<UM_LAG>();  // this thread's copies of chunk c have landed
-            // ... and everyone's; the vote makes the stop decision the same for all moment threads
-            // (a thread that left the loop alone would leave the others waiting at this barrier)
-            if (bar_vote_or(abort_s != 0)) break;
+            cp_wait_group<1>();  // this lane's copies of chunk c have landed
+            __syncwarp();        // ... and the warp's
+            if (warp_aborted(&abort_s)) break;
             const int s = c % UM_NS;
             // the expanded stage was last read by the products of chunk c - UM_NS
-            if (c >= UM_NS && !mbar_wait(&empty[s], ((c / UM_NS) - 1) & 1, limit)) {
-                abort_s = 1;  // the stage may still be read: leave it; the next vote stops the loop
-                continue;
+            if (c >= UM_NS && !warp_wait(&empty[s], ((c / UM_NS) - 1) & 1, limit)) {
+                abort_s = 1;
+                break;
             }
-            const uint32_t rb = raw0 + (uint32_t)(c % UM_RS) * raw_stage_bytes;
+            const uint32_t rb = raw0 + (uint32_t)(2 * bw + (turn & 1)) * raw_stage_bytes;
             const uint32_t hb = smem0 + (uint32_t)s * b_stage_bytes;
             const uint32_t lb = hb + (uint32_t)np * (UM_KC * 4);
-            // raw pieces bt, bt + UM_BT, ... as (row q, k group kg), rows fastest: a quarter-warp
+            // raw pieces lane, lane + 32, ... as (row q, k group kg), rows fastest: a quarter-warp
             // reads 8 rows of one k group and writes 8 consecutive rows of the expanded tile
             // (conflict-free); a complex piece (mr, mi) of two k is split once and written to
             // both its rows, Re (mr, -mi) and Im (mi, mr): negation is exact in TF32 parts
             int q = q0p, kg = kg0;
-            for (int pc = bt; pc < npieces; pc += UM_BT) {
-                if (pc != bt) {
-                    q += UM_BT;
+            for (int pc = lane; pc < npieces; pc += 32) {
+                if (pc != lane) {
+                    q += 32;
                     while (q >= qt_max) {
                         q -= qt_max;
                         ++kg;
@@ -701,6 +694,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(&b_full[s]);
+            __syncwarp();  // this turn's raw stage is copied into in the next one
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (TMA && warp == UM_WARPS) {
@@ -878,7 +872,7 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
 //   * eight coupling warps, four per chunk in turn: read, split, write to tensor memory;
 //   * four moment warps, one chunk each in turn: split its moments into shared memory; operand stages
 //     hold a whole segment (two chunks), so the MMA warp waits once per 24 products;
-//   * MMA thread; eight drain warps, which keep the FP64 sums (32 each) in registers: the kernel starts
+//   * the MMA warp; eight drain warps, which keep the FP64 sums (32 each) in registers: the kernel starts
 //     with 80 registers a thread and moves them to the drain warps (setmaxnreg; 256 threads each at 64,
 //     64 and 112 make the 240 x 256 that the block was launched with).
 // ---------------------------------------------------------------------------------------------
