@@ -890,6 +890,13 @@ h2b_status build_side(h2b_core *c, const h2b_map_desc &d, const h2b_side_desc &s
         if (st) return st;
         h.dis_down.push_back(sg);
     }
+    // dense blocks: the longest interaction lists first, so that no CTA of a receiving node starts a long
+    // one when the others end (FP32 form, p = 6 real, 10,931 points: I2O 4.82 -> 4.45 ms, 2,290 points
+    // 0.475 -> 0.373)
+    if (d.coupling_kind == H2B_COUPLING_DENSE)
+        std::stable_sort(recv.begin(), recv.end(), [&](int p, int q) {
+            return s.i2o_ptr[p + 1] - s.i2o_ptr[p] > s.i2o_ptr[q + 1] - s.i2o_ptr[q];
+        });
     h.n_recv = (int)recv.size();
     st = upload_list(c, recv, &h.d_recv);
     if (st) return st;
