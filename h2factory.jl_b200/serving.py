@@ -276,6 +276,9 @@ class GpuExecutor:
         per = 16 if core.field == "complex" else 8
         far = sum(np.asarray(v).nbytes for v in core.collections_test.values())
         ws = 4 * (core.test.nnodes * 64 * per) * max_block + 4 * core.test.npoints * per * max_block
+        if core.coupling_kind == "dense":  # pair products: of all pairs, at most 512 MiB
+            coef = int(max(np.prod(core.shape_test, axis=1).max(), np.prod(core.shape_trial, axis=1).max()))
+            ws += min(512 << 20, len(core.pair_coupling) * coef * per * max_block)
         return int(2 * near + far + nslots * ws)
 
     def load(self, core):
