@@ -346,7 +346,7 @@ def e2e_run(torch, wss, nrhs, steps, modes, seed):
 def pass_times(h2, ws, x, modes, reps):
     """Average device time (ms) of each pass kind over `reps` profiled products per orientation
     (h2b_profile_matvec: CUDA events on the launching stream, passes serialised), and the number
-    of far-pass launches per product."""
+    of far passes per product (one launch each at least; the dense I2O launches two per unit)."""
     acc, nfar = {}, 0
     for m in modes:
         for _ in range(reps):
@@ -517,10 +517,10 @@ def sphere_leg(args, rank, world, local_rank):
         "served_over_plain": served_rate / plain_rate,
         "accuracy": acc,
         "e2e": e2e,
-        "roofline": {"kernel": "i2o_umma_kernel<cfloat> (served form's dense M2L: tcgen05 kind::tf32, three-term split)",
+        "roofline": {"kernel": "i2o_umma_pairs_kernel<cfloat> (served form's dense M2L with its sums: tcgen05 kind::tf32, three-term split)",
                      "bound": "tensor", "achieved": i2o_tf, "peak": bf16, "unit": "TFLOP/s", "frac": i2o_tf / bf16,
                      "peak_kind": f"{peak_kind} dense bf16 (burst)",
-                     "traffic": traffic_table().get(("i2o_umma_kernel", wl)),
+                     "traffic": traffic_table().get(("i2o_umma_pairs_kernel", wl)),
                      "algorithmic_flops": i2o_flops, "avg_launch_ms": i2o_ms,
                      "issued_tf32_tflops": 3 * i2o_tf, "frac_issued_vs_half_bf16": 3 * i2o_tf / (bf16 / 2)},
         "roofline_near": {"kernel": "near_slab_mma_c_kernel (FP64 tensor cores; plain and served forms)",

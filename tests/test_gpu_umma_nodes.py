@@ -4,9 +4,8 @@ Blocks of an odd number of 32-value chunks keep this form, since an accumulation
 chunks runs on into the next pair. Three moment warps take every third chunk each, so a warp skips
 pairs of one chunk (8 and 27 real coefficients, 8 complex ones) and starts those of seven (216
 real) at its first, second or third chunk; an interaction list may be shorter than three chunks.
-Right-hand sides below, at and past
-a tile's 64 (complex: 32), both orientations, with and without permutations. Compared with the FP64
-form: FP32 storage and TF32-split products with 64-value FP32 segments keep 1e-6.
+Right-hand sides below, at and past a tile's 64 (complex: 32), both orientations, with and without
+permutations. Compared with the FP64 form: FP32 storage and TF32-split products with 64-value FP32 segments keep 1e-6.
 """
 
 import copy
