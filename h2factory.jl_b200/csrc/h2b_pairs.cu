@@ -19,8 +19,8 @@
 // its block once per 64 columns and writes 16 bytes per complex sum (8 real) per row, read once by
 // the sums: 8.5 % of the time at 216 complex coefficients, about half at 64 real ones. Measured
 // (I2O per product, FP64): 65,536-point Helmholtz sphere, p = 6, 1 right-hand side 7.73 -> 0.91 ms;
-// 262,144 points, 32 right-hand sides 211 -> 112 ms (26 TFLOP/s); 8,192-point Laplace cube, p = 4,
-// unreduced blocks 2.56 -> 0.052 ms, against chunks of 16 receiving nodes that each staged every
+// 262,144 points, 32 right-hand sides 211 -> 104 ms (28.5 TFLOP/s); 8,192-point Laplace cube, p = 4,
+// unreduced blocks 2.56 -> 0.050 ms, against chunks of 16 receiving nodes that each staged every
 // block they read (1-4 field columns) and one CTA per receiving node (wider blocks).
 #include <algorithm>
 #include <type_traits>

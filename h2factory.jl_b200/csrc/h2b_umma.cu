@@ -858,8 +858,8 @@ i2o_umma_kernel(DMap m, DSide r, DSide t, const int *__restrict__ nodes, int mod
 // What bounds it: the roles' instructions, about 2,700 per chunk (1,360 cycles against 384 for the
 // chunk's products; ncu: 0.51 issued per scheduler and cycle, tensor operands and L2 far from full).
 // Taking one role's work away gains 4-10 % each (the coupling's split most). Measured (I2O per
-// product, 65,536-point Helmholtz sphere, p = 6): 8 right-hand sides 14.2 -> 3.7 ms, 32 right-hand
-// sides 15.1 -> 12.5 ms (2.4 of them the sums) against one receiving node per CTA.
+// product, 65,536-point Helmholtz sphere, p = 6): 8 right-hand sides 14.2 -> 3.2 ms, 32 right-hand
+// sides 15.1 -> 11.3 ms (2 of them the sums) against one receiving node per CTA.
 // Roles (24 warps, six warpgroups):
 //   * scheduler: turns the CTA's items into records in a ring (the block, and every column's moments
 //     and product), so that no other role chases the plan's arrays;
