@@ -1453,7 +1453,6 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
         const int64_t unit = h->pairs[0].unit_elems * (int64_t)vsz;
         ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min(unit * cols, PAIR_BUFFER_BYTES));
     }
-    if (e == cudaSuccess) e = al(&ws->prod, ws->prod_bytes);
     if (e == cudaSuccess) e = al(&ws->xbuf, ndof * vsz);
     if (e == cudaSuccess) e = al(&ws->ybuf, ndof * vsz);
     if (e == cudaSuccess && !cplx && max_nrhs >= 8)
@@ -1461,6 +1460,15 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
     if (e == cudaSuccess && cplx && max_nrhs >= 8 && core->dnear.kind == H2B_NEAR_STORED)
         e = al(&ws->xnear, (size_t)std::max(core->test.ndofs, core->trial.ndofs) * near_rhs_block(max_nrhs) * 2 *
                                sizeof(double));
+    // the pair products' buffer last, and a smaller one where the device is too full for it: more
+    // passes, or the kernels per receiving node where not even the smallest unit fits
+    while (e == cudaSuccess && ws->prod_bytes > 0) {
+        const cudaError_t ep = al(&ws->prod, ws->prod_bytes);
+        if (ep == cudaSuccess) break;
+        if (ep != cudaErrorMemoryAllocation) e = ep;
+        cudaGetLastError();
+        ws->prod_bytes = ws->prod_bytes > (1 << 20) ? ws->prod_bytes / 4 : 0;
+    }
     // the far passes (a chain of dependent launches, the critical path) run on this stream at the
     // device's greatest priority, so their blocks are scheduled ahead of the near field's, which
     // fills the SMs around them
