@@ -234,6 +234,17 @@ struct PairTiles {
     int pstride = 1;              // scalars per pair and right-hand side
 };
 
+// A launch that needs more than 48 KB of dynamic shared memory asks for it by an attribute of the kernel,
+// one value per device that all host threads share. The value set here is the same in every call (all
+// that a block may have beside `static_bytes` of static arrays), so that no thread can lower it between
+// another thread's call and that thread's launch, as a value that follows the map could.
+constexpr int SMEM_BLOCK_MAX = 227 * 1024;
+
+template <class... P>
+cudaError_t allow_most_smem(void (*kernel)(P...), int static_bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BLOCK_MAX - static_bytes);
+}
+
 inline bool chain_ahead(const DMap &m, int nq) { return nq == 1 && m.coupling_kind != H2B_COUPLING_TOEPLITZ; }
 
 template <class... P, class... A>

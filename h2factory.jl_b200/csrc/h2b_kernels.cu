@@ -335,6 +335,7 @@ leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conj
 // followed one another in one CTA per parent.
 // ---------------------------------------------------------------------------------------------
 constexpr int SEP_CHILDREN = 64;  // children contracted side by side at most
+constexpr int SEP_STATIC = 4 * SEP_CHILDREN * (int)sizeof(void *);  // the kernel's static shared arrays, bytes
 
 template <class T, bool UP>
 __global__ void __launch_bounds__(256)
@@ -435,7 +436,7 @@ cudaError_t launch_transfer_sep(const DMap &m, const DSide &s, const int *nodes,
     while (cg > 1 && (2 * cg + 1) * qc * one > 200 * 1024) --cg;
     const size_t sm = (2 * cg + 1) * qc * one;
     auto kern = &transfer_sep_kernel<T, UP>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_most_smem(kern, SEP_STATIC);
     if (e != cudaSuccess) return e;
     for (int q0 = 0; q0 < nq && e == cudaSuccess; q0 += 65535 * qc)
         e = launch_chain(chain_ahead(m, nq), kern, dim3(nnodes, std::min(65535, (nq - q0 + qc - 1) / qc)), 256, sm, st, m, s, nodes,
@@ -1488,6 +1489,7 @@ int block_for(int n, int lo = 32, int hi = 256) {
     return std::min(std::max(b, lo), hi);
 }
 
+// `bytes`: a constant of the kernel (see allow_most_smem)
 template <class K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
     if (bytes > 48 * 1024)
@@ -1641,7 +1643,7 @@ cudaError_t launch_toeplitz_in(bool cplx, int precision, const DMap &m, const DS
         const size_t sm = (size_t)G * (maxtsize + 3 * FFT_NMAX) * sizeof(cdouble);
         const int ntrans = nnodes * m.ncomp * fa.nrhs;
         auto launch = [&](auto kern) {
-            cudaError_t e2 = allow_smem(kern, sm);
+            cudaError_t e2 = allow_most_smem(kern, 0);  // sm follows the map's transforms
             if (e2 == cudaSuccess)
                 e2 = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                           cudaSharedmemCarveoutMaxShared);
@@ -1672,7 +1674,7 @@ cudaError_t launch_toeplitz_out(bool cplx, int precision, const DMap &m, const D
         const size_t sm = (size_t)G * (maxtsize + 3 * FFT_NMAX) * sizeof(cdouble);
         const int ntrans = nnodes * m.ncomp * fa.nrhs;
         auto launch = [&](auto kern) {
-            cudaError_t e2 = allow_smem(kern, sm);
+            cudaError_t e2 = allow_most_smem(kern, 0);  // sm follows the map's transforms
             if (e2 == cudaSuccess)
                 e2 = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                           cudaSharedmemCarveoutMaxShared);

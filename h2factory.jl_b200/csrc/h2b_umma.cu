@@ -80,6 +80,7 @@ constexpr int UM_NT_MAX_REAL = 64;    // right-hand sides per tile, real maps (M
 constexpr int UM_NT_MAX_CPLX = 32;    // complex maps: Re and Im rows make MMA N = 64
 constexpr uint32_t UM_LBO = 128;            // bytes between the two 16-byte K halves of a k step
 constexpr uint32_t UM_SBO = UM_KG * 128;    // bytes between 8-row groups (4 groups of 128 bytes)
+constexpr int UM_STATIC = 1024;  // bound on the kernel's static shared arrays (384 bytes), bytes
 constexpr unsigned UM_SUSPEND_NS = 1000;   // suspend-time hint of one try_wait attempt
 constexpr unsigned UM_SPIN = 1u << 20;      // default attempts before a wait gives up (about a second)
 constexpr unsigned UM_SPIN_FINAL = 1u << 23;  // the final wait for products already issued
@@ -1487,14 +1488,14 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
     if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e0 != cudaSuccess) return e0;
     DMap mm = m;
-    const bool fits = smem + acols + 1024 <= (size_t)optin;
+    const bool fits = smem + acols + UM_STATIC <= (size_t)optin;
     if ((tma || mm.cpl_vec) && fits)
         smem += acols;
     else
         mm.cpl_vec = 0;
     const dim3 grid(nnodes, (maxcoef + UM_M - 1) / UM_M, ntiles);
     auto go = [&](auto kern, auto *am, auto *dm) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_most_smem(kern, UM_STATIC);
         if (e != cudaSuccess) return e;
         kern<<<grid, tma && fits ? UM_THREADS + 32 : UM_THREADS, smem, st>>>(mm, recv, src, nodes, fa.mode, fa.nrhs, qt_max,
                                                                             am, dm, blocks, pitch, std::max(ld, 1));
