@@ -82,7 +82,8 @@ LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), LIB_NAME)
 # every symbol include/h2b200.h declares
 EXPORTS = [
     "h2b_version", "h2b_last_error", "h2b_core_create", "h2b_core_destroy", "h2b_core_get_info",
-    "h2b_workspace_create", "h2b_workspace_destroy", "h2b_matvec", "h2b_matvec_host",
+    "h2b_workspace_create", "h2b_workspace_destroy", "h2b_workspace_create_limited",
+    "h2b_workspace_product_bytes", "h2b_matvec", "h2b_matvec_host",
     "h2b_farmul", "h2b_nearmul", "h2b_farmul_noalloc", "h2b_map_blob_write", "h2b_map_blob_read",
     "h2b_core_create_from_blob", "h2b_tensor_wait_timeouts", "h2b_matvec_host_async",
     "h2b_profile_matvec", "h2b_set_tensor_wait_limit",
@@ -129,6 +130,8 @@ def load_library(path: str | None = None) -> C.CDLL:
     lib.h2b_core_create_from_blob.argtypes = [vp, C.c_size_t, C.c_int32, C.POINTER(vp)]
     lib.h2b_workspace_create.argtypes = [vp, C.c_int32, C.POINTER(vp)]
     lib.h2b_workspace_destroy.argtypes = [vp]
+    lib.h2b_workspace_create_limited.argtypes = [vp, C.c_int32, C.c_int64, C.POINTER(vp)]
+    lib.h2b_workspace_product_bytes.argtypes = [vp, _i64p]
     lib.h2b_tensor_wait_timeouts.argtypes = [C.c_int32, C.POINTER(C.c_uint32)]
     lib.h2b_set_tensor_wait_limit.argtypes = [C.c_int32, C.c_uint32]
     mv = [vp, C.c_int32, C.c_int32, vp, C.c_int64, vp, C.c_int64, _f64p, _f64p, vp]

@@ -417,16 +417,24 @@ def _colmajor(t, n: int):
 
 
 class H2Workspace:
-    """One request slot on a device core; the map itself in forward orientation."""
+    """One request slot on a device core; the map itself in forward orientation.
 
-    def __init__(self, dcore: DeviceCore | H2Core, max_nrhs: int = 1, device: int = 0):
+    `max_product_bytes` bounds the buffer of the dense I2O's pair products (None: the library's own
+    bounds), for programs with many workspaces; `product_bytes` is the size that it got.
+    """
+
+    def __init__(self, dcore: DeviceCore | H2Core, max_nrhs: int = 1, device: int = 0,
+                 max_product_bytes: int | None = None):
         if isinstance(dcore, H2Core):
             dcore = DeviceCore(dcore, device)
         self.dcore = dcore
         self.lib = dcore.lib
         self.max_nrhs = max_nrhs
         h = C.c_void_p()
-        _abi.check(self.lib.h2b_workspace_create(dcore.handle, max_nrhs, C.byref(h)))
+        if max_product_bytes is None:
+            _abi.check(self.lib.h2b_workspace_create(dcore.handle, max_nrhs, C.byref(h)))
+        else:
+            _abi.check(self.lib.h2b_workspace_create_limited(dcore.handle, max_nrhs, max_product_bytes, C.byref(h)))
         self.handle = h
         self.mode = _abi.H2B_FORWARD
         self._lock = threading.Lock()
@@ -438,6 +446,12 @@ class H2Workspace:
     @property
     def shape(self):
         return self.core.size
+
+    @property
+    def product_bytes(self) -> int:
+        n = C.c_int64(0)
+        _abi.check(self.lib.h2b_workspace_product_bytes(self.handle, C.byref(n)))
+        return n.value
 
     def close(self):
         if getattr(self, "handle", None):

@@ -495,6 +495,9 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
 // 262,144 points, FP64, 32 right-hand sides 154, 122, 112, 104, 103. Five plans: a core of 30,011
 // points takes 73 ms to make with them, 70 with four, 86 with eight.
 constexpr int64_t PAIR_BUFFER_BYTES = 512ll << 20;
+// A buffer also takes at most this share of the memory that is free when it is made: the rest is for
+// what the program allocates after it (further workspaces, the driver's own needs, other libraries).
+constexpr int PAIR_BUFFER_FREE_SHARE = 16;
 constexpr int PAIR_PLANS[] = {1, 8, 16, 32, 128};
 constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 128;
 
@@ -1418,8 +1421,20 @@ h2b_status h2b_workspace_destroy(h2b_workspace *ws) {
 }
 
 h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace **out) {
+    return h2b_workspace_create_limited(core, max_nrhs, PAIR_BUFFER_BYTES, out);
+}
+
+h2b_status h2b_workspace_product_bytes(const h2b_workspace *ws, int64_t *bytes) {
+    if (!ws || !bytes) return fail(H2B_ERR_INVALID, "null argument");
+    *bytes = (int64_t)ws->prod_bytes;
+    return H2B_OK;
+}
+
+h2b_status h2b_workspace_create_limited(h2b_core *core, int32_t max_nrhs, int64_t max_product_bytes,
+                                        h2b_workspace **out) {
     if (!core || !out) return fail(H2B_ERR_INVALID, "null argument");
     if (max_nrhs < 1) return fail(H2B_ERR_INVALID, "max_nrhs must be >= 1");
+    if (max_product_bytes < 0) return fail(H2B_ERR_INVALID, "max_product_bytes must be >= 0");
     *out = nullptr;
     DeviceGuard guard(core->device);
     (void)cudaGetLastError();  // a non-sticky error left by other code is not this call's
@@ -1451,7 +1466,7 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
         int64_t cols = (int64_t)max_nrhs * core->dmap.ncomp;
         if (core->precision == H2B_FP32 && !h->pairs[0].tile32) cols = std::min<int64_t>(cols, PAIR_MAX_COLS32 / (cplx ? 2 : 1));
         const int64_t unit = h->pairs[0].unit_elems * (int64_t)vsz;
-        ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min(unit * cols, PAIR_BUFFER_BYTES));
+        ws->prod_bytes = std::max<size_t>(ws->prod_bytes, std::min({unit * cols, PAIR_BUFFER_BYTES, max_product_bytes}));
     }
     if (e == cudaSuccess) e = al(&ws->xbuf, ndof * vsz);
     if (e == cudaSuccess) e = al(&ws->ybuf, ndof * vsz);
@@ -1460,14 +1475,16 @@ h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace 
     if (e == cudaSuccess && cplx && max_nrhs >= 8 && core->dnear.kind == H2B_NEAR_STORED)
         e = al(&ws->xnear, (size_t)std::max(core->test.ndofs, core->trial.ndofs) * near_rhs_block(max_nrhs) * 2 *
                                sizeof(double));
-    // the pair products' buffer last, and a smaller one where the device is too full for it: more
-    // passes, or the kernels per receiving node where not even the smallest unit fits
-    while (e == cudaSuccess && ws->prod_bytes > 0) {
-        const cudaError_t ep = al(&ws->prod, ws->prod_bytes);
-        if (ep == cudaSuccess) break;
-        if (ep != cudaErrorMemoryAllocation) e = ep;
-        cudaGetLastError();
-        ws->prod_bytes = ws->prod_bytes > (1 << 20) ? ws->prod_bytes / 4 : 0;
+    // the pair products' buffer last, within its share of what is then free. It is not needed: without
+    // one for the smallest unit the kernels per receiving node run
+    if (e == cudaSuccess && ws->prod_bytes > 0) {
+        size_t free_bytes = 0, total_bytes = 0;
+        e = cudaMemGetInfo(&free_bytes, &total_bytes);
+        ws->prod_bytes = std::min(ws->prod_bytes, free_bytes / PAIR_BUFFER_FREE_SHARE);
+        if (e == cudaSuccess && al(&ws->prod, ws->prod_bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            ws->prod_bytes = 0;
+        }
     }
     // the far passes (a chain of dependent launches, the critical path) run on this stream at the
     // device's greatest priority, so their blocks are scheduled ahead of the near field's, which

@@ -251,8 +251,20 @@ h2b_status h2b_core_create_from_blob(const void *blob, size_t bytes, int32_t dev
 
 /* Mutable per-request state (moments, spectra, host staging) for up to `max_nrhs` right-hand
  * sides: H2Workspace(core) / similarworkspace (src/maps/workspace.jl:81-113). Several
- * workspaces may share one core. */
+ * workspaces may share one core.
+ *
+ * On dense couplings a workspace also holds a buffer of pair products for the I2O: as much as all
+ * pairs need for max_nrhs right-hand sides, but at most 512 MiB and at most 1/16 of the device
+ * memory that is free when it is made, so that what comes after it still finds room. A smaller
+ * buffer takes more passes; one that does not hold the smallest unit of pairs (up to 4 MiB per
+ * right-hand side) leaves the I2O to kernels per receiving node, several times slower. The buffer's
+ * size can change the last bits of a result: the same terms are summed in another order.
+ * h2b_workspace_create_limited holds the buffer to `max_product_bytes` too (0: none), for programs
+ * with many workspaces; h2b_workspace_product_bytes gives the size that it got. */
 h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace **out);
+h2b_status h2b_workspace_create_limited(h2b_core *core, int32_t max_nrhs, int64_t max_product_bytes,
+                                        h2b_workspace **out);
+h2b_status h2b_workspace_product_bytes(const h2b_workspace *ws, int64_t *bytes);
 h2b_status h2b_workspace_destroy(h2b_workspace *ws);
 
 /*
