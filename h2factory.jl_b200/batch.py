@@ -11,7 +11,11 @@ from __future__ import annotations
 
 import numpy as np
 
-from .core import H2Workspace, OrientedMap, mul_
+from .core import DeviceCore, H2Workspace, OrientedMap, mul_
+
+# The maps of a batch run beside each other, so each has a buffer of pair products of its own: together
+# they take at most this share of the memory that is free once the cores are on the device.
+PRODUCT_SHARE = 4
 
 
 class BatchedMaps:
@@ -24,7 +28,9 @@ class BatchedMaps:
         self.dev = f"cuda:{device}"
         self.nrhs = [int(r) for r in nrhs]
         self.modes = list(modes) if modes is not None else [0] * len(cores)
-        self.ws = [H2Workspace(c, max_nrhs=r, device=device) for c, r in zip(cores, self.nrhs)]
+        dcores = [DeviceCore(c, device) for c in cores]
+        each = torch.cuda.mem_get_info(self.dev)[0] // (PRODUCT_SHARE * max(1, len(cores)))
+        self.ws = [H2Workspace(d, max_nrhs=r, max_product_bytes=each) for d, r in zip(dcores, self.nrhs)]
         self.streams = [torch.cuda.Stream(self.dev) for _ in cores]
         self.inputs, self.outputs = [], []
         for k, (c, r) in enumerate(zip(cores, self.nrhs)):
