@@ -276,10 +276,15 @@ class GpuExecutor:
         per = 16 if core.field == "complex" else 8
         far = sum(np.asarray(v).nbytes for v in core.collections_test.values())
         ws = 4 * (core.test.nnodes * 64 * per) * max_block + 4 * core.test.npoints * per * max_block
-        if core.coupling_kind == "dense":  # pair products: of all pairs, at most 512 MiB
+        plans = 0
+        if core.coupling_kind == "dense":
+            # a slot's pair products: of all pairs, at most 512 MiB; the core's plans for them: up to five a
+            # side, 16 bytes per pair each
+            pairs = len(core.pair_coupling)
             coef = int(max(np.prod(core.shape_test, axis=1).max(), np.prod(core.shape_trial, axis=1).max()))
-            ws += min(512 << 20, len(core.pair_coupling) * coef * per * max_block)
-        return int(2 * near + far + nslots * ws)
+            ws += min(512 << 20, pairs * coef * per * max_block)
+            plans = 2 * 5 * 16 * pairs
+        return int(2 * near + far + plans + nslots * ws)
 
     def load(self, core):
         from .core import DeviceCore
