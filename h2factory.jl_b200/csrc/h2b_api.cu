@@ -592,28 +592,21 @@ h2b_status build_pair_tiles(h2b_core *c, const h2b_map_desc &d, bool test_side, 
         base.stored32 = true;
         for (size_t i = 0; i < keys.size(); ++i) off32[i] = keys[i].off;
     } else if (tensor) {
-        std::vector<float> blocks;
+        const int64_t ld = (base.nc32 + 4 / W - 1) / (4 / W) * (4 / W), size = ld * base.snc32;
+        std::vector<int64_t> first;  // element offset of every block in the stored array
         for (size_t i = 0; i < keys.size(); ++i) {
-            const Key &k = keys[i];
-            if (i > 0 && block_run[i] == block_run[i - 1]) {
-                off32[i] = off32[i - 1];
-                continue;
-            }
-            const int V = 4 / W, ld = (k.nc + V - 1) / V * V;
-            off32[i] = (int64_t)blocks.size() / W;
-            blocks.resize(blocks.size() + (size_t)ld * k.snc * W, 0.0f);
-            float *dst = blocks.data() + off32[i] * W;
-            const double *src = d.coupling + k.off * W;
-            for (int j = 0; j < k.snc; ++j)
-                for (int r = 0; r < k.nc; ++r)
-                    for (int w = 0; w < W; ++w)
-                        dst[((int64_t)j * ld + r) * W + w] =
-                            (float)src[(test_side ? r + (int64_t)j * k.nc : j + (int64_t)r * k.snc) * W + w];
+            if (i == 0 || block_run[i] != block_run[i - 1]) first.push_back(keys[i].off);
+            off32[i] = ((int64_t)first.size() - 1) * size;
         }
         float *fp;
-        CUDA_TRY(c->upload(&fp, blocks.data(), blocks.size()));
+        int64_t *src;
+        CUDA_TRY(c->alloc(&fp, first.size() * size * W));
+        CUDA_TRY(c->upload(&src, first.data(), first.size()));
+        CUDA_TRY(launch_pad_blocks(W == 2, c->dmap.cpl, src, (int)first.size(), base.nc32, base.snc32, !test_side, (int)ld, fp,
+                                   nullptr));
+        CUDA_TRY(cudaStreamSynchronize(nullptr));  // products run on other streams
         base.blocks32 = fp;
-        base.cols32 = (int64_t)blocks.size() / W / ((base.nc32 + 4 / W - 1) / (4 / W) * (4 / W));
+        base.cols32 = (int64_t)first.size() * base.snc32;
     }
     // every plan's arrays in one upload (an allocation costs about as much as building a plan): their
     // offsets stand in for the pointers until then

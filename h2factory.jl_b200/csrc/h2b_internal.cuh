@@ -302,6 +302,10 @@ cudaError_t launch_i2o_umma(bool cplx, const DMap &m, const DSide &recv, const D
 // The sums of one unit's pair products (right-hand sides [q0, q0 + qn)) into the receiving nodes' moments.
 cudaError_t launch_i2o_pairs_sum(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,
                                  const PairUnit &u, const FarArgs &fa, int maxcoef, int q0, int qn, cudaStream_t st);
+// FP32 blocks (rows x cols, at element offsets `off` of `src`; stored transposed when `trans`) copied one after
+// another to `dst` as columns of `ld` elements, zeros past the rows.
+cudaError_t launch_pad_blocks(bool cplx, const void *src, const int64_t *off, int nblocks, int rows, int cols, bool trans,
+                              int ld, void *dst, cudaStream_t st);
 // The FP32 form's dense I2O by stored block on the tcgen05 tensor cores (PairTiles::tile32).
 bool i2o_umma_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes);
 cudaError_t launch_i2o_umma_pairs(bool cplx, const DMap &m, const DSide &recv, const PairTiles &pt, const FarArgs &fa,
