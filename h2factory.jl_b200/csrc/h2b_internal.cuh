@@ -104,12 +104,12 @@ template <> __device__ __forceinline__ void stv(cfloat *p, cfloat v) { *reinterp
 //
 // Which launches go ahead: those of one column, of dense and diagonal couplings, of up to 16 blocks
 // an SM. Blocks that wait hold their places on the SMs, where the near field's kernels run meanwhile.
-// Per product, us, ordinary -> ahead: Laplace maps of 2,048 points 41 -> 38, of 8,192 points 98 -> 88,
-// Helmholtz ellipsoid of 20,011 points 420 -> 409, sphere of 65,536 points 1288 -> 1267 (1290 without
-// the limit on blocks). Slower, so left out: Toeplitz maps (262,144 points, 1027 -> 1080) and several
+// Device time per product, us, ordinary -> ahead: Laplace maps of 2,048 points 36 -> 32, of 8,192 points
+// 107 -> 97, Helmholtz ellipsoid of 20,011 points 420 -> 409, sphere of 65,536 points 1293 -> 1277 (no gain
+// without the limit on blocks). Slower, so left out: Toeplitz maps (262,144 points, 1027 -> 1080) and several
 // columns (12,289 points, three right-hand sides, 449 -> 456; 7,189 points, fourteen, 254 -> 266).
 // ---------------------------------------------------------------------------------------------
-constexpr int CHAIN_BLOCKS = 16 * 148;
+constexpr int CHAIN_BLOCKS = 16 * 148;  // a B200 has 148 SMs
 
 __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -320,6 +320,18 @@ cudaError_t launch_i2o_siblings(bool cplx, int precision, const DMap &m, const D
                                 const SibGroups &g, int maxslen, const FarArgs &fa, cudaStream_t st);
 // The dense I2O by stored block (PairTiles) with FP64 sums: every FP64 map whose pair products fit
 // `prod_bytes`, and FP32 maps of at most PAIR_MAX_COLS32 field columns (W x nq, W = 2 complex).
+//
+// Why 4: a precision line, not a crossover. FP32 blocks of up to 4 field columns have FP64 sums, whose error
+// is the smaller one; wider ones have the tcgen05 kernels' FP32 segments. Measured (I2O, ms, FP64 sums |
+// tcgen05; p real or complex coefficients an axis):
+//   columns                          4              6              8              16             32
+//   12,289 points, p = 4 real    0.149 | 0.175  0.196 | 0.237  0.255 | 0.302  0.447 | 0.535  0.888 | 1.058
+//   12,289 points, p = 5 real    0.380 | 0.255  0.536 | 0.355  0.691 | 0.443  1.361 | 0.863  2.716 | 1.693
+//   12,289 points, p = 6 real    0.919 | 4.386  1.388 | 4.391  1.816 | 4.396  3.557 | 4.447  7.097 | 4.656
+//   65,536 points, p = 6 complex 1.608 | 1.078  2.480 | 1.642  3.213 | 1.986  6.284 | 3.211  12.50 | 5.944
+// So tcgen05 by stored block is the faster form from 125 coefficients on, and the FP64 sums are faster than
+// what wider blocks get here at 64 real coefficients, and at 216 real ones (seven chunks, per receiving
+// node) up to about 20 columns.
 constexpr int PAIR_MAX_COLS32 = 4;
 bool i2o_pairs_eligible(bool cplx, int precision, const DMap &m, int nq, const PairTiles &pt, size_t prod_bytes);
 cudaError_t launch_i2o_pairs(bool cplx, int precision, const DMap &m, const DSide &recv, const PairTiles &pt,

@@ -293,7 +293,6 @@ template <class T, class V>
 __global__ void __launch_bounds__(256)
 leaf_aggregate_kernel(DMap m, DSide s, const int *__restrict__ leaves, bool conjc, int nrhs,
                       const V *__restrict__ x, int64_t ldx, T *__restrict__ am) {
-    chain_open();
     using A = typename ScalarTraits<T>::Acc;  // == V
     extern __shared__ unsigned char smem_raw[];
     A *Ms = reinterpret_cast<A *>(smem_raw), *Xs = Ms + TG_M * TG_LD;
@@ -1334,9 +1333,10 @@ template <class A> __device__ __forceinline__ A lane_sum(A v) {
     return v;
 }
 
-// `parts` matrices of n columns (n k entries apart) with vectors k entries apart are summed.
+// `parts` matrices of n columns (n k entries apart) with vectors k entries apart are summed. (v may be
+// moments that chain_wait guards: no __restrict__.)
 template <class T, class F>
-__device__ __forceinline__ void column_sums(const T *__restrict__ C, const T *__restrict__ v, int k, int n, int parts,
+__device__ __forceinline__ void column_sums(const T *__restrict__ C, const T *v, int k, int n, int parts,
                                             bool conj, F f) {
     using A = typename ScalarTraits<T>::Acc;
     constexpr int U = 4;

@@ -129,7 +129,6 @@ __device__ __forceinline__ void split2(float x, uint32_t &hi, uint32_t &lo) {
     lo = tf32_bits(x - __uint_as_float(hi));
 }
 
-// D (+)= A (tensor memory) * B (shared memory), kind::tf32, and the commit of the products so far.
 // four rows {r0 .. r3} of a tensor map, from x on, into this CTA's shared memory
 __device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap *map, int x, int4 r, uint64_t *bar) {
     asm volatile(
@@ -148,6 +147,7 @@ __device__ __forceinline__ uint32_t elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
     return e;
 }
+// D (+)= A (tensor memory) * B (shared memory), kind::tf32, and the commit of the products so far.
 __device__ __forceinline__ void umma_ts_if(uint32_t elected, uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc,
                                            uint32_t accumulate) {
     asm volatile(
@@ -1427,8 +1427,8 @@ i2o_umma_pairs_kernel(DMap m, UpArgs g, const __grid_constant__ CUtensorMap bloc
 }
 
 bool i2o_umma_eligible(bool cplx, int precision, const DMap &m, int nq) {
-    // from 4 FP32 columns (2 complex right-hand sides) the MMA tile (padded to N = 16) beats the
-    // FP64 mma.sync tile path; a single right-hand side stays on the FMA tile path
+    // narrower blocks, and those of 4 FP32 columns whose pair products fit the buffer, have FP64 sums
+    // (PAIR_MAX_COLS32); without a buffer 4 columns are the least that fill a quarter of the MMA tile
     return precision == H2B_FP32 && m.coupling_kind == H2B_COUPLING_DENSE && (cplx ? 2 : 1) * nq >= 4;
 }
 
