@@ -486,8 +486,8 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
 
 // A workspace's buffer of pair products, and the units of the dense I2O (PairTiles) that it is used
 // with: plans whose units take at most these shares of it per right-hand side, so that a wide block
-// runs all its right-hand sides in one pass over smaller units. The last one is also what
-// h2b_farmul_noalloc's buffer holds.
+// runs all its right-hand sides in one pass over smaller units. (h2b_farmul_noalloc's buffer holds at least
+// two columns of the last one.)
 //
 // Why 512 MiB: every unit ends in a wave of tiles that leaves SMs idle, and the fewer receivers a unit
 // has, the fewer pairs of it share a block. I2O per product at 64, 128, 256, 512 and 1024 MiB, ms:
@@ -499,7 +499,7 @@ constexpr int64_t PAIR_BUFFER_BYTES = 512ll << 20;
 // what the program allocates after it (further workspaces, the driver's own needs, other libraries).
 constexpr int PAIR_BUFFER_FREE_SHARE = 16;
 constexpr int PAIR_PLANS[] = {1, 8, 16, 32, 128};
-constexpr int64_t NOALLOC_PRODUCT_BYTES = PAIR_BUFFER_BYTES / 128;
+constexpr int64_t NOALLOC_PRODUCT_BYTES = 8ll << 20;
 
 // Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of one side, a
 // plan for each share of PAIR_PLANS that cuts them differently. A plan is left out when one receiving
@@ -1469,7 +1469,7 @@ h2b_status h2b_workspace_create_limited(h2b_core *core, int32_t max_nrhs, int64_
         e = al(&ws->xnear, (size_t)std::max(core->test.ndofs, core->trial.ndofs) * near_rhs_block(max_nrhs) * 2 *
                                sizeof(double));
     // the pair products' buffer last, within its share of what is then free. It is not needed: without
-    // one for the smallest unit the kernels per receiving node run
+    // one for the smallest unit, or with one that takes too many passes, the kernels per receiving node run
     if (e == cudaSuccess && ws->prod_bytes > 0) {
         size_t free_bytes = 0, total_bytes = 0;
         e = cudaMemGetInfo(&free_bytes, &total_bytes);
@@ -1517,6 +1517,57 @@ struct BusyGuard {
     }
 };
 
+// Right-hand sides whose products of one unit fit the buffer, and passes over the units for all of them.
+int64_t pair_columns(const PairTiles &t, bool cplx, size_t prod_bytes) {
+    return (int64_t)(prod_bytes / ((size_t)t.unit_elems * (cplx ? 16 : 8)));
+}
+int64_t pair_passes(const PairTiles &t, int nq, bool cplx, size_t prod_bytes) {
+    const int64_t cols = pair_columns(t, cplx, prod_bytes);
+    return cols > 0 ? (int64_t)t.units.size() * ((nq + cols - 1) / cols) : INT64_MAX;
+}
+
+// The plan of the largest units whose products fit the buffer for all right-hand sides at once, else the
+// one of the fewest passes (some right-hand sides each; the smaller units of two plans, whose tiles hold more
+// columns of a pair).
+const PairTiles *pair_plan(const std::vector<PairTiles> &plans, int nq, bool cplx, size_t prod_bytes) {
+    const PairTiles *best = nullptr;
+    int64_t fewest = INT64_MAX;
+    for (const PairTiles &t : plans) {
+        if (pair_columns(t, cplx, prod_bytes) >= nq) return &t;
+        const int64_t passes = pair_passes(t, nq, cplx, prod_bytes);
+        if (passes <= fewest) {
+            fewest = passes;
+            best = &t;
+        }
+    }
+    return best;
+}
+
+// Whether the dense I2O in several passes takes longer by stored block than per receiving node. A pass costs
+// 45 us (tcgen05: 55) beside its products: two launches, each with a last wave that leaves SMs idle. So passes
+// pay where the buffer holds enough work, whatever the map's size. Break-even buffers, MiB, measured at
+// 55,748 pairs with the buffer at 4 to 512 MiB | the line drawn here:
+//   FP64 sums, 16 right-hand sides  p = 3 real 32 | 32, p = 4 15 | 16, p = 5 7 | 8, p = 6 4 | 5;
+//                                   complex 107 | 64, 27 | 32, 12 | 16, 6 | 10; fewer: in proportion, since a
+//                                   receiving node's tile of 16 columns costs the same
+//   tcgen05 (5 or more FP32 columns), p = 4 complex: 6 columns 10 | 12, 16 columns 40 | 32; p = 5 complex 6
+//                                   columns 9 | 6, 32 columns 123 | 65; p = 6 complex 16 columns 12 | 9, 32 32 |
+//                                   38, 64 170 | 152: per receiving node a tile of 64 columns costs the same
+// (p = 4 real, FP64, 16 right-hand sides: 5.8 ms in 110 passes of 4 MiB, 2.0 ms per node, 0.55 ms in one pass.)
+// (The whole buffer of 512 MiB is below the line only for wide blocks of few coefficients in the FP32 form: p = 3
+// complex, 32 right-hand sides 1.33 ms in two passes, 0.89 per node.)
+bool passes_cost_more(const PairTiles &t, int nq, bool cplx, int precision, int k, size_t prod_bytes) {
+    constexpr double MIB = 1 << 20;
+    const int W = cplx ? 2 : 1, cols = W * nq;
+    const bool tcgen05 = precision == H2B_FP32 && cols > PAIR_MAX_COLS32;
+    if (pair_passes(t, nq, cplx, prod_bytes) <= 1) return false;
+    // (per receiving node 4 FP32 columns have the tcgen05 kernel's FP32 segments: by block they keep FP64 sums)
+    if (precision == H2B_FP32 && cols == PAIR_MAX_COLS32) return false;
+    const double line = tcgen05 ? 256 * MIB * cols / (W * k) * std::max(1.0, cols / 16.0)
+                                : 1024 * MIB * W / std::max(k, 32) * std::min(nq, 16) / 16.0;
+    return (double)prod_bytes < line;
+}
+
 // I2O of all receiving nodes of side D from the moments / spectra of side A.
 h2b_status run_i2o(h2b_core *c, const SideHost &D, const SideHost &A, const FarArgs &fa, cudaStream_t st) {
     const int maxcoef = std::max(A.maxcoef, D.maxcoef);
@@ -1526,19 +1577,14 @@ h2b_status run_i2o(h2b_core *c, const SideHost &D, const SideHost &A, const FarA
         return H2B_OK;
     }
     const bool cplx = c->field == H2B_COMPLEX;
-    // the plan of the largest units whose products fit the buffer for all right-hand sides at once, else
-    // the smallest units, some right-hand sides at a time
     const int nq = c->dmap.ncomp * fa.nrhs;
-    const PairTiles *pt = nullptr;
-    for (const PairTiles &t : D.pairs) {
-        pt = &t;
-        if ((size_t)t.unit_elems * (cplx ? 16 : 8) * nq <= fa.prod_bytes) break;
-    }
-    if (pt && i2o_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
+    const PairTiles *pt = pair_plan(D.pairs, nq, cplx, fa.prod_bytes);
+    const bool by_node = pt && passes_cost_more(*pt, nq, cplx, c->precision, A.maxcoef, fa.prod_bytes);
+    if (pt && !by_node && i2o_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
         CUDA_TRY(launch_i2o_pairs(cplx, c->precision, c->dmap, D.d, *pt, fa, D.maxcoef, st));
         return H2B_OK;
     }
-    if (pt && i2o_umma_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
+    if (pt && !by_node && i2o_umma_pairs_eligible(cplx, c->precision, c->dmap, nq, *pt, fa.prod_bytes)) {
         CUDA_TRY(launch_i2o_umma_pairs(cplx, c->dmap, D.d, *pt, fa, D.maxcoef, st));
         return H2B_OK;
     }
@@ -1829,10 +1875,11 @@ h2b_status h2b_profile_matvec(h2b_workspace *ws, int32_t mode, int32_t nrhs, con
 // =============================================================================================
 namespace {
 
-// The scratch array (H2B_NOALLOC_SCRATCH_BYTES and the dense I2O's pair products behind them, on
-// every device that loads the library, until the process exits). Device code may name it directly; host code must not pass `g_noalloc_scratch`
-// itself to a kernel -- on the host that name is only a stand-in, not a device address -- and
-// asks the runtime for the address on each device instead (noalloc_scratch below).
+// The scratch array (H2B_NOALLOC_SCRATCH_BYTES and more room for the dense I2O's pair products behind
+// them, on every device that loads the library, until the process exits). Device code may name it
+// directly; host code must not pass `g_noalloc_scratch` itself to a kernel -- on the host that name is
+// only a stand-in, not a device address -- and asks the runtime for the address on each device
+// instead (noalloc_scratch below).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[H2B_NOALLOC_SCRATCH_BYTES + NOALLOC_PRODUCT_BYTES];
 
 }  // namespace
@@ -1894,8 +1941,9 @@ extern "C" h2b_status h2b_farmul_noalloc(const h2b_core *core_in, int32_t mode, 
     // Nothing in the scratch needs clearing: every pass overwrites a moment or spectrum slot
     // before any pass reads it (leaf products and first-child / first-pair writes overwrite),
     // so whatever the previous call left there is never read.
-    FarArgs fa{mode, nrhs, b, b + mom, b + 2 * mom, b + 2 * mom + spec, b + H2B_NOALLOC_SCRATCH_BYTES,
-               (size_t)NOALLOC_PRODUCT_BYTES};
+    // The pair products take what the arenas leave of the scratch and the array behind it.
+    FarArgs fa{mode, nrhs, b, b + mom, b + 2 * mom, b + 2 * mom + spec, b + need,
+               (size_t)H2B_NOALLOC_SCRATCH_BYTES - need + (size_t)NOALLOC_PRODUCT_BYTES};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const cdouble aA = c->alpha[mode];
     if (!alpha) {

@@ -256,9 +256,10 @@ h2b_status h2b_core_create_from_blob(const void *blob, size_t bytes, int32_t dev
  * On dense couplings a workspace also holds a buffer of pair products for the I2O: as much as all
  * pairs need for max_nrhs right-hand sides, but at most 512 MiB and at most 1/16 of the device
  * memory that is free when it is made, so that what comes after it still finds room. A smaller
- * buffer takes more passes; one that does not hold the smallest unit of pairs (up to 4 MiB per
- * right-hand side) leaves the I2O to kernels per receiving node, several times slower. The buffer's
- * size can change the last bits of a result: the same terms are summed in another order.
+ * buffer takes more passes; where those would take longer, or the buffer does not hold the smallest
+ * unit of pairs (up to 4 MiB per right-hand side), the I2O runs in kernels per receiving node,
+ * several times slower than with the whole buffer. The buffer's size can change the last bits of a
+ * result: the same terms are summed in another order.
  * h2b_workspace_create_limited holds the buffer to `max_product_bytes` too (0: none), for programs
  * with many workspaces; h2b_workspace_product_bytes gives the size that it got. */
 h2b_status h2b_workspace_create(h2b_core *core, int32_t max_nrhs, h2b_workspace **out);
@@ -350,9 +351,9 @@ h2b_status h2b_nearmul(h2b_workspace *ws, int32_t mode, int32_t nrhs, const void
  * another allocator (a framework's caching pool that holds the GPU), a real-time loop that
  * forbids allocation after start-up, or a binding that cannot create and keep a workspace.
  * Instead of a workspace's moment and spectrum arenas it uses one scratch array compiled into
- * the library (H2B_NOALLOC_SCRATCH_BYTES per device for the arenas and 4 MiB behind them for the
- * dense I2O's pair products, held by every GPU that loads the library
- * until the process exits). Same semantics as h2b_farmul on `core`.
+ * the library (H2B_NOALLOC_SCRATCH_BYTES per device for the arenas and 8 MiB behind them, which hold
+ * the dense I2O's pair products together with what the arenas leave; held by every GPU that loads
+ * the library until the process exits). Same semantics as h2b_farmul on `core`.
  *
  * Limits and rules:
  *   - the map's scratch for `nrhs` right-hand sides (two moment arenas, plus two spectrum arenas
