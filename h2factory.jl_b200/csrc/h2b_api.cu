@@ -486,8 +486,7 @@ h2b_status upload_list(h2b_core *c, const std::vector<int> &v, int **dst) {
 
 // A workspace's buffer of pair products, and the units of the dense I2O (PairTiles) that it is used
 // with: plans whose units take at most these shares of it per right-hand side, so that a wide block
-// runs all its right-hand sides in one pass over smaller units. (h2b_farmul_noalloc's buffer holds at least
-// two columns of the last one.)
+// runs all its right-hand sides in one pass over smaller units.
 //
 // Why 512 MiB: every unit ends in a wave of tiles that leaves SMs idle, and the fewer receivers a unit
 // has, the fewer pairs of it share a block. I2O per product at 64, 128, 256, 512 and 1024 MiB, ms:
@@ -499,7 +498,10 @@ constexpr int64_t PAIR_BUFFER_BYTES = 512ll << 20;
 // what the program allocates after it (further workspaces, the driver's own needs, other libraries).
 constexpr int PAIR_BUFFER_FREE_SHARE = 16;
 constexpr int PAIR_PLANS[] = {1, 8, 16, 32, 128};
-constexpr int64_t NOALLOC_PRODUCT_BYTES = 8ll << 20;
+// Behind h2b_farmul_noalloc's arenas, for a few columns in several passes: 224,416 pairs, p = 4 complex, 2 right-hand
+// sides 6.1 ms with 4 MiB for their products, 3.5 with 8 MiB and what the arenas leave, 1.6 with 32; 404,204 pairs,
+// p = 4 real, 4 of them 9.2, 5.1, 1.9.
+constexpr int64_t NOALLOC_PRODUCT_BYTES = 32ll << 20;
 
 // Units and tiles of the dense I2O by stored block (PairTiles) for the receiving nodes of one side, a
 // plan for each share of PAIR_PLANS that cuts them differently. A plan is left out when one receiving
@@ -1527,16 +1529,21 @@ int64_t pair_passes(const PairTiles &t, int nq, bool cplx, size_t prod_bytes) {
 }
 
 // The plan of the largest units whose products fit the buffer for all right-hand sides at once, else the
-// one of the fewest passes (some right-hand sides each; the smaller units of two plans, whose tiles hold more
-// columns of a pair).
+// smallest units (whose tiles hold the most columns of a pair): unless another one takes 0.6 times its passes or
+// fewer, a few right-hand sides at a time. (A pass fewer out of six gains nothing: 9,640 pairs, p = 4 complex, FP32
+// form, 256 right-hand sides 3.46 ms in six of 128, 3.63 in five of 54.)
 const PairTiles *pair_plan(const std::vector<PairTiles> &plans, int nq, bool cplx, size_t prod_bytes) {
     const PairTiles *best = nullptr;
-    int64_t fewest = INT64_MAX;
     for (const PairTiles &t : plans) {
-        if (pair_columns(t, cplx, prod_bytes) >= nq) return &t;
-        const int64_t passes = pair_passes(t, nq, cplx, prod_bytes);
-        if (passes <= fewest) {
-            fewest = passes;
+        best = &t;
+        if (pair_columns(t, cplx, prod_bytes) >= nq) break;
+    }
+    if (!best || pair_columns(*best, cplx, prod_bytes) == 0) return best;
+    double most = 0.6 * (double)pair_passes(*best, nq, cplx, prod_bytes);
+    for (const PairTiles &t : plans) {
+        const double passes = (double)pair_passes(t, nq, cplx, prod_bytes);
+        if (passes <= most) {
+            most = passes;
             best = &t;
         }
     }
@@ -1563,8 +1570,9 @@ bool passes_cost_more(const PairTiles &t, int nq, bool cplx, int precision, int 
     if (pair_passes(t, nq, cplx, prod_bytes) <= 1) return false;
     // (per receiving node 4 FP32 columns have the tcgen05 kernel's FP32 segments: by block they keep FP64 sums)
     if (precision == H2B_FP32 && cols == PAIR_MAX_COLS32) return false;
-    const double line = tcgen05 ? 256 * MIB * cols / (W * k) * std::max(1.0, cols / 16.0)
-                                : 1024 * MIB * W / std::max(k, 32) * std::min(nq, 16) / 16.0;
+    const int tile = tcgen05 ? std::min(cols, 64) : std::min(nq, 16);
+    const double line = tcgen05 ? 256 * MIB * tile / (W * k) * std::max(1.0, tile / 16.0)
+                                : 1024 * MIB * W / std::max(k, 32) * tile / 16.0;
     return (double)prod_bytes < line;
 }
 

@@ -351,7 +351,7 @@ h2b_status h2b_nearmul(h2b_workspace *ws, int32_t mode, int32_t nrhs, const void
  * another allocator (a framework's caching pool that holds the GPU), a real-time loop that
  * forbids allocation after start-up, or a binding that cannot create and keep a workspace.
  * Instead of a workspace's moment and spectrum arenas it uses one scratch array compiled into
- * the library (H2B_NOALLOC_SCRATCH_BYTES per device for the arenas and 8 MiB behind them, which hold
+ * the library (H2B_NOALLOC_SCRATCH_BYTES per device for the arenas and 32 MiB behind them, which hold
  * the dense I2O's pair products together with what the arenas leave; held by every GPU that loads
  * the library until the process exits). Same semantics as h2b_farmul on `core`.
  *

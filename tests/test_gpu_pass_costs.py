@@ -69,6 +69,15 @@ def test_noalloc_against_the_kernels_per_node(p, cplx, precision, nrhs):
     assert _close(y, want, precision)
 
 
+def test_whole_buffer_for_wide_blocks_of_many_coefficients():
+    """Several passes that do pay: about four fifths of the time per receiving node."""
+    dcore, x, y = _case(6, True, "fp32", 64)
+    node, want = _far(dcore, x, y, 0)
+    full, got = _far(dcore, x, y, 1 << 62)
+    assert full < node
+    assert _close(got, want, "fp32")
+
+
 def test_wide_blocks_of_few_coefficients():
     dcore, x, y = _case(3, True, "fp32", 32)
     node, want = _far(dcore, x, y, 0)
