@@ -430,6 +430,7 @@ class H2Workspace:
         self.dcore = dcore
         self.lib = dcore.lib
         self.max_nrhs = max_nrhs
+        self.max_product_bytes = max_product_bytes
         h = C.c_void_p()
         if max_product_bytes is None:
             _abi.check(self.lib.h2b_workspace_create(dcore.handle, max_nrhs, C.byref(h)))
@@ -599,5 +600,6 @@ def nearmul_(y, A, x, alpha=None, beta=None, stream=None):
 
 
 def similarworkspace(ws: H2Workspace, max_nrhs: int | None = None) -> H2Workspace:
-    """A second workspace over the same device core (src/maps/workspace.jl:109-113)."""
-    return H2Workspace(ws.dcore, max_nrhs or ws.max_nrhs)
+    """A second workspace over the same device core (src/maps/workspace.jl:109-113), with the same bound
+    on its pair products."""
+    return H2Workspace(ws.dcore, max_nrhs or ws.max_nrhs, max_product_bytes=ws.max_product_bytes)

@@ -2,9 +2,10 @@
 dense I2O in every form that a smaller buffer selects (GPU).
 
 A block of right-hand sides takes the plan of the largest units whose products fit the buffer for all
-of them, then smaller units, then the smallest units some right-hand sides at a time, and without room
-for those the kernels per receiving node. The bounds below select each of these on maps of 47 and 57
-MiB of products a right-hand side (units of all pairs, 32, 16 and 4 MiB).
+of them, then smaller units, then some right-hand sides at a time, and where that takes too many
+passes, or there is no room for the smallest units, the kernels per receiving node. The bounds below
+select each of these on maps of 47 and 57 MiB of products a right-hand side (units of all pairs, 32,
+16 and 4 MiB).
 
 Tolerances: FP64 sums of O(1) terms keep 1e-12 relative by three orders of magnitude, in whatever
 order; FP32 storage and TF32-split products with 64-value FP32 segments keep 1e-6.
@@ -64,6 +65,9 @@ def test_bound_and_size():
     for limit, least in ((0, 0), (5 * MIB, 5 * MIB), (1 << 62, 15 * MIB)):
         ws = h2.H2Workspace(dcore, max_nrhs=1, max_product_bytes=limit)
         assert least <= ws.product_bytes <= min(limit, 20 * MIB)
+        twin = h2.similarworkspace(ws)
+        assert twin.product_bytes == ws.product_bytes
+        twin.close()
         ws.close()
     with pytest.raises(_abi.H2BError) as err:
         h2.H2Workspace(dcore, max_nrhs=1, max_product_bytes=-1)
