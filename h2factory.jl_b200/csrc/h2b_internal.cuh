@@ -105,7 +105,7 @@ template <> __device__ __forceinline__ void stv(cfloat *p, cfloat v) { *reinterp
 // Which launches go ahead: those of one column, of dense and diagonal couplings, of up to 16 blocks
 // an SM. Blocks that wait hold their places on the SMs, where the near field's kernels run meanwhile.
 // Device time per product, us, ordinary -> ahead: Laplace maps of 2,048 points 36 -> 32, of 8,192 points
-// 107 -> 97, Helmholtz ellipsoid of 20,011 points 420 -> 409, sphere of 65,536 points 1293 -> 1277 (no gain
+// 107 -> 95-97, Helmholtz ellipsoid of 20,011 points 420 -> 409, sphere of 65,536 points 1293 -> 1277 (no gain
 // without the limit on blocks). Slower, so left out: Toeplitz maps (262,144 points, 1027 -> 1080) and several
 // columns (12,289 points, three right-hand sides, 449 -> 456; 7,189 points, fourteen, 254 -> 266).
 // ---------------------------------------------------------------------------------------------
